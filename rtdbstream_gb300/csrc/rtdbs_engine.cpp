@@ -230,6 +230,11 @@ size_t plan_layout(rtdbs_engine* e, std::vector<Part>& parts) {
     // window is a few waves of items at most, so its densest cells must not
     // be one warp's long chain)
     v.item_pts = W < 65536 ? 8 : 32;
+    // blocks of the union: 16 positions on small windows (2,000 warps at most,
+    // so shorter chains count for more than fuller lookups: 10k points in 3-D,
+    // union 45 -> 37 us, 2-D 33 -> 31), 32 above (48k points 51 -> 45 us, 1M
+    // walkers 186 -> 168)
+    v.block_pts = W < 32768 ? 16 : 32;
     v.max_items = W + W / v.item_pts + 64;
     // Neighbour lists of non-core points (MinPts - 2 entries each) replace the
     // label pass's grid scan up to kListCap entries; above that the scan stays.
@@ -703,8 +708,8 @@ int rtdbs_get_stats(rtdbs_engine* e, rtdbs_stats* s) {
     const int nchunks = (e->p.stride + e->chunk - 1) / e->chunk;
     s->chunks_per_slide = nchunks;
     // per chunk 6 kernels, 7 when the sort phase needs a run merge (a chunk
-    // of more than one sort run); then union, flatten and label (or border)
-    int launches = 3;
+    // of more than one sort run); then link, union, flatten and label (or border)
+    int launches = 4;
     for (int j = 0; j < nchunks; ++j) {
         const int c = std::min(e->chunk, e->p.stride - j * e->chunk);
         launches += rtdbs::kChunkPhases + (c > rtdbs::kSortRun ? 1 : 0);
@@ -847,10 +852,9 @@ void pool_drop_shape(rtdbs_pool* p) {
 }
 
 // Phases launched once per stream group: those whose bodies are instantiated
-// per group, and the forest-reuse passes between them (so the increment
-// through the label phase form one run of grouped phases).
+// per group (the increment through the label phase form one run of them).
 bool pool_grouped(int phase) {
-    return rtdbs::batch_phase_split(phase) || phase == rtdbs::kBatchDamage || phase == rtdbs::kBatchReuse;
+    return rtdbs::batch_phase_split(phase);
 }
 
 // Builds (and uploads) the launch tables of one round over `ids`.
@@ -940,9 +944,7 @@ int pool_build_shape(rtdbs_pool* p, const std::vector<int>& ids) {
         for (int ph = 0; ph < rtdbs::kBatchChunkPhases; ++ph) add_launches(ph, items);
     }
     for (auto& it : all_items) it.c = 0;  // cluster phases size by W only
-    // (no damage or reuse launch: the ingest and the decrement mark the lost
-    // cores, the merge and the increment set the start hints)
-    for (int ph = rtdbs::kBatchUnion; ph <= rtdbs::kBatchLabel; ++ph) add_launches(ph, all_items);
+    for (int ph = rtdbs::kBatchLink; ph <= rtdbs::kBatchLabel; ++ph) add_launches(ph, all_items);
     if (img.size() > p->tables_cap) {
         // (cudaFree waits for the rounds that still read the old buffer)
         if (p->d_tables) cudaFree(p->d_tables);
@@ -1330,8 +1332,8 @@ int rtdbs_pool_slide_profiled(rtdbs_pool* p, int32_t n, const int32_t* ids, cons
     if (rc == RTDBS_OK) rc = rtdbs_pool_sync(p);
     if (rc == RTDBS_OK) {
         // batch phases -> the engine's phase slots (sort + run merge are one)
-        // (the forest-reuse passes belong to the union phase, as in the single-stream launch)
-        static const int slot[rtdbs::kNumBatchPhases] = {0, 1, 1, 2, 3, 4, 5, 6, 6, 6, 7, 8};
+        // (the link pass belongs to the union phase, as in the single-stream launch)
+        static const int slot[rtdbs::kNumBatchPhases] = {0, 1, 1, 2, 3, 4, 5, 6, 6, 7, 8};
         float ph[9] = {0};
         for (size_t i = 0; i < p->plan.size(); ++i) {
             float ms = 0.f;

@@ -44,6 +44,7 @@ constexpr int kMergeThreads = 256;
 constexpr int kSortRun = 1024;     // words per radix-sort CTA (one per thread)
 constexpr int kBuildThreads = 512;
 constexpr int kClusterThreads = 256;
+constexpr int kLinkThreads = 256;
 constexpr int kBatch = 8;          // default work items a clustering warp takes at a time
                                    // in a pool launch
 constexpr int kQueryLanes = 16;    // default lanes per query point in the count passes (one
@@ -95,8 +96,8 @@ struct View {
     int dim;
     int cell_mult;              // K: cells per Eps along each axis (1 or 2)
     int grab;                   // work items a clustering warp takes from the queue at a time
-                                // (0: 8 in pool launches; for a large window slid alone 5
-                                // or 8 by items per point, fewer on small ones)
+                                // (0: 8 in pool launches, fewer on small windows slid alone;
+                                // the union: one block of positions per 16)
     int qlanes;                 // lanes per query point in the count passes (16 or 32)
     // parameters
     int W, S, min_pts, units;   // units = W / S
@@ -113,6 +114,8 @@ struct View {
     int item_pts;               // most points of a work item slid alone (8 or 32; 0 = 32; pool
                                 // launches take 32): small windows take short items, so
                                 // dense cells spread over more warps
+    int block_pts;              // sorted positions a union warp takes as one block (16 or 32;
+                                // pool launches take 32)
     int precision;              // RTDBS_PREC_* (batched launches dispatch on it)
     int list_cap;               // entries per neighbour list; -1: no lists (the
                                 // label pass then scans the grid)
@@ -217,8 +220,7 @@ enum BatchPhase : int {
     kBatchMerge,
     kBatchBuild,
     kBatchIncrement,
-    kBatchDamage,
-    kBatchReuse,
+    kBatchLink,
     kBatchUnion,
     kBatchFlatten,
     kBatchLabel,

@@ -43,6 +43,7 @@
 #include <atomic>
 #include <climits>
 #include <cstdint>
+#include <type_traits>
 
 namespace rtdbs {
 namespace {
@@ -1386,148 +1387,403 @@ __global__ void k_hints(View v) {
     }
 }
 
-// Union of every core-core neighbour pair, each unordered pair once (the
-// candidate's sorted position is above the home point's).  A candidate's
-// root is found once per candidate chunk and compared with cached roots of
-// the home points (shared memory, per warp); a link is attempted only where
-// the two differ, so same-set pairs cost no memory traffic.  Finds start
-// from per-position root hints.  Each warp walks
-// a contiguous range of work items (neighbouring cells), so candidate loads
-// reuse L1.
-constexpr int kSingleGrab = 5;  // default work items per grab of a large window slid alone
-                                // whose cells hold several points
+// Cores linked within their own warp's 32 sorted positions, before the union:
+// the points of one cell, and of the cells that follow it in its stencil row,
+// are neighbours in the sorted window, so most sets can be joined there from
+// coalesced loads and warp votes alone -- no table lookups, no walks and no
+// atomics (a point's parent is written only by the warp that holds it; a
+// component kept from the last slide is joined by smaller roots in the union
+// only).  The union then starts from these sets' roots as hints.  Each lane
+// looks at the kLinkReach positions after its own.
+// Bound by instruction issue (22 M warp instructions for a 1M-point walker
+// window with a reach of 8).  Link and union together, us, by reach 0 / 4 / 8:
+// 1M walkers 207 / 168 / 170, 200k trajectories 107 / 80 / 82, 100k prices
+// 131 / 61 / 64, a pool of 32 mixed streams 505 / 338 / 342.
+constexpr int kLinkReach = 4;
+
+struct LinkSmem {
+    float4 pt[kLinkThreads / 32][32];  // .w = root hint
+    unsigned long long key[kLinkThreads / 32][32];
+};
+
+template <int MODE, int DK>
+__device__ __forceinline__ void link_body(const View& v, int bx, LinkSmem& sm) {
+    constexpr int DIM = DK & 3, K = (DK >> 2) + 1;  // dimension, cells per Eps
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const int cur = (int)(v.ctl->b & 1);
+    const int n = v.ctl->nocc[cur];
+    const int i = bx * blockDim.x + threadIdx.x;
+    if ((i & ~31) >= n) return;
+    const bool valid = i < n;
+    const int hint = valid ? v.sroot[i] : -1;
+    const bool core = hint >= 0;
+    const unsigned cores = __ballot_sync(kFull, core);
+    if (!cores) return;
+    const int h0 = __shfl_sync(kFull, hint, __ffs(cores) - 1);
+    if (__all_sync(kFull, !core || hint == h0)) return;  // one set already (or one core)
+    float4 p = valid ? v.spt[cur][i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const unsigned long long key = valid ? v.skey[cur][i] : ~0ull;
+    const int slot = slot_of(p);
+    p.w = __int_as_float(hint);
+    sm.pt[wib][lane] = p;
+    sm.key[wib][lane] = key;
+    __syncwarp();
+    Tally tally;
+    unsigned adj = 1u << lane;  // lanes in this lane's set
+    for (int d = 1; d <= kLinkReach; ++d) {
+        const int o = lane + d;
+        const bool near = o < 32 && valid && sm.key[wib][o & 31] - key <= (unsigned long long)K;
+        if (!__any_sync(kFull, near)) break;
+        bool nb = false;
+        if (near && core) {
+            const float4 q = sm.pt[wib][o];
+            const int qh = __float_as_int(q.w);
+            nb = qh >= 0 && qh != hint && is_nbr<MODE, DIM>(v, p, q, tally);
+        }
+        const unsigned b = __ballot_sync(kFull, nb);
+        if (nb) adj |= 1u << o;
+        if (lane >= d && ((b >> (lane - d)) & 1u)) adj |= 1u << (lane - d);
+    }
+    // transitive closure: each lane takes in the sets of its set's lanes
+    unsigned todo = adj & ~(1u << lane);
+    while (__any_sync(kFull, todo != 0)) {
+        const int src = todo ? __ffs(todo) - 1 : lane;
+        const unsigned m = __shfl_sync(kFull, adj, src);
+        todo &= ~(1u << src);
+        todo |= m & ~adj;
+        adj |= m;
+    }
+    if (core && (adj & (adj - 1u))) {
+        const int root = (int)__reduce_min_sync(adj, (unsigned)hint);
+        // a core under the old root of a kept component stays under it
+        if (hint == slot && root < slot) {
+            v.parent[slot] = root;
+            v.sroot[i] = root;
+        }
+    }
+    flush_stats(v, tally, 0, lane, 1);
+}
+
+template <int MODE, int DK>
+__global__ void __launch_bounds__(kLinkThreads) k_link(View v) {
+    __shared__ LinkSmem sm;
+    link_body<MODE, DK>(v, blockIdx.x, sm);
+}
 
 struct ClusterSmem {
-    int home_root[kClusterThreads / 32][32];
     float4 home_pt[kClusterThreads / 32][32];
     int rstart[kClusterThreads / 32][kMaxRows], rpre[kClusterThreads / 32][kMaxRows + 1];
 };
 
-// Work items a warp takes at a time: the stream's setting, or by default 8
-// in a pool launch (many streams share the GPU); for a single stream up to 8
-// on large windows, fewer on small ones (a 10k-point window has a few hundred
-// to a few thousand items: 8 per grab would leave them to a few dozen warps),
-// and 5 where cells hold several points (fewer than 0.4 items per window
-// point): items are then costly enough that balance beats the queue's atomics
-// (a 1M-point walker window, 0.3 items per point: union 233 us with 8, 224
-// with 5), where on windows of near-empty cells (one item per point, most of
-// them without a core) the atomics dominate and 8 stays faster.
+// Work items the label scan's warps take at a time: the stream's setting, or
+// by default 8 in a pool launch (many streams share the GPU); for a single
+// stream up to 8 on large windows, fewer on small ones (a 10k-point window has
+// a few hundred to a few thousand items: 8 per grab would leave them to a few
+// dozen warps).
 __device__ __forceinline__ int work_grab(const View& v, bool pooled) {
     if (v.grab > 0) return v.grab;
     if (pooled) return kBatch;
-    const int g = max(1, min(kBatch, v.W >> 14));
-    const long long items = v.ctl->nitems;
-    return (g > kSingleGrab && items * 5 < (long long)v.W * 2) ? kSingleGrab : g;
+    return max(1, min(kBatch, v.W >> 14));
 }
 
-template <int MODE, int DK>
-__device__ __forceinline__ void union_body(const View& v, ClusterSmem& sm, int grab) {
+// Blocks of positions a union warp takes at a time: one, as a block holds
+// about 8 cell runs (2 blocks: walkers 168 -> 178 us, trajectories 79 -> 109);
+// the stream's setting counts cell runs.
+__device__ __forceinline__ int union_grab(const View& v) { return max(1, v.grab >> 4); }
+
+// One row of the stencil around a cell, looked up by one lane: kept row
+// `row` of Stencil<DIM, HALF, K> as a range of sorted positions (empty: 0, 0).
+// The first probes of the row's cells are issued together.
+template <int DIM, bool HALF, int K, bool SMALL>
+__device__ __forceinline__ int2 row_range_lane_t(const View& v, const ulonglong2* T, unsigned gen,
+                                                 unsigned long long key, int row) {
+    using St = Stencil<DIM, HALF, K>;
+    using C = typename std::conditional<SMALL, int, long long>::type;  // cell coordinates
+    constexpr int kW = St::kW;
+    const int arow = St::kFirst + row;
+    const bool centre = HALF && row == 0;  // its cells below the home cell are not kept
+    const int s0 = v.shift[0], s1 = v.shift[1];
+    C q0 = (C)(key >> s0), q1 = (C)((key >> s1) & ((1ull << (s0 - s1)) - 1ull)), q2 = (C)(key & ((1ull << s1) - 1ull));
+    if (DIM == 2) {
+        q0 += arow - K;
+    } else if (DIM == 3) {
+        q0 += arow / kW - K;
+        q1 += arow % kW - K;
+    }
+    const C e0 = (C)v.ext[0], e1 = (C)v.ext[1], e2 = (C)v.ext[2];
+    C& ql = DIM == 1 ? q0 : (DIM == 2 ? q1 : q2);  // the axis along the row
+    const C el = DIM == 1 ? e0 : (DIM == 2 ? e1 : e2);
+    const bool in = (DIM == 1 || (q0 >= 0 && q0 < e0)) && (DIM < 3 || (q1 >= 0 && q1 < e1));
+    if (!in) return make_int2(0, 0);
+    const C mid = ql;
+    ql = 0;
+    const unsigned long long rowkey =
+        ((unsigned long long)q0 << s0) | ((unsigned long long)q1 << s1) | (unsigned long long)q2;
+    const int sl = DIM == 1 ? s0 : (DIM == 2 ? s1 : 0);
+    const unsigned long long gtag = (unsigned long long)gen << kKeyBitsMax;
+    ulonglong2 e[kW];
+    unsigned home[kW];
+#pragma unroll
+    for (int k = 0; k < kW; ++k) {
+        const C q = mid + (k - K);
+        e[k].x = 0ull;  // no generation
+        home[k] = 0;
+        if (q >= 0 && q < el && !(centre && k < K)) {
+            const unsigned long long nk = rowkey | ((unsigned long long)q << sl);
+            home[k] = SMALL ? table_home32((unsigned)nk, v.pbits) : table_home(nk, v.pbits);
+            e[k] = T[home[k]];
+        }
+    }
+    int rs = INT_MAX, re = 0;
+#pragma unroll
+    for (int k = 0; k < kW; ++k) {
+        if ((e[k].x >> kKeyBitsMax) != gen) continue;  // out of the grid, or an empty or stale slot
+        const unsigned long long tag = gtag | rowkey | ((unsigned long long)(mid + (k - K)) << sl);
+        const int2 c = e[k].x == tag ? make_int2((int)(unsigned)e[k].y, (int)(unsigned)(e[k].y >> 32))
+                                     : table_find_at(T, v.pmask, (home[k] + 1) & v.pmask, tag);
+        if (c.y > c.x) {
+            rs = min(rs, c.x);
+            re = max(re, c.y);
+        }
+    }
+    return re > 0 ? make_int2(rs, re) : make_int2(0, 0);
+}
+
+template <int DIM, bool HALF, int K>
+__device__ __forceinline__ int2 row_range_lane(const View& v, const ulonglong2* T, unsigned gen,
+                                               unsigned long long key, int row) {
+    if (v.key_bits <= 31) return row_range_lane_t<DIM, HALF, K, true>(v, T, gen, key, row);
+    return row_range_lane_t<DIM, HALF, K, false>(v, T, gen, key, row);
+}
+
+// Union of every core-core neighbour pair.  A warp takes a block of P
+// consecutive sorted positions (View::block_pts), whose cores fall into runs
+// of one cell (segments).  The upper-half stencil rows of all segments are
+// looked up by lanes side by side, the non-empty ones are laid end to end as
+// one candidate stream (positions above a segment's first core), and every
+// lane tests its candidate against the cores of its own segment until one
+// under another root is near.  Hints may be behind the forest, so before any
+// test the open candidates and the home points look up their current roots:
+// a load or two in place of a test against every home point, as most of the
+// pairs whose hints differ have been joined meanwhile.  The near pairs of a
+// chunk are then joined at once: the smallest root per home root by a warp
+// minimum, every other root hooked under it by a lane of its own, so lanes of
+// a warp rarely meet on one parent.  Roots known for home points are kept in
+// shared memory, for candidates in their hints.
+//
+// Bound by instruction issue and L2 latency (DRAM throughput 5%).  Against one
+// cell per warp, candidates looked up 14 cells at a time with shuffles, a find
+// and a hook per near pair: link and union 225 -> 168 us on the 1M-point
+// walker window (10.8 -> 4.4 M distance tests), 74 -> 41 us on the 500k precision stream, 297 -> 79 us on 200k trajectories, 520
+// -> 62 us on 100k prices, 606 -> 286 us per round of a 32-stream pool.
+// Without the root lookups before the tests: 204, 41, 129, 142, 430.
+// Thread blocks per SM 4 / 5 / 6: pool round 312 / 286 / 304 us, walkers at 5 /
+// 6 167 / 168 (registers against warps in flight).
+constexpr int kUnionBlocks = 5;
+
+template <int DIM, int K>
+struct UnionRows {
+    static constexpr int kRows = Stencil<DIM, true, K>::kRows;
+    static constexpr int kTasks = 32 * kRows;  // stencil rows of a block's segments, at most
+};
+
+template <int DIM, int K>
+struct UnionSmem {
+    float4 pt[kClusterThreads / 32][32];  // home points, .w = root known
+    unsigned long long skey[kClusterThreads / 32][32];
+    unsigned segm[kClusterThreads / 32][32];  // home cores of a segment
+    int tstart[kClusterThreads / 32][UnionRows<DIM, K>::kTasks];
+    int tpre[kClusterThreads / 32][UnionRows<DIM, K>::kTasks + 1];
+    unsigned char tseg[kClusterThreads / 32][UnionRows<DIM, K>::kTasks];
+};
+
+template <int MODE, int DK, class Smem>
+__device__ __forceinline__ void union_body(const View& v, Smem& sm, int P, int grab) {
     constexpr int DIM = DK & 3, K = (DK >> 2) + 1;  // dimension, cells per Eps
-    float4(&home_pt)[kClusterThreads / 32][32] = sm.home_pt;
-    int(&rstart)[kClusterThreads / 32][kMaxRows] = sm.rstart;
-    int(&rpre)[kClusterThreads / 32][kMaxRows + 1] = sm.rpre;
+    constexpr int R = UnionRows<DIM, K>::kRows;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    volatile int* rh = sm.home_root[wib];
-    const float4* hpt = home_pt[wib];
+    float4* hpt = sm.pt[wib];
+    int* tstart = sm.tstart[wib];
+    int* tpre = sm.tpre[wib];
+    unsigned char* tseg = sm.tseg[wib];
+    unsigned* segm = sm.segm[wib];
     const long long b = v.ctl->b;
     const int cur = (int)(b & 1);
     const unsigned gen = gen_of_build(b);
-    const int nitems = min(v.ctl->nitems, v.max_items);
+    const int n = v.ctl->nocc[cur];
+    const int nblk = (n + P - 1) / P;
     const float4* spt = v.spt[cur];
-    const unsigned long long* skey = v.skey[cur];
     const ulonglong2* T = v.table[cur];
     int* parent = v.parent;
-    // Root hints by sorted position (an ancestor of the point: its own slot
-    // or the old root of its intact component; -1 for a non-core point, so
-    // the hint alone tells a core; set by the merge and the increment, see
-    // start_hint): coalesced with the candidate loads, and refreshed as roots
-    // are found, so find walks stay short.
+    // Root hints by sorted position (an ancestor of the point: its own slot,
+    // its set's root from the link pass or the old root of its intact
+    // component; -1 for a non-core point, so the hint alone tells a core):
+    // coalesced with the candidate loads, and refreshed as roots are found,
+    // so find walks stay short.
     volatile int* hint = v.sroot;
     Tally tally;
     int err = 0;
-    // Warps take batches of `grab` consecutive work items (neighbouring
-    // cells: candidate loads reuse L1) from a counter, so uneven items do not
-    // leave warps idle at the end.
-    int it1 = 0;
-    for (int itx = nitems;;) {
-        if (itx >= it1) {
+    int bk1 = 0;
+    for (int bk = nblk;;) {
+        if (bk >= bk1) {
             int got = 0;
             if (lane == 0) got = atomicAdd(&v.ctl->union_next, grab);
-            itx = __shfl_sync(kFull, got, 0);
-            if (itx >= nitems) break;
-            it1 = min(itx + grab, nitems);
+            bk = __shfl_sync(kFull, got, 0);
+            if (bk >= nblk) break;
+            bk1 = min(bk + grab, nblk);
         }
-        const int2 item = v.items[itx++];
-        const int start = item.x, len = item.y;
-        const bool hv = lane < len;
-        float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
-        bool hcore = false;
-        int hh = -1;
-        if (hv) {
-            h = spt[start + lane];
-            hh = hint[start + lane];
-            hcore = hh >= 0;
-        }
+        const int start = bk++ * P;
+        const int i = start + lane;
+        const bool hv = lane < P && i < n;
+        const int hh = hv ? hint[i] : -1;
+        const bool hcore = hh >= 0;
         const unsigned hmask = __ballot_sync(kFull, hcore);
         if (!hmask) continue;
+        float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+        unsigned long long key = 0;
+        if (hcore) {
+            h = spt[i];
+            key = v.skey[cur][i];
+        }
+        int hr = hh;  // the root known for the lane's home point
+        h.w = __int_as_float(hh);
+        // segments: the cores of one cell
+        const unsigned below = hmask & lanemask_lt(lane);
+        const unsigned long long kprev = __shfl_sync(kFull, key, below ? 31 - __clz(below) : lane);
+        const unsigned leaders = __ballot_sync(kFull, hcore && (!below || kprev != key));
+        const int ns = __popc(leaders);
+        const unsigned upto = leaders & (lanemask_lt(lane) | (1u << lane));
+        const int first = upto ? 31 - __clz(upto) : 0;  // first core of the lane's segment
         __syncwarp();
-        if (hcore) rh[lane] = hh;
-        home_pt[wib][lane] = h;
-        // All home cores under one hint r0 (common once the previous forest is
-        // reused): a candidate chunk whose cores all carry r0 is one set with
-        // them and is skipped without the per-home loop.
-        const int r0 = __shfl_sync(kFull, hh, __ffs(hmask) - 1);
-        const bool uni = __all_sync(kFull, !hcore || hh == r0);
-        const int hmin = start + __ffs(hmask) - 1;
-        int rs, re;
-        row_ranges<DIM, true, K>(v, T, gen, skey[start], lane, rs, re);
-        const int total = candidate_stream<Stencil<DIM, true, K>::kRows>(rs, re, hmin + 1, lane, rstart[wib], rpre[wib]);
+        hpt[lane] = h;
+        if ((leaders >> lane) & 1u) {
+            const unsigned later = leaders & ~((2u << lane) - 1u);
+            const int at = __popc(upto) - 1;
+            segm[at] = hmask & ~lanemask_lt(lane) & (later ? lanemask_lt(__ffs(later) - 1) : kFull);
+            sm.skey[wib][at] = key;
+        }
+        __syncwarp();
+        // rows of all segments, the non-empty ones end to end
+        int nt = 0, total = 0;
+        for (int t0 = 0; t0 < ns * R; t0 += 32) {
+            const int t = t0 + lane, seg = t / R;
+            int a = 0, len = 0;
+            if (t < ns * R) {
+                const int2 rr = row_range_lane<DIM, true, K>(v, T, gen, sm.skey[wib][seg], t - seg * R);
+                a = max(rr.x, start + __ffs(segm[seg]));
+                len = max(rr.y - a, 0);
+            }
+            int incl = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(kFull, incl, o);
+                if (lane >= o) incl += x;
+            }
+            const unsigned some = __ballot_sync(kFull, len > 0);
+            if (len > 0) {
+                const int at = nt + __popc(some & lanemask_lt(lane));
+                tstart[at] = a;
+                tpre[at] = total + incl - len;
+                tseg[at] = (unsigned char)seg;
+            }
+            nt += __popc(some);
+            total += __shfl_sync(kFull, incl, 31);
+        }
+        if (lane == 0) tpre[nt] = total;
+        int fr = __shfl_sync(kFull, hr, first);
+        unsigned mixed = __ballot_sync(kFull, hcore && hr != fr);  // cores not under their segment's first root
+        __syncwarp();
         int r = 0;
         for (int base = 0; base < total; base += 32) {
             const int idx = base + lane;
-            int pos = 0, qh = 0;
+            int pos = 0, qh = -1;
+            unsigned mm = 0;
             float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-            bool qc = false;
             if (idx < total) {
-                pos = stream_pos(idx, r, rstart[wib], rpre[wib]);
+                while (idx >= tpre[r + 1]) ++r;
+                pos = tstart[r] + idx - tpre[r];
                 q = spt[pos];
                 qh = hint[pos];
-                qc = qh >= 0;
+                mm = segm[tseg[r]];
+                // a segment under one root and a candidate under it: one set
+                if (qh < 0 || (!(mixed & mm) && __float_as_int(hpt[__ffs(mm) - 1].w) == qh)) mm = 0;
             }
-            if (!__any_sync(kFull, qc && !(uni && qh == r0))) continue;
-            // Pairs whose hints already agree are in one set: no test, no link.
-            unsigned adj = 0;
-            unsigned mm = hmask;
-            while (mm) {
-                const int hi = __ffs(mm) - 1;
-                mm &= mm - 1;
-                if (qc && pos > start + hi && qh != rh[hi] && is_nbr<MODE, DIM>(v, hpt[hi], q, tally))
-                    adj |= 1u << hi;
+            if (!__any_sync(kFull, mm != 0)) continue;
+            {
+                // hints may be behind the forest: the current roots of the open
+                // candidates and of the home points
+                volatile int* up = parent;
+                const int uq = mm ? up[qh] : qh, uh = hcore ? up[hr] : hr;
+                if (uq != qh) {
+                    qh = uf_find(parent, uq);
+                    hint[pos] = qh;
+                }
+                if (uh != hr) hr = uf_find(parent, uh);
+                __syncwarp();
+                if (__any_sync(kFull, uh != hr || uh != __float_as_int(h.w))) {
+                    h.w = __int_as_float(hr);
+                    if (hcore) hpt[lane].w = h.w;
+                    fr = __shfl_sync(kFull, hr, first);
+                    mixed = __ballot_sync(kFull, hcore && hr != fr);
+                    __syncwarp();
+                }
+                if (mm && !(mixed & mm) && __float_as_int(hpt[__ffs(mm) - 1].w) == qh) mm = 0;
             }
-            if (adj) {
-                int rq = uf_find(parent, qh);
-                while (adj) {
-                    const int hi = __ffs(adj) - 1;
-                    adj &= adj - 1;
-                    const int ra = rh[hi];
-                    if (ra != rq) {
-                        rq = uf_hook(parent, ra, rq, err);
-                        rh[hi] = rq;  // an ancestor of both points (benign race)
+            while (__any_sync(kFull, mm != 0)) {
+                int ga = 0;
+                bool nb = false;
+                while (__any_sync(kFull, mm != 0 && !nb)) {
+                    if (mm != 0 && !nb) {
+                        const float4 hp = hpt[__ffs(mm) - 1];
+                        mm &= mm - 1;
+                        ga = __float_as_int(hp.w);
+                        nb = ga != qh && is_nbr<MODE, DIM>(v, hp, q, tally);
                     }
                 }
-                if (rq != qh) hint[pos] = rq;
+                const unsigned near = __ballot_sync(kFull, nb);
+                if (!near) break;
+                int top = 0;
+                bool lead = false;
+                if (nb) {
+                    const unsigned pq = __match_any_sync(near, qh), pa = __match_any_sync(near, ga);
+                    top = min(ga, (int)__reduce_min_sync(pa, (unsigned)qh));
+                    int res = top;
+                    if (!(pq & pa & lanemask_lt(lane)) && qh != top) res = uf_hook(parent, qh, top, err);
+                    lead = !(pa & lanemask_lt(lane));
+                    if (lead && ga != top) res = min(res, uf_hook(parent, ga, top, err));
+                    __syncwarp(near);
+                    top = (int)__reduce_min_sync(pa, (unsigned)res);
+                    if (qh != top) {
+                        hint[pos] = top;
+                        qh = top;
+                    }
+                }
+                // the home points' roots
+                unsigned todo = __ballot_sync(kFull, lead);
+                while (todo) {
+                    const int l = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const int from = __shfl_sync(kFull, ga, l), to = __shfl_sync(kFull, top, l);
+                    if (hr == from) hr = to;
+                }
+                __syncwarp();
+                h.w = __int_as_float(hr);
+                if (hcore) hpt[lane].w = h.w;
+                fr = __shfl_sync(kFull, hr, first);
+                mixed = __ballot_sync(kFull, hcore && hr != fr);
+                __syncwarp();
             }
-            __syncwarp();
         }
-        if (hcore) hint[start + lane] = rh[lane];
+        if (hcore && hr != hh) hint[i] = hr;
+        __syncwarp();
     }
     flush_stats(v, tally, err, lane, 1);
 }
 
 template <int MODE, int DK>
-__global__ void __launch_bounds__(kClusterThreads, 8) k_union(View v) {
-    __shared__ ClusterSmem sm;
-    union_body<MODE, DK>(v, sm, work_grab(v, false));
+__global__ void __launch_bounds__(kClusterThreads, kUnionBlocks) k_union(View v) {
+    __shared__ UnionSmem<(DK & 3), (DK >> 2) + 1> sm;
+    union_body<MODE, DK>(v, sm, v.block_pts, union_grab(v));
 }
 
 // The neighbour list of the non-core point at sorted position `at`, from one
@@ -1799,9 +2055,8 @@ template <> struct PhaseShape<kBatchDecrement> { static constexpr int threads = 
 template <> struct PhaseShape<kBatchMerge> { static constexpr int threads = kMergeThreads, min_blocks = 1; };
 template <> struct PhaseShape<kBatchBuild> { static constexpr int threads = kBuildThreads, min_blocks = 1; };
 template <> struct PhaseShape<kBatchIncrement> { static constexpr int threads = 256, min_blocks = 8; };
-template <> struct PhaseShape<kBatchDamage> { static constexpr int threads = 256, min_blocks = 1; };
-template <> struct PhaseShape<kBatchReuse> { static constexpr int threads = 256, min_blocks = 1; };
-template <> struct PhaseShape<kBatchUnion> { static constexpr int threads = kClusterThreads, min_blocks = 8; };
+template <> struct PhaseShape<kBatchLink> { static constexpr int threads = kLinkThreads, min_blocks = 1; };
+template <> struct PhaseShape<kBatchUnion> { static constexpr int threads = kClusterThreads, min_blocks = kUnionBlocks; };
 template <> struct PhaseShape<kBatchFlatten> { static constexpr int threads = 256, min_blocks = 6; };
 template <> struct PhaseShape<kBatchLabel> { static constexpr int threads = kClusterThreads, min_blocks = 6; };
 
@@ -1860,9 +2115,12 @@ __global__ void __launch_bounds__(PhaseShape<PHASE>::threads, PhaseShape<PHASE>:
     } else if constexpr (PHASE == kBatchIncrement) {
         __shared__ StreamSmem sm;
         incr_body<MODE, DK>(sv, it.j, it.c, 0, bx, sm);
+    } else if constexpr (PHASE == kBatchLink) {
+        __shared__ LinkSmem sm;
+        link_body<MODE, DK>(sv, bx, sm);
     } else if constexpr (PHASE == kBatchUnion) {
-        __shared__ ClusterSmem sm;
-        union_body<MODE, DK>(sv, sm, work_grab(sv, true));
+        __shared__ UnionSmem<(DK & 3), (DK >> 2) + 1> sm;
+        union_body<MODE, DK>(sv, sm, 32, union_grab(sv));
     } else if constexpr (PHASE == kBatchFlatten) {
         __shared__ StreamSmem sm;
         flatten_body<MODE, DK>(sv, bx, nbx, sm);
@@ -1968,9 +2226,10 @@ cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, 
             // each on sparse windows), all the SMs hold on large ones
             const int need = (v.W + 95) / 96;
             const int blocks = max(1, min(sms * 6, need));
-            if (phase == kPhaseUnion)
-                RTDBS_DISPATCH(precision, dk_of(v), k_union, max(1, min(sms * 8, need)), kClusterThreads, s, v);
-            else
+            if (phase == kPhaseUnion) {
+                RTDBS_DISPATCH(precision, dk_of(v), k_link, (v.W + kLinkThreads - 1) / kLinkThreads, kLinkThreads, s, v);
+                RTDBS_DISPATCH(precision, dk_of(v), k_union, max(1, min(sms * kUnionBlocks, (v.W + v.block_pts * 8 - 1) / (v.block_pts * 8))), kClusterThreads, s, v);
+            } else
                 RTDBS_DISPATCH(precision, dk_of(v), k_label, blocks, kClusterThreads, s, v, advance);
             break;
         }
@@ -2043,8 +2302,7 @@ int batch_blocks(int phase, const View& v, int c) {
         case kBatchIncrement: return (c * v.qlanes + 255) / 256;
         case kBatchMerge: return (v.W + kMergeTile - 1) / kMergeTile;
         case kBatchBuild: return (v.W + kBuildThreads - 1) / kBuildThreads;
-        case kBatchDamage: return 0;  // marked in the ingest and the decrement
-        case kBatchReuse: return 0;  // start hints set by the merge and the increment
+        case kBatchLink: return (v.W + kLinkThreads - 1) / kLinkThreads;
         case kBatchUnion: return max(1, min(1024, (v.W + 1023) / 1024));  // persistent, queue-fed
         case kBatchLabel:
             if (v.list_cap >= 0) return max(1, min(1024, (v.W + 1023) / 1024));  // k_border
@@ -2055,7 +2313,7 @@ int batch_blocks(int phase, const View& v, int c) {
 }
 
 bool batch_phase_split(int phase) {
-    return phase == kBatchDecrement || phase == kBatchIncrement || phase == kBatchUnion ||
+    return phase == kBatchDecrement || phase == kBatchIncrement || phase == kBatchLink || phase == kBatchUnion ||
            phase == kBatchFlatten || phase == kBatchLabel;
 }
 
@@ -2098,8 +2356,7 @@ cudaError_t launch_batch(int phase, int prec, int dim, const BatchLaunch& L, int
         case kBatchBuild: k_batch<kBatchBuild, 0, 0><<<total_blocks, t, 0, s>>>(L); break;
         case kBatchDecrement: RTDBS_BATCH_MD(kBatchDecrement, total_blocks, t, s); break;
         case kBatchIncrement: RTDBS_BATCH_MD(kBatchIncrement, total_blocks, t, s); break;
-        case kBatchDamage: break;  // no kernel: marked in the ingest and the decrement
-        case kBatchReuse: break;  // no kernel: start hints set by the merge and the increment
+        case kBatchLink: RTDBS_BATCH_MD(kBatchLink, total_blocks, t, s); break;
         case kBatchUnion: RTDBS_BATCH_MD(kBatchUnion, total_blocks, t, s); break;
         case kBatchFlatten: RTDBS_BATCH_MD(kBatchFlatten, total_blocks, t, s); break;
         case kBatchLabel: RTDBS_BATCH_MD(kBatchLabel, total_blocks, t, s); break;

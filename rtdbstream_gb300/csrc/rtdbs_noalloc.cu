@@ -163,6 +163,8 @@ int window_view(View& v, unsigned char* base, const float* d_points, int n, int 
     v.pbits = 15;
     v.pmask = (unsigned)(kTableSlots - 1);
     v.max_items = kMaxItems;
+    v.item_pts = 32;
+    v.block_pts = 16;
     v.list_cap = -1;  // no neighbour lists: the label pass scans the grid
     v.list_stride = 0;
     v.nlist = v.ntrack = v.rslot = v.damaged = v.sorder = nullptr;
