@@ -171,7 +171,9 @@ struct rtdbs_engine {
     int staging_points = 0;  // capacity of the staging buffer in points
     void* dev_block = nullptr;
     size_t dev_bytes = 0;
+    void* d_box = nullptr;   // bounding box of a window being loaded
     Ctl* h_ctl = nullptr;    // pinned mirror of the control block
+    bool pooled = false;     // slid by a pool's rounds
     bool geometry_ready = false;
     bool loaded = false;
     cudaGraphExec_t slide_graph = nullptr;
@@ -274,6 +276,7 @@ size_t plan_layout(rtdbs_engine* e, std::vector<Part>& parts) {
         {(void**)&v.xpt, sizeof(float4) * C},
         {(void**)&v.sorder, sizeof(int) * W},
         {(void**)&v.staging, sizeof(float) * (size_t)e->staging_points * dim},
+        {(void**)&e->d_box, sizeof(unsigned) * 6},
         {(void**)&v.ctl, sizeof(Ctl)},
     };
     size_t total = 0;
@@ -308,12 +311,26 @@ int check_device_error(rtdbs_engine* e) {
     return RTDBS_OK;
 }
 
+// Whether a slide builds the grid anew from all slots instead of by chunk
+// steps: where the new points make two chunks or more and at least a
+// twentieth of the window.  Device us per slide, chunk steps against a whole
+// build (2-D mixture / walkers): W = 50k, S = W 358 / 391 against 144 / 177,
+// S = W/2 207 / 236 against 144 / 175; W = 200k, S = 20k 257 / 232 against 223
+// / 232; W = 1M, S = 100k 1085 / 1077 against 613 / 699, S = 50k 720 / 706
+// against 597 / 697, S = 20k 492 / 450 against 565 / 693.  One chunk is always
+// better stepped (W = S = 10k: 102 against 107).
+bool slide_builds_window(const rtdbs_engine* e) {
+    return e->p.stride > e->chunk && 20ll * e->p.stride >= e->p.window && rtdbs::window_build_fits(e->v);
+}
+
 // (pipelined: the label pass first waits for the last output copies; while
 // capturing, that wait becomes an external-event wait node of the graph)
 int enqueue_slide(rtdbs_engine* e, bool capturing, bool pipelined) {
     const int S = e->p.stride, C = e->chunk;
     const int nchunks = (S + C - 1) / C;
-    for (int j = 0; j < nchunks; ++j) {
+    const bool whole = slide_builds_window(e);
+    if (whole) CUDA_TRY(rtdbs::launch_window_build(e->v, e->p.precision, e->v.staging, S, 0, e->stream));
+    for (int j = 0; j < nchunks && !whole; ++j) {
         const int c = std::min(C, S - j * C);
         CUDA_TRY(rtdbs::launch_chunk_step(e->v, e->p.precision, j, c, 0, j * C, e->stream, e->side, e->ev_fork,
                                           e->ev_join));
@@ -395,6 +412,37 @@ int fetch_ctl_and_sync(rtdbs_engine* e) {
     if (e->copy) CUDA_TRY(cudaStreamSynchronize(e->copy));
     e->pipe_pending = false;  // everything queued, pipelined slides included, is done
     return check_device_error(e);
+}
+
+// Finite bounding box of the window's points, from the device; per axis 0 to
+// 0 where no coordinate is finite.  Device points of the caller are read on
+// the legacy default stream, after all work queued there and on the engine's
+// stream (they may have been written on either).
+int device_bbox(rtdbs_engine* e, const float* d_points, int callers, float* mn, float* mx) {
+    cudaStream_t s = e->stream;
+    if (callers) {
+        const int rc = ensure_side(e);
+        if (rc != RTDBS_OK) return rc;
+        s = cudaStreamLegacy;
+        CUDA_TRY(cudaEventRecord(e->ev_fork, e->stream));
+        CUDA_TRY(cudaStreamWaitEvent(s, e->ev_fork, 0));
+    }
+    unsigned box[6];
+    unsigned* d_box = reinterpret_cast<unsigned*>(e->d_box);
+    CUDA_TRY(rtdbs::launch_bbox(d_points, e->p.window, e->p.dim, d_box, s));
+    CUDA_TRY(cudaMemcpyAsync(box, d_box, sizeof(box), cudaMemcpyDeviceToHost, s));
+    CUDA_TRY(cudaStreamSynchronize(s));
+    for (int a = 0; a < e->p.dim; ++a) {
+        if (box[a] > box[3 + a]) {
+            mn[a] = mx[a] = 0.0f;
+            continue;
+        }
+        for (int k = 0; k < 2; ++k) {
+            const unsigned u = box[a + 3 * k], bits = (u >> 31) ? u & 0x7fffffffu : ~u;
+            std::memcpy(k ? &mx[a] : &mn[a], &bits, sizeof(float));
+        }
+    }
+    return RTDBS_OK;
 }
 
 }  // namespace
@@ -526,27 +574,33 @@ int rtdbs_load_window(rtdbs_engine* e, const float* points, int points_on_device
     DeviceGuard guard(e->device);
     CUDA_TRY(guard.err);
     const int W = e->p.window, dim = e->p.dim;
+    // Host points go to the device once (the sorted points of the side that
+    // this build does not lay out hold them); device points are read in place.
+    const float* d_points = points;
+    if (!points_on_device) {
+        d_points = reinterpret_cast<const float*>(e->v.spt[0]);
+        CUDA_TRY(cudaMemcpyAsync(e->v.spt[0], points, sizeof(float) * (size_t)W * dim, cudaMemcpyHostToDevice,
+                                 e->stream));
+    }
     if (!e->p.has_bbox) {
-        std::vector<float> host;
-        const float* h = points;
-        if (points_on_device) {
-            host.resize((size_t)W * dim);
-            CUDA_TRY(cudaMemcpy(host.data(), points, sizeof(float) * host.size(), cudaMemcpyDeviceToHost));
-            h = host.data();
-        }
         float mn[3] = {0, 0, 0}, mx[3] = {0, 0, 0};
-        for (int a = 0; a < dim; ++a) {
-            float lo = INFINITY, hi = -INFINITY;
-            for (int i = 0; i < W; ++i) {
-                const float x = h[(size_t)i * dim + a];
-                if (std::isfinite(x)) {
-                    lo = std::min(lo, x);
-                    hi = std::max(hi, x);
+        if (points_on_device || W > rtdbs::kChunkMax) {
+            const int rc = device_bbox(e, d_points, points_on_device, mn, mx);
+            if (rc != RTDBS_OK) return rc;
+        } else {
+            for (int a = 0; a < dim; ++a) {
+                float lo = INFINITY, hi = -INFINITY;
+                for (int i = 0; i < W; ++i) {
+                    const float x = points[(size_t)i * dim + a];
+                    if (std::isfinite(x)) {
+                        lo = std::min(lo, x);
+                        hi = std::max(hi, x);
+                    }
                 }
+                if (!(lo <= hi)) lo = hi = 0.0f;
+                mn[a] = lo;
+                mx[a] = hi;
             }
-            if (!(lo <= hi)) lo = hi = 0.0f;
-            mn[a] = lo;
-            mx[a] = hi;
         }
         int rc = engine_geometry(e, mn, mx, true);
         if (rc != RTDBS_OK) return rc;
@@ -563,14 +617,18 @@ int rtdbs_load_window(rtdbs_engine* e, const float* points, int points_on_device
     CUDA_TRY(cudaMemsetAsync(e->v.ctl, 0, sizeof(Ctl), e->stream));
     CUDA_TRY(cudaMemsetAsync(e->v.table[0], 0, sizeof(ulonglong2) * ((size_t)e->v.pmask + 1), e->stream));
     CUDA_TRY(cudaMemsetAsync(e->v.table[1], 0, sizeof(ulonglong2) * ((size_t)e->v.pmask + 1), e->stream));
-    const int C = std::min(W, rtdbs::kChunkMax);
-    View v = e->v;
-    v.chunk = C;  // load chunks tile the slots [0, W)
-    for (int j = 0, off = 0; off < W; ++j, off += C) {
-        const int c = std::min(C, W - off);
-        int rc = copy_in(e, points + (size_t)off * dim, c, points_on_device);
-        if (rc != RTDBS_OK) return rc;
-        CUDA_TRY(rtdbs::launch_chunk_step(v, e->p.precision, j, c, 1, 0, e->stream));
+    if (rtdbs::window_build_fits(e->v)) {
+        CUDA_TRY(rtdbs::launch_window_build(e->v, e->p.precision, d_points, W, 1, e->stream));
+    } else {  // key and slot do not fit one sort word: by chunks
+        const int C = std::min(W, rtdbs::kChunkMax);
+        View v = e->v;
+        v.chunk = C;  // load chunks tile the slots [0, W)
+        for (int j = 0, off = 0; off < W; ++j, off += C) {
+            const int c = std::min(C, W - off);
+            int rc = copy_in(e, points + (size_t)off * dim, c, points_on_device);
+            if (rc != RTDBS_OK) return rc;
+            CUDA_TRY(rtdbs::launch_chunk_step(v, e->p.precision, j, c, 1, 0, e->stream));
+        }
     }
     int rc = fetch_ctl_and_sync(e);
     if (rc != RTDBS_OK) return rc;
@@ -705,12 +763,14 @@ int rtdbs_get_stats(rtdbs_engine* e, rtdbs_stats* s) {
     s->key_bits = e->v.key_bits;
     s->cell_side = e->cell_side;
     s->device_bytes = (int64_t)e->dev_bytes;
-    const int nchunks = (e->p.stride + e->chunk - 1) / e->chunk;
+    const bool whole = e->geometry_ready && !e->pooled && slide_builds_window(e);
+    const int nchunks = whole ? 1 : (e->p.stride + e->chunk - 1) / e->chunk;
     s->chunks_per_slide = nchunks;
     // per chunk 6 kernels, 7 when the sort phase needs a run merge (a chunk
     // of more than one sort run); then link, union, flatten and label (or border)
     int launches = 4;
-    for (int j = 0; j < nchunks; ++j) {
+    if (whole) launches += rtdbs::window_build_launches(e->v);
+    for (int j = 0; j < nchunks && !whole; ++j) {
         const int c = std::min(e->chunk, e->p.stride - j * e->chunk);
         launches += rtdbs::kChunkPhases + (c > rtdbs::kSortRun ? 1 : 0);
     }
@@ -724,7 +784,8 @@ int rtdbs_slide_profiled(rtdbs_engine* e, const float* d_new_points, rtdbs_phase
     DeviceGuard guard(e->device);
     CUDA_TRY(guard.err);
     const int S = e->p.stride, C = e->chunk;
-    const int nchunks = (S + C - 1) / C;
+    const bool whole = slide_builds_window(e);
+    const int nchunks = whole ? 1 : (S + C - 1) / C;
     const int nev = nchunks * rtdbs::kChunkPhases + 4;
     std::vector<cudaEvent_t> ev(nev, nullptr);
     for (auto& x : ev) CUDA_TRY(cudaEventCreate(&x));
@@ -736,7 +797,9 @@ int rtdbs_slide_profiled(rtdbs_engine* e, const float* d_new_points, rtdbs_phase
         for (int j = 0; j < nchunks && rc == RTDBS_OK; ++j) {
             const int c = std::min(C, S - j * C);
             for (int ph = 0; ph < rtdbs::kChunkPhases; ++ph) {
-                cudaError_t ce = rtdbs::launch_phase(ph, e->v, e->p.precision, j, c, 0, j * C, 0, e->stream);
+                cudaError_t ce =
+                    whole ? rtdbs::launch_window_phase(ph, e->v, e->p.precision, e->v.staging, S, 0, e->stream)
+                          : rtdbs::launch_phase(ph, e->v, e->p.precision, j, c, 0, j * C, 0, e->stream);
                 if (ce != cudaSuccess) {
                     rc = fail(RTDBS_ERR_CUDA, "launch failed: %s", cudaGetErrorString(ce));
                     break;
@@ -1148,6 +1211,7 @@ int rtdbs_pool_add_stream(rtdbs_pool* p, const rtdbs_params* params, int32_t* st
     if (rc != RTDBS_OK) return rc;
     // this stream's control block lives in the pool's contiguous array
     e->v.ctl = p->d_ctls + slot;
+    e->pooled = true;
     {
         DeviceGuard guard(p->device);
         if (cudaMemsetAsync(e->v.ctl, 0, sizeof(Ctl), p->stream) != cudaSuccess) {

@@ -82,7 +82,8 @@ struct Ctl {
     int reused;                // cores that joined a reused component this slide
     int reuse_skip;            // slides left without forest reuse (it paid off too little)
     long long last_reused;     // `reused` of the last clustering
-    long long reserved[1];
+    long long kept_from;       // first slide since when every slide kept its chunks' orders
+    long long b_done;          // builds whose table is in place (b, while no build is under way)
 };
 
 // Everything a kernel needs for one stream, passed by value.
@@ -182,6 +183,26 @@ cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, 
 cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int init,
                               int staging_offset, cudaStream_t s, cudaStream_t side = nullptr,
                               cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
+// The grid of all W slots built at once (see the kernels): slots
+// [0, count) while loading (init), else the slide's slots, take the points at
+// `input` (device memory, count = S in a slide).
+cudaError_t launch_window_build(const View& v, int precision, const float* input, int count, int init,
+                                cudaStream_t s);
+cudaError_t launch_window_phase(int phase, const View& v, int precision, const float* input, int count, int init,
+                                cudaStream_t s);
+int window_build_launches(const View& v);
+// Bounding box of n points per axis as order-keeping unsigned keys: minima
+// in box[0..2] (~0: no finite coordinate), maxima in box[3..5] (device).
+cudaError_t launch_bbox(const float* pts, long long n, int dim, unsigned* box, cudaStream_t s);
+inline int slot_bits(int W) {
+    int b = 0;
+    while ((1ll << b) < (long long)W) ++b;
+    return b;
+}
+// Whether key and slot fit one sort word there.
+inline bool window_build_fits(const View& v) {
+    return v.W <= kChunkMax || v.key_bits + slot_bits(v.W) <= 64;
+}
 // fresh_hints: start the union from fresh hints and forest (no reuse), for a
 // clustering of the window as it stands rather than after a slide.
 // outputs_free: an event the label pass (which rewrites label/cid) waits for

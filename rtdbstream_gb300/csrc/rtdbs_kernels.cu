@@ -88,10 +88,10 @@ __device__ __forceinline__ int chunk_base_slot(const View& v, int j, int init) {
 
 // The expiring chunk's (key, slot) order is known from the slide that
 // brought it in (sorder), so its words need no sort: true once every slot of
-// the window arrived by a slide (the first window's load chunks tile the
-// slots differently).  Keys do not change while a point is in the window.
+// the window arrived by a slide that kept its order (a whole-window build
+// keeps none).  Keys do not change while a point is in the window.
 __device__ __forceinline__ bool expired_presorted(const View& v, int init) {
-    return !init && v.sorder != nullptr && v.ctl->slide >= (long long)v.units;
+    return !init && v.sorder != nullptr && v.ctl->slide >= v.ctl->kept_from + (long long)v.units;
 }
 
 // ----------------------------------------------------------------- predicate
@@ -390,6 +390,71 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
     if (e == INT_MIN) s = e = 0;
     rs = s;
     re = e;
+}
+
+// One row of the stencil around a cell, looked up by one lane: kept row
+// `row` of Stencil<DIM, HALF, K> as a range of sorted positions (empty: 0, 0).
+// The first probes of the row's cells are issued together.
+template <int DIM, bool HALF, int K, bool SMALL>
+__device__ __forceinline__ int2 row_range_lane_t(const View& v, const ulonglong2* T, unsigned gen,
+                                                 unsigned long long key, int row) {
+    using St = Stencil<DIM, HALF, K>;
+    using C = typename std::conditional<SMALL, int, long long>::type;  // cell coordinates
+    constexpr int kW = St::kW;
+    const int arow = St::kFirst + row;
+    const bool centre = HALF && row == 0;  // its cells below the home cell are not kept
+    const int s0 = v.shift[0], s1 = v.shift[1];
+    C q0 = (C)(key >> s0), q1 = (C)((key >> s1) & ((1ull << (s0 - s1)) - 1ull)), q2 = (C)(key & ((1ull << s1) - 1ull));
+    if (DIM == 2) {
+        q0 += arow - K;
+    } else if (DIM == 3) {
+        q0 += arow / kW - K;
+        q1 += arow % kW - K;
+    }
+    const C e0 = (C)v.ext[0], e1 = (C)v.ext[1], e2 = (C)v.ext[2];
+    C& ql = DIM == 1 ? q0 : (DIM == 2 ? q1 : q2);  // the axis along the row
+    const C el = DIM == 1 ? e0 : (DIM == 2 ? e1 : e2);
+    const bool in = (DIM == 1 || (q0 >= 0 && q0 < e0)) && (DIM < 3 || (q1 >= 0 && q1 < e1));
+    if (!in) return make_int2(0, 0);
+    const C mid = ql;
+    ql = 0;
+    const unsigned long long rowkey =
+        ((unsigned long long)q0 << s0) | ((unsigned long long)q1 << s1) | (unsigned long long)q2;
+    const int sl = DIM == 1 ? s0 : (DIM == 2 ? s1 : 0);
+    const unsigned long long gtag = (unsigned long long)gen << kKeyBitsMax;
+    ulonglong2 e[kW];
+    unsigned home[kW];
+#pragma unroll
+    for (int k = 0; k < kW; ++k) {
+        const C q = mid + (k - K);
+        e[k].x = 0ull;  // no generation
+        home[k] = 0;
+        if (q >= 0 && q < el && !(centre && k < K)) {
+            const unsigned long long nk = rowkey | ((unsigned long long)q << sl);
+            home[k] = SMALL ? table_home32((unsigned)nk, v.pbits) : table_home(nk, v.pbits);
+            e[k] = T[home[k]];
+        }
+    }
+    int rs = INT_MAX, re = 0;
+#pragma unroll
+    for (int k = 0; k < kW; ++k) {
+        if ((e[k].x >> kKeyBitsMax) != gen) continue;  // out of the grid, or an empty or stale slot
+        const unsigned long long tag = gtag | rowkey | ((unsigned long long)(mid + (k - K)) << sl);
+        const int2 c = e[k].x == tag ? make_int2((int)(unsigned)e[k].y, (int)(unsigned)(e[k].y >> 32))
+                                     : table_find_at(T, v.pmask, (home[k] + 1) & v.pmask, tag);
+        if (c.y > c.x) {
+            rs = min(rs, c.x);
+            re = max(re, c.y);
+        }
+    }
+    return re > 0 ? make_int2(rs, re) : make_int2(0, 0);
+}
+
+template <int DIM, bool HALF, int K>
+__device__ __forceinline__ int2 row_range_lane(const View& v, const ulonglong2* T, unsigned gen,
+                                               unsigned long long key, int row) {
+    if (v.key_bits <= 31) return row_range_lane_t<DIM, HALF, K, true>(v, T, gen, key, row);
+    return row_range_lane_t<DIM, HALF, K, false>(v, T, gen, key, row);
 }
 
 // The group's row ranges (group lanes 0..ROWS-1), clipped below at `lo`,
@@ -1237,6 +1302,7 @@ __device__ __forceinline__ void build_body(const View& v, int bx, BuildSmem& sm,
     }
     __syncthreads();
     if (threadIdx.x == 0 && bcells) atomicAdd(&v.ctl->ncells, bcells);
+    if (bx == 0 && threadIdx.x == 0) v.ctl->b_done = b;  // not read here
     if (valid && (first || (lane & (ip - 1)) == 0)) {
         const int rank = __popc(starts & lanemask_lt(lane));
         const unsigned above = starts & ~((2u << lane) - 1u);
@@ -1371,6 +1437,397 @@ __global__ void __launch_bounds__(256, 5) k_incr(View v, int j, int c, int init)
     incr_body<MODE, DK>(v, j, c, init, blockIdx.x, sm);
 }
 
+// ------------------------------------------------------ whole-window build
+// The first window, and a slide that replaces a large share of the window,
+// build the grid from all W slots at once: one pass writes every slot's sort
+// word, a radix sort orders them, one pass lays the window out in that order,
+// the cell table is built once and every point's neighbours are counted once
+// (k_count), instead of W / 16384 chunk steps that each rewrite the window.
+// A 1M-point walker window: load 9.9 -> 0.6 ms (sort 97 us, count 349 us; the
+// box of the points is taken on the device, not in a host loop over a copy);
+// 48k points replaced per slide: 327 -> 137 us for the grid.
+// Words are key << ob | slot (ob bits for the slots; the host takes the chunk
+// steps where key and slot do not fit 64 bits).  The sort alternates between
+// the two key buffers and ends in the one that the window's layout does not
+// take; the counters of its tiles lie in that side's counts.
+
+constexpr int kRadThreads = 512;
+constexpr int kRadItems = 8;                           // words per thread
+constexpr int kRadTile = kRadThreads * kRadItems;      // words per block
+constexpr int kRadWarps = kRadThreads / 32;
+// Up to this many tiles every scatter block sums the tiles' counters itself
+// (12 tiles: sort 52 -> 44 us without the scan's launches); above, a scan
+// kernel does it once.
+constexpr int kRadInline = 64;
+
+// Input buffer of radix pass `pass` of `passes` (pass == passes: the sorted words).
+__device__ __forceinline__ unsigned long long* rad_buffer(const View& v, int pass, int passes) {
+    const int cur = (int)(v.ctl->b & 1);
+    return v.skey[((passes - pass) & 1) ? cur : cur ^ 1];
+}
+
+// Slots [base, base + count) take the new points (base by the slide's place
+// in the ring, 0 while loading); every slot's sort word goes to the first
+// pass's input (chunk < 0), or the new points' chunk words to nsort.
+__global__ void k_ingest_all(View v, const float* input, int count, int init, int ob, int passes) {
+    const long long b = v.ctl->b_done + 1;  // this build (k_build keeps b_done)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        v.ctl->b = b;
+        if (!init) {
+            v.ctl->prev_ok = 0;     // no forest reuse in this clustering,
+            v.ctl->reuse_skip = 2;  // no roots kept for the next,
+            v.ctl->kept_from = v.ctl->slide + 1;  // nor this slide's order
+        }
+    }
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= v.W) return;
+    const int base = chunk_base_slot(v, 0, init);
+    unsigned long long key;
+    if (s >= base && s < base + count) {
+        const float* p = input + (size_t)(s - base) * v.dim;
+        const float x = p[0];
+        const float y = v.dim > 1 ? p[1] : 0.0f;
+        const float z = v.dim > 2 ? p[2] : 0.0f;
+        v.ring[s] = make_float4(x, y, z, __int_as_float(s));
+        key = cell_key(v, x, y, z);
+        v.kslot[s] = key;
+    } else {
+        key = v.kslot[s];
+    }
+    const unsigned long long word = (key << ob) | (unsigned long long)s;
+    if (passes < 0) {
+        v.nsort[s] = word;
+    } else {
+        const int cur = (int)(b & 1);
+        v.skey[(passes & 1) ? cur : cur ^ 1][s] = word;
+    }
+}
+
+__global__ void __launch_bounds__(kRadThreads) k_rad_hist(View v, int pass, int passes, int shift) {
+    __shared__ int hist[256];
+    const unsigned long long* in = rad_buffer(v, pass, passes);
+    int* counts = v.scnt[(v.ctl->b & 1) ^ 1];
+    if (threadIdx.x < 256) hist[threadIdx.x] = 0;
+    __syncthreads();
+    unsigned long long w[kRadItems];
+#pragma unroll
+    for (int k = 0; k < kRadItems; ++k) {
+        const int i = blockIdx.x * kRadTile + k * kRadThreads + threadIdx.x;
+        w[k] = i < v.W ? in[i] : 0ull;
+    }
+#pragma unroll
+    for (int k = 0; k < kRadItems; ++k) {
+        const int i = blockIdx.x * kRadTile + k * kRadThreads + threadIdx.x;
+        if (i < v.W) atomicAdd(&hist[(unsigned)(w[k] >> shift) & 255u], 1);
+    }
+    __syncthreads();
+    if (threadIdx.x < 256) counts[blockIdx.x * 256 + threadIdx.x] = hist[threadIdx.x];
+}
+
+// Exclusive scan over the tiles of 32 digits per block (a warp's lanes side by
+// side), 8 warps on an eighth of the tiles each; the digits' totals follow
+// the tiles' counters.  Only where there are many tiles (kRadInline).
+__global__ void __launch_bounds__(256) k_rad_scan(View v, int ntiles) {
+    __shared__ int part[8][32];
+    int* counts = v.scnt[(v.ctl->b & 1) ^ 1];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = blockIdx.x * 32 + lane;
+    const int per = (ntiles + 7) / 8, t0 = min(w * per, ntiles), t1 = min(t0 + per, ntiles);
+    int sum = 0;
+#pragma unroll 8
+    for (int t = t0; t < t1; ++t) sum += counts[t * 256 + d];
+    part[w][lane] = sum;
+    __syncthreads();
+    int at = 0;
+    for (int k = 0; k < w; ++k) at += part[k][lane];
+#pragma unroll 8
+    for (int t = t0; t < t1; ++t) {
+        const int x = counts[t * 256 + d];
+        counts[t * 256 + d] = at;
+        at += x;
+    }
+    if (w == 7) counts[(size_t)256 * ntiles + d] = at;
+}
+
+// Stable scatter of one tile by its digit: each warp ranks its 256
+// consecutive words in order (lanes with equal digits from eight ballots),
+// warp counters are scanned per digit, and every word goes to its place.
+__global__ void __launch_bounds__(kRadThreads) k_rad_scatter(View v, int pass, int passes, int shift, int scanned) {
+    __shared__ int cnt[kRadWarps][256];
+    __shared__ int wsum[8];
+    const unsigned long long* in = rad_buffer(v, pass, passes);
+    unsigned long long* out = rad_buffer(v, pass + 1, passes);
+    const int* counts = v.scnt[(v.ctl->b & 1) ^ 1];
+    const int ntiles = gridDim.x, tile = blockIdx.x;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int k = threadIdx.x; k < kRadWarps * 256; k += kRadThreads) (&cnt[0][0])[k] = 0;
+    unsigned long long it[kRadItems];
+    int rank[kRadItems];
+    const int i0 = tile * kRadTile + w * (32 * kRadItems) + lane;
+#pragma unroll
+    for (int k = 0; k < kRadItems; ++k) it[k] = i0 + 32 * k < v.W ? in[i0 + 32 * k] : ~0ull;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kRadItems; ++k) {
+        const bool has = i0 + 32 * k < v.W;
+        const unsigned d = (unsigned)(it[k] >> shift) & 255u;
+        unsigned peers = __ballot_sync(kFull, has);
+#pragma unroll
+        for (int bit = 0; bit < 8; ++bit) {
+            const unsigned bm = __ballot_sync(kFull, (d >> bit) & 1u);
+            peers &= ((d >> bit) & 1u) ? bm : ~bm;
+        }
+        const int before = cnt[w][d];
+        __syncwarp();
+        rank[k] = before + __popc(peers & lanemask_lt(lane));
+        if (has && !(peers & lanemask_lt(lane))) cnt[w][d] = before + __popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    // digit totals -> digit bases, then every warp's first place per digit
+    int total = 0, incl = 0, mine = 0;  // the digit's words: all, running, before this tile
+    if (threadIdx.x < 256) {
+        if (scanned) {
+            total = counts[(size_t)256 * ntiles + threadIdx.x];
+            mine = counts[tile * 256 + threadIdx.x];
+        } else {
+#pragma unroll 8
+            for (int t = 0; t < ntiles; ++t) {
+                const int x = counts[t * 256 + threadIdx.x];
+                total += x;
+                mine += t < tile ? x : 0;
+            }
+        }
+        incl = total;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += y;
+        }
+        if (lane == 31) wsum[w] = incl;
+    }
+    __syncthreads();
+    if (threadIdx.x < 256) {
+        int at = incl - total + mine;
+        for (int k = 0; k < w; ++k) at += wsum[k];
+        for (int k = 0; k < kRadWarps; ++k) {
+            const int x = cnt[k][threadIdx.x];
+            cnt[k][threadIdx.x] = at;
+            at += x;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kRadItems; ++k) {
+        if (i0 + 32 * k >= v.W) continue;
+        const int o = cnt[w][(unsigned)(it[k] >> shift) & 255u] + rank[k];
+        if (o >= 0 && o < v.W)
+            out[o] = it[k];
+        else
+            atomicOr(&v.ctl->err, kErrChunk);
+    }
+}
+
+// The window laid out in the order of its sorted words (counts and hints
+// follow in k_count), a fresh forest, and the build's counters reset.
+__global__ void k_fill(View v, int ob, int passes) {
+    const long long b = v.ctl->b;
+    const int cur = (int)(b & 1);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        v.ctl->nocc[cur] = v.W;
+        v.ctl->nitems = 0;
+        v.ctl->ncells = 0;
+        v.ctl->union_next = 0;
+        v.ctl->label_next = 0;
+    }
+    // table generations wrap every kGenMod builds of a table, as in the merge
+    if (b >= 2 && ((b >> 1) % (long long)kGenMod) == 0) {
+        ulonglong2* T = v.table[cur];
+        for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i <= v.pmask; i += gridDim.x * blockDim.x)
+            T[i] = make_ulonglong2(0ull, 0ull);
+    }
+    const int o = blockIdx.x * blockDim.x + threadIdx.x;
+    if (o >= v.W) return;
+    const unsigned long long word = passes < 0 ? v.nword[o] : v.skey[cur ^ 1][o];
+    const int slot = (int)(word & ((1ull << ob) - 1ull));
+    if (slot >= v.W) {
+        atomicOr(&v.ctl->err, kErrChunk);
+        return;
+    }
+    v.skey[cur][o] = word >> ob;
+    v.spt[cur][o] = v.ring[slot];
+    v.parent[slot] = slot;
+}
+
+// Neighbour counts, start hints and neighbour lists of every point, from one
+// scan of the grid.  As in the union, a warp takes a block of consecutive
+// sorted positions, looks up the stencil rows of all its cells (the whole
+// stencil here) lane by lane and walks them as one candidate stream; every
+// lane tests its candidate against the points of its own cell run, the runs'
+// points in step, so one vote counts a whole chunk for each of them.  Bound by
+// instruction issue (one test, vote and count per candidate chunk and home
+// point); against one whole-stencil query per point with atomics on its
+// neighbours, as the chunk steps count: 1M walkers 1.8 ms -> 0.35 ms.
+constexpr int kCountThreads = 128;
+
+template <int DIM, int K>
+struct CountShape {
+    static constexpr int kRows = Stencil<DIM, false, K>::kRows;
+    static constexpr int kBlock = kRows > 9 ? 16 : 32;  // positions per warp (shared memory)
+    static constexpr int kTasks = kBlock * kRows;
+};
+
+template <int DIM, int K>
+struct CountSmem {
+    using C = CountShape<DIM, K>;
+    static constexpr int kWarps = kCountThreads / 32;
+    float4 pt[kWarps][C::kBlock];  // home points
+    unsigned long long skey[kWarps][C::kBlock];
+    int first[kWarps][C::kBlock + 1];  // first home point of a run
+    int sbeg[kWarps][C::kBlock + 1];   // first candidate of a run
+    int cnt[kWarps][C::kBlock];        // neighbours found
+    int buf[kWarps][C::kBlock * kListCap];
+    int tstart[kWarps][C::kTasks];
+    int tpre[kWarps][C::kTasks + 1];
+    unsigned char tseg[kWarps][C::kTasks];
+};
+
+__device__ __forceinline__ unsigned lane_range(int lo, int hi) {  // lanes [lo, hi), clamped
+    const unsigned up = hi >= 32 ? kFull : (hi <= 0 ? 0u : lanemask_lt(hi));
+    return up & ~(lo >= 32 ? kFull : (lo <= 0 ? 0u : lanemask_lt(lo)));
+}
+
+template <int MODE, int DK>
+__global__ void __launch_bounds__(kCountThreads) k_count(View v) {
+    constexpr int DIM = DK & 3, K = (DK >> 2) + 1;
+    using C = CountShape<DIM, K>;
+    constexpr int R = C::kRows, P = C::kBlock;
+    __shared__ CountSmem<DIM, K> sm;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const long long b = v.ctl->b;
+    const int cur = (int)(b & 1);
+    const unsigned gen = gen_of_build(b);
+    const int n = v.ctl->nocc[cur];
+    const int start = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * P;
+    if (start >= n) return;
+    const int m = min(P, n - start);
+    const bool hv = lane < m;
+    float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+    unsigned long long key = 0;
+    if (hv) {
+        h = v.spt[cur][start + lane];
+        key = v.skey[cur][start + lane];
+    }
+    // runs of one cell
+    const unsigned long long kprev = __shfl_up_sync(kFull, key, 1);
+    const unsigned leaders = __ballot_sync(kFull, hv && (lane == 0 || kprev != key));
+    const int ns = __popc(leaders);
+    const int run = __popc(leaders & (lanemask_lt(lane) | (1u << lane))) - 1;
+    if (hv) {
+        sm.pt[wib][lane] = h;
+        sm.cnt[wib][lane] = 0;
+        if ((leaders >> lane) & 1u) {
+            sm.skey[wib][run] = key;
+            sm.first[wib][run] = lane;
+        }
+    }
+    if (lane == 0) sm.first[wib][ns] = m;
+    __syncwarp();
+    int* tstart = sm.tstart[wib];
+    int* tpre = sm.tpre[wib];
+    unsigned char* tseg = sm.tseg[wib];
+    int nt = 0, total = 0;
+    for (int t0 = 0; t0 < ns * R; t0 += 32) {
+        const int t = t0 + lane, seg = t / R;
+        int a = 0, len = 0;
+        if (t < ns * R) {
+            const int2 rr = row_range_lane<DIM, false, K>(v, v.table[cur], gen, sm.skey[wib][seg], t - seg * R);
+            a = rr.x;
+            len = rr.y - rr.x;
+        }
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += x;
+        }
+        if (t < ns * R && t == seg * R) sm.sbeg[wib][seg] = total + incl - len;
+        const unsigned some = __ballot_sync(kFull, len > 0);
+        if (len > 0) {
+            const int at = nt + __popc(some & lanemask_lt(lane));
+            tstart[at] = a;
+            tpre[at] = total + incl - len;
+            tseg[at] = (unsigned char)seg;
+        }
+        nt += __popc(some);
+        total += __shfl_sync(kFull, incl, 31);
+    }
+    if (lane == 0) {
+        tpre[nt] = total;
+        sm.sbeg[wib][ns] = total;
+    }
+    __syncwarp();
+    const int ord = hv ? lane - sm.first[wib][run] : -1;
+    const int hb = hv ? sm.sbeg[wib][run] : 0, he = hv ? sm.sbeg[wib][run + 1] : 0;
+    const int cap = max(v.list_cap, 0);
+    const float4* spt = v.spt[cur];
+    Tally tally;
+    int r = 0, count = 0;
+    for (int base = 0; base < total; base += 32) {
+        const int idx = base + lane;
+        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+        int f = 0, len = 0;
+        unsigned mine = 0;  // the chunk's candidates of the lane's run
+        if (idx < total) {
+            while (idx >= tpre[r + 1]) ++r;
+            q = spt[tstart[r] + idx - tpre[r]];
+            const int s = tseg[r];
+            f = sm.first[wib][s];
+            len = sm.first[wib][s + 1] - f;
+            mine = lane_range(sm.sbeg[wib][s] - base, sm.sbeg[wib][s + 1] - base) & lanemask_lt(lane);
+        }
+        const unsigned home = lane_range(hb - base, he - base);  // the chunk's candidates of the home point
+        const int steps = (int)__reduce_max_sync(kFull, (unsigned)len);
+        for (int t = 0; t < steps; ++t) {
+            bool nb = false;
+            if (t < len) {
+                const float4 hp = sm.pt[wib][f + t];
+                nb = slot_of(hp) != slot_of(q) && is_nbr<MODE, DIM>(v, hp, q, tally);
+            }
+            const unsigned hits = __ballot_sync(kFull, nb);
+            if (cap > 0) {
+                if (nb) {
+                    const int k = sm.cnt[wib][f + t] + __popc(hits & mine);
+                    if (k < cap) sm.buf[wib][(f + t) * kListCap + k] = slot_of(q);
+                }
+                __syncwarp();
+                if (t == ord) sm.cnt[wib][lane] = count + __popc(hits & home);
+            }
+            if (t == ord) count += __popc(hits & home);
+        }
+        __syncwarp();
+    }
+    __syncwarp();
+    if (hv) {
+        const int slot = slot_of(h), all = count + 1;  // the point itself included
+        const bool core = all >= v.min_pts;
+        v.scnt[cur][start + lane] = all;
+        v.sroot[start + lane] = core ? slot : -1;
+        if (v.list_cap >= 0) {
+            v.ntrack[slot] = core ? 0 : 1;
+            if (!core) {
+                int4* L = reinterpret_cast<int4*>(v.nlist + (size_t)slot * v.list_stride);
+                const int* bf = sm.buf[wib] + lane * kListCap;
+                for (int k = 0; k < v.list_stride; k += 4)
+                    L[k >> 2] = make_int4(k < count ? bf[k] : -1, k + 1 < count ? bf[k + 1] : -1,
+                                          k + 2 < count ? bf[k + 2] : -1, k + 3 < count ? bf[k + 3] : -1);
+            }
+        }
+    }
+    const unsigned most = __reduce_max_sync(kFull, (unsigned)max(he - hb - 1, 0));
+    if (lane == 0 && most) atomicMax(&v.ctl->qmax[wib & 7], (int)most);
+    flush_stats(v, tally, 0, lane, 0);
+}
+
 // Fresh start hints without reuse (-1 for a non-core position, its own
 // slot for a core) and a fresh forest, for a clustering of the window as it
 // stands (rtdbs_cluster), whose hints may hold the last union's roots.
@@ -1490,71 +1947,6 @@ __device__ __forceinline__ int work_grab(const View& v, bool pooled) {
 // about 8 cell runs (2 blocks: walkers 168 -> 178 us, trajectories 79 -> 109);
 // the stream's setting counts cell runs.
 __device__ __forceinline__ int union_grab(const View& v) { return max(1, v.grab >> 4); }
-
-// One row of the stencil around a cell, looked up by one lane: kept row
-// `row` of Stencil<DIM, HALF, K> as a range of sorted positions (empty: 0, 0).
-// The first probes of the row's cells are issued together.
-template <int DIM, bool HALF, int K, bool SMALL>
-__device__ __forceinline__ int2 row_range_lane_t(const View& v, const ulonglong2* T, unsigned gen,
-                                                 unsigned long long key, int row) {
-    using St = Stencil<DIM, HALF, K>;
-    using C = typename std::conditional<SMALL, int, long long>::type;  // cell coordinates
-    constexpr int kW = St::kW;
-    const int arow = St::kFirst + row;
-    const bool centre = HALF && row == 0;  // its cells below the home cell are not kept
-    const int s0 = v.shift[0], s1 = v.shift[1];
-    C q0 = (C)(key >> s0), q1 = (C)((key >> s1) & ((1ull << (s0 - s1)) - 1ull)), q2 = (C)(key & ((1ull << s1) - 1ull));
-    if (DIM == 2) {
-        q0 += arow - K;
-    } else if (DIM == 3) {
-        q0 += arow / kW - K;
-        q1 += arow % kW - K;
-    }
-    const C e0 = (C)v.ext[0], e1 = (C)v.ext[1], e2 = (C)v.ext[2];
-    C& ql = DIM == 1 ? q0 : (DIM == 2 ? q1 : q2);  // the axis along the row
-    const C el = DIM == 1 ? e0 : (DIM == 2 ? e1 : e2);
-    const bool in = (DIM == 1 || (q0 >= 0 && q0 < e0)) && (DIM < 3 || (q1 >= 0 && q1 < e1));
-    if (!in) return make_int2(0, 0);
-    const C mid = ql;
-    ql = 0;
-    const unsigned long long rowkey =
-        ((unsigned long long)q0 << s0) | ((unsigned long long)q1 << s1) | (unsigned long long)q2;
-    const int sl = DIM == 1 ? s0 : (DIM == 2 ? s1 : 0);
-    const unsigned long long gtag = (unsigned long long)gen << kKeyBitsMax;
-    ulonglong2 e[kW];
-    unsigned home[kW];
-#pragma unroll
-    for (int k = 0; k < kW; ++k) {
-        const C q = mid + (k - K);
-        e[k].x = 0ull;  // no generation
-        home[k] = 0;
-        if (q >= 0 && q < el && !(centre && k < K)) {
-            const unsigned long long nk = rowkey | ((unsigned long long)q << sl);
-            home[k] = SMALL ? table_home32((unsigned)nk, v.pbits) : table_home(nk, v.pbits);
-            e[k] = T[home[k]];
-        }
-    }
-    int rs = INT_MAX, re = 0;
-#pragma unroll
-    for (int k = 0; k < kW; ++k) {
-        if ((e[k].x >> kKeyBitsMax) != gen) continue;  // out of the grid, or an empty or stale slot
-        const unsigned long long tag = gtag | rowkey | ((unsigned long long)(mid + (k - K)) << sl);
-        const int2 c = e[k].x == tag ? make_int2((int)(unsigned)e[k].y, (int)(unsigned)(e[k].y >> 32))
-                                     : table_find_at(T, v.pmask, (home[k] + 1) & v.pmask, tag);
-        if (c.y > c.x) {
-            rs = min(rs, c.x);
-            re = max(re, c.y);
-        }
-    }
-    return re > 0 ? make_int2(rs, re) : make_int2(0, 0);
-}
-
-template <int DIM, bool HALF, int K>
-__device__ __forceinline__ int2 row_range_lane(const View& v, const ulonglong2* T, unsigned gen,
-                                               unsigned long long key, int row) {
-    if (v.key_bits <= 31) return row_range_lane_t<DIM, HALF, K, true>(v, T, gen, key, row);
-    return row_range_lane_t<DIM, HALF, K, false>(v, T, gen, key, row);
-}
 
 // Union of every core-core neighbour pair.  A warp takes a block of P
 // consecutive sorted positions (View::block_pts), whose cores fall into runs
@@ -2263,6 +2655,100 @@ cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int in
         }
     }
     return cudaSuccess;
+}
+
+cudaError_t launch_window_phase(int phase, const View& v, int precision, const float* input, int count, int init,
+                                cudaStream_t s) {
+    const int grid = (v.W + 255) / 256;
+    const bool chunk = v.W <= kChunkMax;  // one chunk: its runs are sorted and ranked on chip
+    const int ob = chunk ? kOffBits : slot_bits(v.W);
+    const int passes = chunk ? -1 : (v.key_bits + 7) / 8;
+    switch (phase) {
+        case kPhaseIngest:
+            k_ingest_all<<<grid, 256, 0, s>>>(v, input, count, init, ob, passes);
+            break;
+        case kPhaseSort:
+            if (chunk) {
+                const int runs = (v.W + kSortRun - 1) / kSortRun;
+                k_sort<<<dim3(runs, 1), kSortRun, 0, s>>>(v, 0, v.W, 1, runs == 1);
+                if (runs == 1) break;
+                ensure_runmerge_smem();
+                k_runmerge<<<dim3(runs, 1), kSortRun, sizeof(unsigned long long) * v.W, s>>>(v, 0, v.W, 1);
+                break;
+            }
+            for (int p = 0; p < passes; ++p) {
+                const int tiles = (v.W + kRadTile - 1) / kRadTile;
+                k_rad_hist<<<tiles, kRadThreads, 0, s>>>(v, p, passes, ob + 8 * p);
+                const int scanned = tiles > kRadInline;
+                if (scanned) k_rad_scan<<<8, 256, 0, s>>>(v, tiles);
+                k_rad_scatter<<<tiles, kRadThreads, 0, s>>>(v, p, passes, ob + 8 * p, scanned);
+            }
+            break;
+        case kPhaseDecrement: break;  // counted afresh
+        case kPhaseMerge:
+            k_fill<<<grid, 256, 0, s>>>(v, ob, passes);
+            break;
+        case kPhaseBuild:
+            k_build<<<(v.W + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, s>>>(v);
+            break;
+        case kPhaseIncrement: {
+            const int block = v.dim == 3 && v.cell_mult == 2 ? 16 : 32;  // positions per warp (CountShape)
+            const int per = block * (kCountThreads / 32);
+            RTDBS_DISPATCH(precision, dk_of(v), k_count, (v.W + per - 1) / per, kCountThreads, s, v);
+            break;
+        }
+        default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_window_build(const View& v, int precision, const float* input, int count, int init,
+                                cudaStream_t s) {
+    if (!window_build_fits(v)) return cudaErrorInvalidValue;
+    cudaError_t e = cudaSuccess;
+    for (int ph = 0; ph < kChunkPhases && e == cudaSuccess; ++ph)
+        e = launch_window_phase(ph, v, precision, input, count, init, s);
+    return e;
+}
+
+int window_build_launches(const View& v) {
+    const int per = (v.W + kRadTile - 1) / kRadTile > kRadInline ? 3 : 2;
+    const int sorts = v.W > kChunkMax ? per * ((v.key_bits + 7) / 8) : (v.W > kSortRun ? 2 : 1);
+    return 4 + sorts;
+}
+
+// Finite bounding box of n points per axis, as order-keeping unsigned keys
+// (box[0..2] minima from ~0, box[3..5] maxima from 0).
+__global__ void k_bbox(const float* pts, long long n, int dim, unsigned* box) {
+    const int lane = threadIdx.x & 31;
+    unsigned lo[3] = {~0u, ~0u, ~0u}, hi[3] = {0u, 0u, 0u};
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+        for (int a = 0; a < 3; ++a) {
+            if (a >= dim) break;
+            const float x = pts[i * dim + a];
+            if (!isfinite(x)) continue;
+            const unsigned u = __float_as_uint(x);
+            const unsigned k = (u >> 31) ? ~u : u | 0x80000000u;
+            lo[a] = min(lo[a], k);
+            hi[a] = max(hi[a], k);
+        }
+    for (int a = 0; a < 3; ++a) {
+        if (a >= dim) break;
+        const unsigned l = __reduce_min_sync(kFull, lo[a]), h = __reduce_max_sync(kFull, hi[a]);
+        if (lane == 0 && l <= h) {
+            atomicMin(&box[a], l);
+            atomicMax(&box[3 + a], h);
+        }
+    }
+}
+
+cudaError_t launch_bbox(const float* pts, long long n, int dim, unsigned* box, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(box, 0xff, 3 * sizeof(unsigned), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(box + 3, 0, 3 * sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+    const int sms = g_num_sms > 0 ? g_num_sms : 152;
+    k_bbox<<<(int)max(1ll, min((long long)sms * 4, (n + 255) / 256)), 256, 0, s>>>(pts, n, dim, box);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_cluster(const View& v, int precision, int advance, cudaStream_t s, bool fresh_hints,
