@@ -1443,7 +1443,7 @@ __global__ void __launch_bounds__(256, 5) k_incr(View v, int j, int c, int init)
 // word, a radix sort orders them, one pass lays the window out in that order,
 // the cell table is built once and every point's neighbours are counted once
 // (k_count), instead of W / 16384 chunk steps that each rewrite the window.
-// A 1M-point walker window: load 9.9 -> 0.6 ms (sort 97 us, count 349 us; the
+// A 1M-point walker window: load 9.9 -> 0.5 ms (sort 97 us, count 276 us; the
 // box of the points is taken on the device, not in a host loop over a copy);
 // 48k points replaced per slide: 327 -> 137 us for the grid.
 // Words are key << ob | slot (ob bits for the slots; the host takes the chunk
@@ -1663,10 +1663,13 @@ __global__ void k_fill(View v, int ob, int passes) {
 // sorted positions, looks up the stencil rows of all its cells (the whole
 // stencil here) lane by lane and walks them as one candidate stream; every
 // lane tests its candidate against the points of its own cell run, the runs'
-// points in step, so one vote counts a whole chunk for each of them.  Bound by
-// instruction issue (one test, vote and count per candidate chunk and home
-// point); against one whole-stencil query per point with atomics on its
-// neighbours, as the chunk steps count: 1M walkers 1.8 ms -> 0.35 ms.
+// points in step, two at a time, so one vote counts a whole chunk for each of
+// them.  The lists of the few non-core points with neighbours are collected
+// from their candidates afterwards (kept while counting, they took a
+// rank and a store per test: 1M walkers 349 us against 276, 200k dense
+// trajectories 263 against 136).  Bound by instruction issue; against one
+// whole-stencil query per point with atomics on its neighbours, as the chunk
+// steps count, 1M walkers take 0.28 ms instead of 1.8.
 constexpr int kCountThreads = 128;
 
 template <int DIM, int K>
@@ -1684,8 +1687,7 @@ struct CountSmem {
     unsigned long long skey[kWarps][C::kBlock];
     int first[kWarps][C::kBlock + 1];  // first home point of a run
     int sbeg[kWarps][C::kBlock + 1];   // first candidate of a run
-    int cnt[kWarps][C::kBlock];        // neighbours found
-    int buf[kWarps][C::kBlock * kListCap];
+    int tbeg[kWarps][C::kBlock];       // first stored row of a run
     int tstart[kWarps][C::kTasks];
     int tpre[kWarps][C::kTasks + 1];
     unsigned char tseg[kWarps][C::kTasks];
@@ -1697,10 +1699,10 @@ __device__ __forceinline__ unsigned lane_range(int lo, int hi) {  // lanes [lo, 
 }
 
 template <int MODE, int DK>
-__global__ void __launch_bounds__(kCountThreads) k_count(View v) {
+__global__ void __launch_bounds__(kCountThreads, 8) k_count(View v, int P) {
     constexpr int DIM = DK & 3, K = (DK >> 2) + 1;
     using C = CountShape<DIM, K>;
-    constexpr int R = C::kRows, P = C::kBlock;
+    constexpr int R = C::kRows;
     __shared__ CountSmem<DIM, K> sm;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const long long b = v.ctl->b;
@@ -1724,7 +1726,6 @@ __global__ void __launch_bounds__(kCountThreads) k_count(View v) {
     const int run = __popc(leaders & (lanemask_lt(lane) | (1u << lane))) - 1;
     if (hv) {
         sm.pt[wib][lane] = h;
-        sm.cnt[wib][lane] = 0;
         if ((leaders >> lane) & 1u) {
             sm.skey[wib][run] = key;
             sm.first[wib][run] = lane;
@@ -1750,8 +1751,11 @@ __global__ void __launch_bounds__(kCountThreads) k_count(View v) {
             const int x = __shfl_up_sync(kFull, incl, o);
             if (lane >= o) incl += x;
         }
-        if (t < ns * R && t == seg * R) sm.sbeg[wib][seg] = total + incl - len;
         const unsigned some = __ballot_sync(kFull, len > 0);
+        if (t < ns * R && t == seg * R) {
+            sm.sbeg[wib][seg] = total + incl - len;
+            sm.tbeg[wib][seg] = nt + __popc(some & lanemask_lt(lane));
+        }
         if (len > 0) {
             const int at = nt + __popc(some & lanemask_lt(lane));
             tstart[at] = a;
@@ -1768,7 +1772,6 @@ __global__ void __launch_bounds__(kCountThreads) k_count(View v) {
     __syncwarp();
     const int ord = hv ? lane - sm.first[wib][run] : -1;
     const int hb = hv ? sm.sbeg[wib][run] : 0, he = hv ? sm.sbeg[wib][run + 1] : 0;
-    const int cap = max(v.list_cap, 0);
     const float4* spt = v.spt[cur];
     Tally tally;
     int r = 0, count = 0;
@@ -1776,50 +1779,67 @@ __global__ void __launch_bounds__(kCountThreads) k_count(View v) {
         const int idx = base + lane;
         float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
         int f = 0, len = 0;
-        unsigned mine = 0;  // the chunk's candidates of the lane's run
         if (idx < total) {
             while (idx >= tpre[r + 1]) ++r;
             q = spt[tstart[r] + idx - tpre[r]];
             const int s = tseg[r];
             f = sm.first[wib][s];
             len = sm.first[wib][s + 1] - f;
-            mine = lane_range(sm.sbeg[wib][s] - base, sm.sbeg[wib][s + 1] - base) & lanemask_lt(lane);
         }
         const unsigned home = lane_range(hb - base, he - base);  // the chunk's candidates of the home point
         const int steps = (int)__reduce_max_sync(kFull, (unsigned)len);
-        for (int t = 0; t < steps; ++t) {
-            bool nb = false;
+        for (int t = 0; t < steps; t += 2) {  // two home points a step
+            bool n0 = false, n1 = false;
             if (t < len) {
-                const float4 hp = sm.pt[wib][f + t];
-                nb = slot_of(hp) != slot_of(q) && is_nbr<MODE, DIM>(v, hp, q, tally);
+                const float4 h0 = sm.pt[wib][f + t], h1 = sm.pt[wib][f + min(t + 1, len - 1)];
+                float d0, d1;
+                sqdist32x2<DIM>(q, h0, h1, d0, d1);
+                n0 = slot_of(h0) != slot_of(q) && nbr_decide<MODE, DIM>(v, d0, h0, q, tally);
+                n1 = t + 1 < len && slot_of(h1) != slot_of(q) && nbr_decide<MODE, DIM>(v, d1, h1, q, tally);
             }
-            const unsigned hits = __ballot_sync(kFull, nb);
-            if (cap > 0) {
-                if (nb) {
-                    const int k = sm.cnt[wib][f + t] + __popc(hits & mine);
-                    if (k < cap) sm.buf[wib][(f + t) * kListCap + k] = slot_of(q);
-                }
-                __syncwarp();
-                if (t == ord) sm.cnt[wib][lane] = count + __popc(hits & home);
-            }
-            if (t == ord) count += __popc(hits & home);
+            const unsigned b0 = __ballot_sync(kFull, n0), b1 = __ballot_sync(kFull, n1);
+            if ((ord >> 1) == (t >> 1)) count += __popc(((ord & 1) ? b1 : b0) & home);
         }
-        __syncwarp();
     }
-    __syncwarp();
+    const int slot = slot_of(h), all = count + 1;  // the point itself included
+    const bool core = all >= v.min_pts;
     if (hv) {
-        const int slot = slot_of(h), all = count + 1;  // the point itself included
-        const bool core = all >= v.min_pts;
         v.scnt[cur][start + lane] = all;
         v.sroot[start + lane] = core ? slot : -1;
-        if (v.list_cap >= 0) {
-            v.ntrack[slot] = core ? 0 : 1;
-            if (!core) {
-                int4* L = reinterpret_cast<int4*>(v.nlist + (size_t)slot * v.list_stride);
-                const int* bf = sm.buf[wib] + lane * kListCap;
-                for (int k = 0; k < v.list_stride; k += 4)
-                    L[k >> 2] = make_int4(k < count ? bf[k] : -1, k + 1 < count ? bf[k + 1] : -1,
-                                          k + 2 < count ? bf[k + 2] : -1, k + 3 < count ? bf[k + 3] : -1);
+    }
+    if (v.list_cap >= 0) {
+        if (hv) v.ntrack[slot] = core ? 0 : 1;
+        if (hv && !core) {
+            int4* L = reinterpret_cast<int4*>(v.nlist + (size_t)slot * v.list_stride);
+            for (int k = 0; k < v.list_stride >> 2; ++k) L[k] = make_int4(-1, -1, -1, -1);
+        }
+        __syncwarp();
+        // lists of the non-core points with neighbours: the point's candidates
+        // once more (few points, in the sparser cells)
+        unsigned todo = __ballot_sync(kFull, hv && !core && count > 0);
+        while (todo) {
+            const int l = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const int s = __shfl_sync(kFull, run, l), aslot = __shfl_sync(kFull, slot, l);
+            const int from = sm.sbeg[wib][s], to = sm.sbeg[wib][s + 1];
+            const float4 hp = sm.pt[wib][l];
+            int* L = v.nlist + (size_t)aslot * v.list_stride;
+            int found = 0;
+            r = sm.tbeg[wib][s];
+            for (int base = from; base < to; base += 32) {
+                const int idx = base + lane;
+                bool nb = false;
+                int qs = -1;
+                if (idx < to) {
+                    while (idx >= tpre[r + 1]) ++r;
+                    const float4 q = spt[tstart[r] + idx - tpre[r]];
+                    qs = slot_of(q);
+                    nb = qs != aslot && is_nbr<MODE, DIM>(v, hp, q, tally);
+                }
+                const unsigned hits = __ballot_sync(kFull, nb);
+                const int k = found + __popc(hits & lanemask_lt(lane));
+                if (nb && k < v.list_cap) L[k] = qs;
+                found += __popc(hits);
             }
         }
     }
@@ -2692,9 +2712,13 @@ cudaError_t launch_window_phase(int phase, const View& v, int precision, const f
             k_build<<<(v.W + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, s>>>(v);
             break;
         case kPhaseIncrement: {
-            const int block = v.dim == 3 && v.cell_mult == 2 ? 16 : 32;  // positions per warp (CountShape)
+            // positions per warp (at most CountShape's): short chains while the
+            // blocks are few, fuller lookups above.  us with 8 / 16 / 32: 20k
+            // points 14 / 20 / 28, 48k 39 / 43 / 66, 200k trajectories 141 / 136
+            // / 152, 1M walkers 358 / 300 / 276
+            const int block = v.W < 65536 ? 8 : (v.W < 524288 || (v.dim == 3 && v.cell_mult == 2) ? 16 : 32);
             const int per = block * (kCountThreads / 32);
-            RTDBS_DISPATCH(precision, dk_of(v), k_count, (v.W + per - 1) / per, kCountThreads, s, v);
+            RTDBS_DISPATCH(precision, dk_of(v), k_count, (v.W + per - 1) / per, kCountThreads, s, v, block);
             break;
         }
         default: return cudaErrorInvalidValue;
