@@ -99,9 +99,10 @@ typedef struct rtdbs_params {
                              warps, picked by rtdbstream_gb300/autotune.py.  No reference
                              counterpart */
     int32_t query_lanes;  /* lanes that scan one expired or new point's neighbourhood in the
-                             count passes, 16 or 32 (0 = 16 with one cell per Eps, 32 with
-                             two; two cells per Eps needs 32): the block shape of those
-                             passes (a 256-thread block takes 16 or 8 points), picked by
+                             count passes, 16 or 32 (0 = 16 with one cell per Eps in a pool
+                             or at strides above 6,080 points, else 32; two cells per Eps
+                             needs 32): the block shape of those passes (a 256-thread
+                             block takes 16 or 8 points), picked by
                              rtdbstream_gb300/autotune.py.  No reference counterpart */
     int32_t reserved[3];
 } rtdbs_params;

@@ -525,7 +525,13 @@ int rtdbs_create(const rtdbs_params* params, void* cuda_stream, rtdbs_engine** o
     v.dim = p.dim;
     v.cell_mult = p.cell_mult > 0 ? p.cell_mult : 1;
     v.grab = p.work_grab;  // 0: by launch kind and window size (work_grab in the kernels)
-    v.qlanes = p.query_lanes > 0 ? p.query_lanes : (v.cell_mult == 1 ? rtdbs::kQueryLanes : 32);
+    // a stride of few points leaves the count passes short of warps: the whole
+    // warp for one query while all fit the GPU at once (152 SMs of 40 warps).
+    // Decrement and increment, us, with 16 / 32 lanes: 500 points 16 + 16 / 12 +
+    // 12, 1k 14 + 14 / 10 + 10, 5k 52 + 67 / 32 + 35, 10k (1M walkers) 31 + 24 /
+    // 36 + 31
+    v.qlanes = p.query_lanes > 0 ? p.query_lanes
+                                 : (v.cell_mult == 1 && p.stride > 6080 ? rtdbs::kQueryLanes : 32);
     v.W = p.window;
     v.S = p.stride;
     v.min_pts = p.min_pts;
@@ -1212,6 +1218,8 @@ int rtdbs_pool_add_stream(rtdbs_pool* p, const rtdbs_params* params, int32_t* st
     // this stream's control block lives in the pool's contiguous array
     e->v.ctl = p->d_ctls + slot;
     e->pooled = true;
+    // a round's streams fill the GPU together: two queries per warp
+    if (q.query_lanes == 0 && e->v.cell_mult == 1) e->v.qlanes = rtdbs::kQueryLanes;
     {
         DeviceGuard guard(p->device);
         if (cudaMemsetAsync(e->v.ctl, 0, sizeof(Ctl), p->stream) != cudaSuccess) {

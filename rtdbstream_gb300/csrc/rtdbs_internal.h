@@ -47,8 +47,9 @@ constexpr int kClusterThreads = 256;
 constexpr int kLinkThreads = 256;
 constexpr int kBatch = 8;          // default work items a clustering warp takes at a time
                                    // in a pool launch
-constexpr int kQueryLanes = 16;    // default lanes per query point in the count passes (one
-                                   // cell per Eps: two points per warp overlap their loads)
+constexpr int kQueryLanes = 16;    // lanes per query point in the count passes where the queries
+                                   // fill the GPU (one cell per Eps: two points per warp
+                                   // overlap their loads)
 constexpr int kMaxIter = 1 << 20;  // bound on every device-side retry loop
 constexpr int kListCap = 30;       // longest neighbour list kept (MinPts <= 32)
 
@@ -177,9 +178,10 @@ constexpr int kChunkPhases = 6;  // ingest .. increment, once per chunk
 // load), c = points in the chunk, init = 1 while loading the first window,
 // advance = 1 when the label phase ends a slide.
 cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, int init,
-                         int staging_offset, int advance, cudaStream_t s);
+                         int staging_offset, int advance, cudaStream_t s, bool pdl = false);
 // With a side stream and two events, the decrement pass (which needs only
-// the ingest) runs on `side` beside the sort, joined before the merge.
+// the ingest) runs on `side` beside the sort, joined before the merge.  pdl:
+// programmatic dependence on the kernel launched before on the same stream.
 cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int init,
                               int staging_offset, cudaStream_t s, cudaStream_t side = nullptr,
                               cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
@@ -189,7 +191,7 @@ cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int in
 cudaError_t launch_window_build(const View& v, int precision, const float* input, int count, int init,
                                 cudaStream_t s);
 cudaError_t launch_window_phase(int phase, const View& v, int precision, const float* input, int count, int init,
-                                cudaStream_t s);
+                                cudaStream_t s, bool pdl = false);
 int window_build_launches(const View& v);
 // Bounding box of n points per axis as order-keeping unsigned keys: minima
 // in box[0..2] (~0: no finite coordinate), maxima in box[3..5] (device).

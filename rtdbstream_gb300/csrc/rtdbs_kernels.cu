@@ -52,6 +52,15 @@ constexpr unsigned kFull = 0xffffffffu;
 constexpr int kPrecFp64 = 0;
 constexpr int kPrecFp32 = 1;
 
+// Programmatic dependent launch: a kernel so launched starts while its
+// predecessor runs and waits here, before anything else, for the
+// predecessor's end and memory; its own successor may then start likewise.
+// (No effect on other launches.)
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ int slot_of(const float4& p) { return __float_as_int(p.w); }
 
 
@@ -723,6 +732,7 @@ __device__ __forceinline__ void ingest_body(const View& v, int j, int c, int ini
 }
 
 __global__ void k_ingest(View v, int j, int c, int init, int stg_off) {
+    pdl_wait();
     ingest_body(v, j, c, init, stg_off, v.staging, blockIdx.x);
 }
 
@@ -835,6 +845,7 @@ __device__ __forceinline__ void sort_body(const View& v, int j, int c, int init,
 }
 
 __global__ void __launch_bounds__(kSortRun) k_sort(View v, int j, int c, int init, int single) {
+    pdl_wait();
     __shared__ SortSmem sm;
     sort_body(v, j, c, init, blockIdx.x, blockIdx.y, sm, single != 0);
 }
@@ -888,6 +899,7 @@ __device__ __forceinline__ void runmerge_body(const View& v, int j, int c, int i
 }
 
 __global__ void __launch_bounds__(kSortRun) k_runmerge(View v, int j, int c, int init) {
+    pdl_wait();
     extern __shared__ unsigned long long words[];
     runmerge_body(v, j, c, init, blockIdx.x, blockIdx.y, words);
 }
@@ -997,6 +1009,7 @@ __device__ __forceinline__ void decr_body(const View& v, int j, int c, int bx, S
 
 template <int MODE, int DK>
 __global__ void __launch_bounds__(256) k_decr(View v, int j, int c) {
+    pdl_wait();
     __shared__ StreamSmem sm;
     decr_body<MODE, DK>(v, j, c, blockIdx.x, sm);
 }
@@ -1055,17 +1068,20 @@ __device__ __forceinline__ int warp_count_words_less(const unsigned long long* w
 // new entries; tile t of the old window goes to output offset
 // ts - (#expired before ts) + (#new before old[ts]).
 constexpr int kMergeStage = 1024;  // new words of a tile staged in shared memory
+template <int TILE>
 struct MergeSmem {
-    unsigned long long tkey[kMergeTile];
+    unsigned long long tkey[TILE];
     unsigned long long nw[kMergeStage];
-    int tslot[kMergeTile];
-    int spre[kMergeTile + 1];
+    int tslot[TILE];
+    int spre[TILE + 1];
     unsigned wsum[32];
     int bnd[3];
 };
 
+template <int TILE>
 __device__ __forceinline__ void merge_body(const View& v, int j, int c, int init, int bx, int nbx,
-                                           MergeSmem& sm) {
+                                           MergeSmem<TILE>& sm) {
+    constexpr int kPer = TILE / kMergeThreads;  // old entries per thread
     unsigned long long* tkey = sm.tkey;
     int* tslot = sm.tslot;
     int* spre = sm.spre;
@@ -1097,11 +1113,11 @@ __device__ __forceinline__ void merge_body(const View& v, int j, int c, int init
         for (unsigned i = bx * blockDim.x + tid; i <= v.pmask; i += nbx * blockDim.x)
             T[i] = make_ulonglong2(0ull, 0ull);
     }
-    const int ntiles = n_old > 0 ? (n_old + kMergeTile - 1) / kMergeTile : 1;
+    const int ntiles = n_old > 0 ? (n_old + TILE - 1) / TILE : 1;
     const int t = bx;
     if (t >= ntiles) return;
-    const int ts = t * kMergeTile;
-    const int te = min(ts + kMergeTile, n_old);
+    const int ts = t * TILE;
+    const int te = min(ts + TILE, n_old);
     const int tlen = te - ts;
     const unsigned long long* okey = v.skey[src];
     const float4* opt = v.spt[src];
@@ -1141,11 +1157,11 @@ __device__ __forceinline__ void merge_body(const View& v, int j, int c, int init
     const unsigned long long* nw = staged ? sm.nw : v.nword + jt0;  // the tile's new words
     if (staged)
         for (int i = tid; i < m; i += kMergeThreads) sm.nw[i] = v.nword[jt0 + i];
-    unsigned flags[4];
+    unsigned flags[kPer];
     unsigned cnt = 0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        const int i = tid * 4 + k;
+    for (int k = 0; k < kPer; ++k) {
+        const int i = tid * kPer + k;
         const bool surv = i < tlen && (init || tslot[i] < el || tslot[i] >= el + c);
         flags[k] = surv ? 1u : 0u;
         cnt += flags[k];
@@ -1173,11 +1189,11 @@ __device__ __forceinline__ void merge_body(const View& v, int j, int c, int init
         __syncthreads();
         unsigned pre = wsum[w] + incl - cnt;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            spre[tid * 4 + k] = (int)pre;
+        for (int k = 0; k < kPer; ++k) {
+            spre[tid * kPer + k] = (int)pre;
             pre += flags[k];
         }
-        if (tid == kMergeThreads - 1) spre[kMergeTile] = (int)pre;
+        if (tid == kMergeThreads - 1) spre[TILE] = (int)pre;
     }
     __syncthreads();
 
@@ -1234,8 +1250,10 @@ __device__ __forceinline__ void merge_body(const View& v, int j, int c, int init
     }
 }
 
+template <int TILE>
 __global__ void __launch_bounds__(kMergeThreads) k_merge(View v, int j, int c, int init) {
-    __shared__ MergeSmem sm;
+    pdl_wait();
+    __shared__ MergeSmem<TILE> sm;
     merge_body(v, j, c, init, blockIdx.x, gridDim.x, sm);
 }
 
@@ -1318,6 +1336,7 @@ __device__ __forceinline__ void build_body(const View& v, int bx, BuildSmem& sm,
 }
 
 __global__ void __launch_bounds__(kBuildThreads) k_build(View v) {
+    pdl_wait();
     __shared__ BuildSmem sm;
     build_body(v, blockIdx.x, sm, false);
 }
@@ -1433,6 +1452,7 @@ __device__ __forceinline__ void incr_body(const View& v, int j, int c, int init,
 
 template <int MODE, int DK>
 __global__ void __launch_bounds__(256, 5) k_incr(View v, int j, int c, int init) {
+    pdl_wait();
     __shared__ StreamSmem sm;
     incr_body<MODE, DK>(v, j, c, init, blockIdx.x, sm);
 }
@@ -1470,6 +1490,7 @@ __device__ __forceinline__ unsigned long long* rad_buffer(const View& v, int pas
 // in the ring, 0 while loading); every slot's sort word goes to the first
 // pass's input (chunk < 0), or the new points' chunk words to nsort.
 __global__ void k_ingest_all(View v, const float* input, int count, int init, int ob, int passes) {
+    pdl_wait();
     const long long b = v.ctl->b_done + 1;  // this build (k_build keeps b_done)
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         v.ctl->b = b;
@@ -1504,6 +1525,7 @@ __global__ void k_ingest_all(View v, const float* input, int count, int init, in
 }
 
 __global__ void __launch_bounds__(kRadThreads) k_rad_hist(View v, int pass, int passes, int shift) {
+    pdl_wait();
     __shared__ int hist[256];
     const unsigned long long* in = rad_buffer(v, pass, passes);
     int* counts = v.scnt[(v.ctl->b & 1) ^ 1];
@@ -1528,6 +1550,7 @@ __global__ void __launch_bounds__(kRadThreads) k_rad_hist(View v, int pass, int 
 // side), 8 warps on an eighth of the tiles each; the digits' totals follow
 // the tiles' counters.  Only where there are many tiles (kRadInline).
 __global__ void __launch_bounds__(256) k_rad_scan(View v, int ntiles) {
+    pdl_wait();
     __shared__ int part[8][32];
     int* counts = v.scnt[(v.ctl->b & 1) ^ 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = blockIdx.x * 32 + lane;
@@ -1552,6 +1575,7 @@ __global__ void __launch_bounds__(256) k_rad_scan(View v, int ntiles) {
 // consecutive words in order (lanes with equal digits from eight ballots),
 // warp counters are scanned per digit, and every word goes to its place.
 __global__ void __launch_bounds__(kRadThreads) k_rad_scatter(View v, int pass, int passes, int shift, int scanned) {
+    pdl_wait();
     __shared__ int cnt[kRadWarps][256];
     __shared__ int wsum[8];
     const unsigned long long* in = rad_buffer(v, pass, passes);
@@ -1630,6 +1654,7 @@ __global__ void __launch_bounds__(kRadThreads) k_rad_scatter(View v, int pass, i
 // The window laid out in the order of its sorted words (counts and hints
 // follow in k_count), a fresh forest, and the build's counters reset.
 __global__ void k_fill(View v, int ob, int passes) {
+    pdl_wait();
     const long long b = v.ctl->b;
     const int cur = (int)(b & 1);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1700,6 +1725,7 @@ __device__ __forceinline__ unsigned lane_range(int lo, int hi) {  // lanes [lo, 
 
 template <int MODE, int DK>
 __global__ void __launch_bounds__(kCountThreads, 8) k_count(View v, int P) {
+    pdl_wait();
     constexpr int DIM = DK & 3, K = (DK >> 2) + 1;
     using C = CountShape<DIM, K>;
     constexpr int R = C::kRows;
@@ -1852,6 +1878,7 @@ __global__ void __launch_bounds__(kCountThreads, 8) k_count(View v, int P) {
 // slot for a core) and a fresh forest, for a clustering of the window as it
 // stands (rtdbs_cluster), whose hints may hold the last union's roots.
 __global__ void k_hints(View v) {
+    pdl_wait();
     const int cur = (int)(v.ctl->b & 1);
     const int n = v.ctl->nocc[cur];
     const int* scnt = v.scnt[cur];
@@ -1943,6 +1970,7 @@ __device__ __forceinline__ void link_body(const View& v, int bx, LinkSmem& sm) {
 
 template <int MODE, int DK>
 __global__ void __launch_bounds__(kLinkThreads) k_link(View v) {
+    pdl_wait();
     __shared__ LinkSmem sm;
     link_body<MODE, DK>(v, blockIdx.x, sm);
 }
@@ -2194,6 +2222,7 @@ __device__ __forceinline__ void union_body(const View& v, Smem& sm, int P, int g
 
 template <int MODE, int DK>
 __global__ void __launch_bounds__(kClusterThreads, kUnionBlocks) k_union(View v) {
+    pdl_wait();
     __shared__ UnionSmem<(DK & 3), (DK >> 2) + 1> sm;
     union_body<MODE, DK>(v, sm, v.block_pts, union_grab(v));
 }
@@ -2297,6 +2326,7 @@ __device__ __forceinline__ void flatten_body(const View& v, int bx, int nbx, Str
 
 template <int MODE, int DK>
 __global__ void __launch_bounds__(256, 6) k_flatten(View v) {
+    pdl_wait();
     __shared__ StreamSmem sm;
     flatten_body<MODE, DK>(v, blockIdx.x, gridDim.x, sm);
 }
@@ -2395,6 +2425,7 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, C
 
 template <int MODE, int DK>
 __global__ void __launch_bounds__(kClusterThreads, 6) k_label(View v, int advance) {
+    pdl_wait();
     __shared__ ClusterSmem sm;
     label_body<MODE, DK>(v, advance, blockIdx.x, sm, work_grab(v, false));
 }
@@ -2446,7 +2477,7 @@ __device__ __forceinline__ void border_body(const View& v, int advance, int bx, 
     }
 }
 
-__global__ void k_border(View v, int advance) { border_body(v, advance, blockIdx.x, gridDim.x); }
+__global__ void k_border(View v, int advance) { pdl_wait(); border_body(v, advance, blockIdx.x, gridDim.x); }
 
 __global__ void k_counts_by_slot(View v, int* nn) {
     const int cur = (int)(v.ctl->b & 1);
@@ -2519,7 +2550,7 @@ __global__ void __launch_bounds__(PhaseShape<PHASE>::threads, PhaseShape<PHASE>:
         __shared__ StreamSmem sm;
         decr_body<MODE, DK>(sv, it.j, it.c, bx, sm);
     } else if constexpr (PHASE == kBatchMerge) {
-        __shared__ MergeSmem sm;
+        __shared__ MergeSmem<kMergeTile> sm;
         merge_body(sv, it.j, it.c, 0, bx, nbx, sm);
     } else if constexpr (PHASE == kBatchBuild) {
         __shared__ BuildSmem sm;
@@ -2563,27 +2594,44 @@ void ensure_runmerge_smem() {
 
 }  // namespace
 
+// Kernel launch, with programmatic dependence on the launch before it on this
+// stream where `pdl` (that launch must be a kernel that calls pdl_wait).
+template <class... P, class... A>
+void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl, A... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&c, kernel, P(args)...);
+}
+
 // Launch of a work kernel instantiated for (precision, DK); dk = dim + 4 (K - 1).
-#define RTDBS_DISPATCH(prec, dk_expr, KERNEL, GRID, BLOCK, STREAM, ...)          \
+#define RTDBS_DISPATCH(prec, dk_expr, KERNEL, GRID, BLOCK, STREAM, PDL, ...)          \
     do {                                                                         \
         const int dk = (dk_expr);                                                \
         if ((prec) == kPrecFp32) {                                               \
             switch (dk) {                                                        \
-                case 1: KERNEL<kPrecFp32, 1><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
-                case 2: KERNEL<kPrecFp32, 2><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
-                case 3: KERNEL<kPrecFp32, 3><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
-                case 5: KERNEL<kPrecFp32, 5><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
-                case 6: KERNEL<kPrecFp32, 6><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
-                default: KERNEL<kPrecFp32, 7><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
+                case 1: launch(KERNEL<kPrecFp32, 1>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
+                case 2: launch(KERNEL<kPrecFp32, 2>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
+                case 3: launch(KERNEL<kPrecFp32, 3>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
+                case 5: launch(KERNEL<kPrecFp32, 5>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
+                case 6: launch(KERNEL<kPrecFp32, 6>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
+                default: launch(KERNEL<kPrecFp32, 7>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
             }                                                                    \
         } else {                                                                 \
             switch (dk) {                                                        \
-                case 1: KERNEL<kPrecFp64, 1><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
-                case 2: KERNEL<kPrecFp64, 2><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
-                case 3: KERNEL<kPrecFp64, 3><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
-                case 5: KERNEL<kPrecFp64, 5><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
-                case 6: KERNEL<kPrecFp64, 6><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
-                default: KERNEL<kPrecFp64, 7><<<GRID, BLOCK, 0, STREAM>>>(__VA_ARGS__); break; \
+                case 1: launch(KERNEL<kPrecFp64, 1>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
+                case 2: launch(KERNEL<kPrecFp64, 2>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
+                case 3: launch(KERNEL<kPrecFp64, 3>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
+                case 5: launch(KERNEL<kPrecFp64, 5>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
+                case 6: launch(KERNEL<kPrecFp64, 6>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
+                default: launch(KERNEL<kPrecFp64, 7>, GRID, BLOCK, 0, STREAM, PDL, __VA_ARGS__); break; \
             }                                                                    \
         }                                                                        \
     } while (0)
@@ -2597,38 +2645,51 @@ cudaError_t configure_kernels() {
     return cudaSuccess;
 }
 
+// Slides of windows up to this size launch their kernels with programmatic
+// dependence: they are short enough for the launch and the first instructions
+// to show (slides of 2.5k / 10k / 100k points 112 -> 106, 98 -> 95, 312 -> 291
+// us); on larger ones the waiting blocks take SM slots from the running kernel
+// (500k points 168 -> 186 us, 1M 324 -> 342).
+constexpr int kPdlWindow = 131072;
+bool pdl_on(const View& v) { return v.W <= kPdlWindow; }
+
 cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, int init,
-                         int stg_off, int advance, cudaStream_t s) {
+                         int stg_off, int advance, cudaStream_t s, bool pdl) {
     const int warp_blocks = (c * v.qlanes + 255) / 256;  // count passes
     switch (phase) {
         case kPhaseIngest:
-            k_ingest<<<(c + 255) / 256, 256, 0, s>>>(v, j, c, init, stg_off);
+            launch(k_ingest, (c + 255) / 256, 256, 0, s, pdl, v, j, c, init, stg_off);
             break;
         case kPhaseSort: {
             const int single = c <= kSortRun;  // one run: sorted straight into place, no run merge
-            k_sort<<<dim3((c + kSortRun - 1) / kSortRun, init ? 1 : 2), kSortRun, 0, s>>>(v, j, c, init, single);
+            launch(k_sort, dim3((c + kSortRun - 1) / kSortRun, init ? 1 : 2), kSortRun, 0, s, pdl, v, j, c, init, single);
             if (single) break;
             ensure_runmerge_smem();
-            k_runmerge<<<dim3((c + kSortRun - 1) / kSortRun, init ? 1 : 2), kSortRun,
-                         sizeof(unsigned long long) * c, s>>>(v, j, c, init);
+            launch(k_runmerge, dim3((c + kSortRun - 1) / kSortRun, init ? 1 : 2), kSortRun, sizeof(unsigned long long) * c,
+                   s, pdl, v, j, c, init);
             break;
         }
         case kPhaseDecrement:
-            if (!init) RTDBS_DISPATCH(precision, dk_of(v), k_decr, warp_blocks, 256, s, v, j, c);
+            if (!init) RTDBS_DISPATCH(precision, dk_of(v), k_decr, warp_blocks, 256, s, pdl, v, j, c);
             break;
         case kPhaseMerge:
-            k_merge<<<(v.W + kMergeTile - 1) / kMergeTile, kMergeThreads, 0, s>>>(v, j, c, init);
+            // short tiles where the blocks are few (10k points 14 -> 10 us, 200k
+            // 14 -> 10), fewer searches above (500k 25 -> 16, 1M 37 -> 25)
+            if (v.W < 262144)
+                launch(k_merge<256>, (v.W + 255) / 256, kMergeThreads, 0, s, pdl, v, j, c, init);
+            else
+                launch(k_merge<kMergeTile>, (v.W + kMergeTile - 1) / kMergeTile, kMergeThreads, 0, s, pdl, v, j, c, init);
             break;
         case kPhaseBuild:
-            k_build<<<(v.W + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, s>>>(v);
+            launch(k_build, (v.W + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, s, pdl, v);
             break;
         case kPhaseIncrement:
-            RTDBS_DISPATCH(precision, dk_of(v), k_incr, warp_blocks, 256, s, v, j, c, init);
+            RTDBS_DISPATCH(precision, dk_of(v), k_incr, warp_blocks, 256, s, pdl, v, j, c, init);
             break;
         case kPhaseLabel:
             if (v.list_cap >= 0) {
                 const int sms = g_num_sms > 0 ? g_num_sms : 152;
-                k_border<<<max(1, min(sms * 8, (v.W + 255) / 256)), 256, 0, s>>>(v, advance);
+                launch(k_border, max(1, min(sms * 8, (v.W + 255) / 256)), 256, 0, s, pdl, v, advance);
                 break;
             }
             [[fallthrough]];
@@ -2639,15 +2700,15 @@ cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, 
             const int need = (v.W + 95) / 96;
             const int blocks = max(1, min(sms * 6, need));
             if (phase == kPhaseUnion) {
-                RTDBS_DISPATCH(precision, dk_of(v), k_link, (v.W + kLinkThreads - 1) / kLinkThreads, kLinkThreads, s, v);
-                RTDBS_DISPATCH(precision, dk_of(v), k_union, max(1, min(sms * kUnionBlocks, (v.W + v.block_pts * 8 - 1) / (v.block_pts * 8))), kClusterThreads, s, v);
+                RTDBS_DISPATCH(precision, dk_of(v), k_link, (v.W + kLinkThreads - 1) / kLinkThreads, kLinkThreads, s, pdl, v);
+                RTDBS_DISPATCH(precision, dk_of(v), k_union, max(1, min(sms * kUnionBlocks, (v.W + v.block_pts * 8 - 1) / (v.block_pts * 8))), kClusterThreads, s, pdl, v);
             } else
-                RTDBS_DISPATCH(precision, dk_of(v), k_label, blocks, kClusterThreads, s, v, advance);
+                RTDBS_DISPATCH(precision, dk_of(v), k_label, blocks, kClusterThreads, s, pdl, v, advance);
             break;
         }
         case kPhaseFlatten: {
             const int sms = g_num_sms > 0 ? g_num_sms : 152;
-            RTDBS_DISPATCH(precision, dk_of(v), k_flatten, max(1, min(sms * 16, (v.W + 255) / 256)), 256, s, v);
+            RTDBS_DISPATCH(precision, dk_of(v), k_flatten, max(1, min(sms * 16, (v.W + 255) / 256)), 256, s, pdl, v);
             break;
         }
         default:
@@ -2662,12 +2723,17 @@ cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int in
     const bool beside = side && fork && join && !init;  // the decrement beside the sort
     for (int ph = 0; ph < kChunkPhases; ++ph) {
         cudaError_t e = cudaSuccess;
-        if (beside && ph == kPhaseDecrement) continue;  // launched right after the ingest
+        if (beside && ph == kPhaseDecrement) continue;  // launched on the side stream
         if (beside && ph == kPhaseMerge && (e = cudaStreamWaitEvent(s, join, 0)) != cudaSuccess) return e;
-        e = launch_phase(ph, v, precision, j, c, init, stg_off, 0, s);
+        // (the ingest follows a copy or another chunk's work, the merge two streams)
+        const bool pdl = pdl_on(v) && ph != kPhaseIngest && ph != kPhaseDecrement && ph != kPhaseMerge;
+        e = launch_phase(ph, v, precision, j, c, init, stg_off, 0, s, pdl);
         if (e != cudaSuccess) return e;
-        if (beside && ph == kPhaseIngest) {
-            if ((e = cudaEventRecord(fork, s)) != cudaSuccess) return e;
+        // (after the ingest, but launched behind the sort, whose few large blocks
+        // should not wait for the decrement's to leave: 500k points 174 -> 166 us
+        // per slide, 1M 325 -> 318)
+        if (beside && ph == kPhaseIngest && (e = cudaEventRecord(fork, s)) != cudaSuccess) return e;
+        if (beside && ph == kPhaseSort) {
             if ((e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess) return e;
             if ((e = launch_phase(kPhaseDecrement, v, precision, j, c, init, stg_off, 0, side)) != cudaSuccess)
                 return e;
@@ -2678,38 +2744,38 @@ cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int in
 }
 
 cudaError_t launch_window_phase(int phase, const View& v, int precision, const float* input, int count, int init,
-                                cudaStream_t s) {
+                                cudaStream_t s, bool pdl) {
     const int grid = (v.W + 255) / 256;
     const bool chunk = v.W <= kChunkMax;  // one chunk: its runs are sorted and ranked on chip
     const int ob = chunk ? kOffBits : slot_bits(v.W);
     const int passes = chunk ? -1 : (v.key_bits + 7) / 8;
     switch (phase) {
         case kPhaseIngest:
-            k_ingest_all<<<grid, 256, 0, s>>>(v, input, count, init, ob, passes);
+            launch(k_ingest_all, grid, 256, 0, s, pdl, v, input, count, init, ob, passes);
             break;
         case kPhaseSort:
             if (chunk) {
                 const int runs = (v.W + kSortRun - 1) / kSortRun;
-                k_sort<<<dim3(runs, 1), kSortRun, 0, s>>>(v, 0, v.W, 1, runs == 1);
+                launch(k_sort, dim3(runs, 1), kSortRun, 0, s, pdl, v, 0, v.W, 1, runs == 1);
                 if (runs == 1) break;
                 ensure_runmerge_smem();
-                k_runmerge<<<dim3(runs, 1), kSortRun, sizeof(unsigned long long) * v.W, s>>>(v, 0, v.W, 1);
+                launch(k_runmerge, dim3(runs, 1), kSortRun, sizeof(unsigned long long) * v.W, s, pdl, v, 0, v.W, 1);
                 break;
             }
             for (int p = 0; p < passes; ++p) {
                 const int tiles = (v.W + kRadTile - 1) / kRadTile;
-                k_rad_hist<<<tiles, kRadThreads, 0, s>>>(v, p, passes, ob + 8 * p);
+                launch(k_rad_hist, tiles, kRadThreads, 0, s, pdl, v, p, passes, ob + 8 * p);
                 const int scanned = tiles > kRadInline;
-                if (scanned) k_rad_scan<<<8, 256, 0, s>>>(v, tiles);
-                k_rad_scatter<<<tiles, kRadThreads, 0, s>>>(v, p, passes, ob + 8 * p, scanned);
+                if (scanned) launch(k_rad_scan, 8, 256, 0, s, pdl, v, tiles);
+                launch(k_rad_scatter, tiles, kRadThreads, 0, s, pdl, v, p, passes, ob + 8 * p, scanned);
             }
             break;
         case kPhaseDecrement: break;  // counted afresh
         case kPhaseMerge:
-            k_fill<<<grid, 256, 0, s>>>(v, ob, passes);
+            launch(k_fill, grid, 256, 0, s, pdl, v, ob, passes);
             break;
         case kPhaseBuild:
-            k_build<<<(v.W + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, s>>>(v);
+            launch(k_build, (v.W + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, s, pdl, v);
             break;
         case kPhaseIncrement: {
             // positions per warp (at most CountShape's): short chains while the
@@ -2718,7 +2784,7 @@ cudaError_t launch_window_phase(int phase, const View& v, int precision, const f
             // / 152, 1M walkers 358 / 300 / 276
             const int block = v.W < 65536 ? 8 : (v.W < 524288 || (v.dim == 3 && v.cell_mult == 2) ? 16 : 32);
             const int per = block * (kCountThreads / 32);
-            RTDBS_DISPATCH(precision, dk_of(v), k_count, (v.W + per - 1) / per, kCountThreads, s, v, block);
+            RTDBS_DISPATCH(precision, dk_of(v), k_count, (v.W + per - 1) / per, kCountThreads, s, pdl, v, block);
             break;
         }
         default: return cudaErrorInvalidValue;
@@ -2731,7 +2797,9 @@ cudaError_t launch_window_build(const View& v, int precision, const float* input
     if (!window_build_fits(v)) return cudaErrorInvalidValue;
     cudaError_t e = cudaSuccess;
     for (int ph = 0; ph < kChunkPhases && e == cudaSuccess; ++ph)
-        e = launch_window_phase(ph, v, precision, input, count, init, s);
+        // (kernels that follow each other closely at any size: a first window of
+        // 1M points 864 -> 820 us, of 20k 205 -> 179)
+        e = launch_window_phase(ph, v, precision, input, count, init, s, ph != kPhaseIngest);
     return e;
 }
 
@@ -2785,7 +2853,8 @@ cudaError_t launch_cluster(const View& v, int precision, int advance, cudaStream
     }
     for (int ph = kPhaseUnion; ph <= kPhaseLabel && e == cudaSuccess; ++ph) {
         if (ph == kPhaseLabel && outputs_free) e = cudaStreamWaitEvent(s, outputs_free, wait_flags);
-        if (e == cudaSuccess) e = launch_phase(ph, v, precision, 0, 0, 0, 0, advance, s);
+        const bool pdl = pdl_on(v) && !(ph == kPhaseLabel && outputs_free);
+        if (e == cudaSuccess) e = launch_phase(ph, v, precision, 0, 0, 0, 0, advance, s, pdl);
     }
     return e;
 }

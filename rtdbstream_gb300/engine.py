@@ -284,7 +284,7 @@ def make_params(dim: int, window_size: int, stride_size: int, radius: float, min
     """rtdbs_params for one stream; cell_mult = grid cells per Eps (1 or 2),
     work_grab = work items per queue grab of the clustering warps (0: 8),
     query_lanes = lanes per query point in the count passes (0: 16 with one
-    cell per Eps, 32 with two; 16 or 32)."""
+    cell per Eps in a pool or at strides above 6,080 points, else 32; 16 or 32)."""
     L = load_library()
     p = Params()
     _check(L.rtdbs_params_init(ctypes.byref(p)))
