@@ -51,8 +51,8 @@ extern "C" {
 #define RTDBS_ERR_CUDA      -2  /* a CUDA runtime call failed (rtdbs_last_error has the text) */
 #define RTDBS_ERR_OOM       -3  /* device or pinned allocation failed */
 #define RTDBS_ERR_STATE     -4  /* call out of order (slide before rtdbs_load_window) */
-#define RTDBS_ERR_DEVICE    -5  /* a device-side bound was hit (hash probe, union-find retry,
-                                   work-list capacity); the engine must be reloaded */
+#define RTDBS_ERR_DEVICE    -5  /* a device-side bound was hit (hash probe, union-find retry);
+                                   the engine must be reloaded */
 #define RTDBS_ERR_NO_DEVICE -6  /* no CUDA device / library built without one */
 #define RTDBS_ERR_BUDGET    -7  /* pool admission refused: HBM budget or stream slots exhausted */
 
@@ -92,12 +92,11 @@ typedef struct rtdbs_params {
                              work items where they are sparse (rtdbstream_gb300/autotune.py
                              picks it per stream).  The reference's grid has side Eps/sqrt(3)
                              (src/dbscan/dbscan.cpp:34-37) */
-    int32_t work_grab;    /* work items (cell runs) a clustering warp takes from the shared
-                             queue at a time, 1..64 (0 = 8 in a pool; for a stream slid on
-                             its own, 5 or 8 on large windows by cell occupancy and fewer
-                             on small ones: 1 below 32,768 points): the work split between
-                             warps, picked by rtdbstream_gb300/autotune.py.  No reference
-                             counterpart */
+    int32_t work_grab;    /* cell runs a union warp takes from the shared queue at a time,
+                             1..64 (0 = the default), in whole blocks of sorted positions
+                             (16 or 32 of them, about 16 runs: one block up to 31): the
+                             work split between warps, picked by
+                             rtdbstream_gb300/autotune.py.  No reference counterpart */
     int32_t query_lanes;  /* lanes that scan one expired or new point's neighbourhood in the
                              count passes, 16 or 32 (0 = 16 with one cell per Eps in a pool
                              or at strides above 6,080 points, else 32; two cells per Eps
@@ -112,7 +111,7 @@ typedef struct rtdbs_stats {
     int64_t slides;          /* slides completed */
     int64_t band_rechecks;   /* pair tests re-decided in FP64 (FP64 mode) */
     int64_t cells;           /* non-empty grid cells of the current window */
-    int64_t work_items;      /* cell runs scheduled by the clustering kernels */
+    int64_t work_items;      /* cell runs (within 32 sorted positions) of the current window */
     int32_t error_bits;      /* device error word (0 = healthy) */
     int32_t key_bits;        /* bits of the cell key */
     double  cell_side;       /* grid cell side (>= Eps) */
@@ -237,7 +236,7 @@ RTDBS_API int rtdbs_get_stats(rtdbs_engine* engine, rtdbs_stats* stats);
  * d_label[n], d_cluster_id[n] (NULL allowed when n = 0; index = the point's
  * position in d_points, with the same labels and ids as rtdbs_load_window +
  * rtdbs_cluster on a window of n slots).  Working memory is one static
- * device array of about 3.4 MB, part of the library: every GPU that loads the
+ * device array of about 3.3 MB, part of the library: every GPU that loads the
  * library holds it until the process exits.  The first call on a device looks up that array's device
  * address, with that device current.  All calls share the array: calls whose
  * work overlaps on a GPU race and corrupt each other's results, so serialise
@@ -258,7 +257,7 @@ RTDBS_API int rtdbs_cluster_window_noalloc(const float* d_points, int32_t n, int
  * host memory; points outside it fall into its edge cells and are still
  * clustered exactly, a tight box just keeps the grid small) and a device int
  * *d_status, which receives the device error bits (0: success; 1 table full,
- * 2 union-find bound, 4 work list full, 8 chunk bookkeeping) in stream order.
+ * 2 union-find bound, 8 chunk bookkeeping) in stream order.
  * Everything is queued on cuda_stream and the call returns; the outputs and
  * *d_status are ready when the stream reaches that point.  Calls share the
  * scratch array with rtdbs_cluster_window_noalloc: serialise them (calls on

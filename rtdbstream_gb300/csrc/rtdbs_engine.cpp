@@ -228,16 +228,11 @@ size_t plan_layout(rtdbs_engine* e, std::vector<Part>& parts) {
     }
     v.pbits = pbits;
     v.pmask = (unsigned)(P - 1);
-    // work items: cell runs cut at 32 points, at 8 below 65,536 points (a small
-    // window is a few waves of items at most, so its densest cells must not
-    // be one warp's long chain)
-    v.item_pts = W < 65536 ? 8 : 32;
     // blocks of the union: 16 positions on small windows (2,000 warps at most,
     // so shorter chains count for more than fuller lookups: 10k points in 3-D,
     // union 45 -> 37 us, 2-D 33 -> 31), 32 above (48k points 51 -> 45 us, 1M
     // walkers 186 -> 168)
     v.block_pts = W < 32768 ? 16 : 32;
-    v.max_items = W + W / v.item_pts + 64;
     // Neighbour lists of non-core points (MinPts - 2 entries each) replace the
     // label pass's grid scan up to kListCap entries; above that the scan stays.
     const int mp = e->p.min_pts;
@@ -258,7 +253,6 @@ size_t plan_layout(rtdbs_engine* e, std::vector<Part>& parts) {
         {(void**)&v.scnt[1], sizeof(int) * W},
         {(void**)&v.table[0], sizeof(ulonglong2) * P},
         {(void**)&v.table[1], sizeof(ulonglong2) * P},
-        {(void**)&v.items, sizeof(int2) * v.max_items},
         {(void**)&v.parent, sizeof(int) * W},
         {(void**)&v.sroot, sizeof(int) * W},
         {(void**)&v.label, sizeof(int) * W},
@@ -307,7 +301,7 @@ int allocate(rtdbs_engine* e) {
 int check_device_error(rtdbs_engine* e) {
     if (e->h_ctl->err)
         return fail(RTDBS_ERR_DEVICE, "device error bits 0x%x (1 table full, 2 union-find bound, "
-                    "4 work list full, 8 chunk bookkeeping, 16 neighbour lists)", e->h_ctl->err);
+                    "8 chunk bookkeeping, 16 neighbour lists)", e->h_ctl->err);
     return RTDBS_OK;
 }
 

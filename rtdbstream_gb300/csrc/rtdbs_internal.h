@@ -12,7 +12,6 @@
 //                         tmp_pos_arr, src/dbscan/grid.cpp:181-199)
 //   table  {u64,u64}[2][P] open-addressed cell table: tagged key -> [start,end)
 //                         (replaces the OptiX BVH, src/dbscan/optix.cpp:438-483)
-//   items  int2[W+W/32+64] work list: runs of <= 32 sorted points of one cell
 //   parent i32[W]         union-find forest by slot (reference: cluster_id)
 //   sroot  i32[W]         per sorted position: root hint during the union, then
 //                         the root (-1: not core)
@@ -45,8 +44,6 @@ constexpr int kSortRun = 1024;     // words per radix-sort CTA (one per thread)
 constexpr int kBuildThreads = 512;
 constexpr int kClusterThreads = 256;
 constexpr int kLinkThreads = 256;
-constexpr int kBatch = 8;          // default work items a clustering warp takes at a time
-                                   // in a pool launch
 constexpr int kQueryLanes = 16;    // lanes per query point in the count passes where the queries
                                    // fill the GPU (one cell per Eps: two points per warp
                                    // overlap their loads)
@@ -56,7 +53,6 @@ constexpr int kListCap = 30;       // longest neighbour list kept (MinPts <= 32)
 // Bits of Ctl::err.
 constexpr int kErrHashFull = 1;
 constexpr int kErrUnionIter = 2;
-constexpr int kErrItems = 4;
 constexpr int kErrChunk = 8;
 constexpr int kErrList = 16;
 
@@ -67,13 +63,12 @@ struct Ctl {
     long long b;               // grid builds so far (merge + table build)
     long long slide;           // slides completed
     int nocc[2];               // entries in sorted buffer 0 / 1
-    int nitems;                // work items of the current grid
+    int nitems;                // cell runs (within 32 sorted positions) of the current grid
     int ncells;                // cells of the current grid
     int err;                   // kErr* bits
     int prev_ok;               // label/cid hold the clustering of the window before
                                // this slide's changes (the forest can be reused)
-    int union_next;            // next work item handed out by k_union
-    int label_next;            // next work item handed out by k_label
+    int union_next;            // next block of positions handed out by k_union
     unsigned long long band_rechecks;
     // counters of the reference's debug build (src/dbscan/dbscan.cpp:145-212):
     // [0] count passes (core identification), [1] clustering scans; spread over 8
@@ -97,9 +92,8 @@ struct View {
     int shift[3];
     int dim;
     int cell_mult;              // K: cells per Eps along each axis (1 or 2)
-    int grab;                   // work items a clustering warp takes from the queue at a time
-                                // (0: 8 in pool launches, fewer on small windows slid alone;
-                                // the union: one block of positions per 16)
+    int grab;                   // cell runs a union warp takes from the queue at a time (whole
+                                // blocks of positions: one per 16 runs, at least one)
     int qlanes;                 // lanes per query point in the count passes (16 or 32)
     // parameters
     int W, S, min_pts, units;   // units = W / S
@@ -112,10 +106,6 @@ struct View {
     int filter_ok;              // FP64 mode: band valid (else every test in FP64)
     int key_bits;
     int sort_passes;
-    int max_items;
-    int item_pts;               // most points of a work item slid alone (8 or 32; 0 = 32; pool
-                                // launches take 32): small windows take short items, so
-                                // dense cells spread over more warps
     int block_pts;              // sorted positions a union warp takes as one block (16 or 32;
                                 // pool launches take 32)
     int precision;              // RTDBS_PREC_* (batched launches dispatch on it)
@@ -129,7 +119,6 @@ struct View {
     float4* spt[2];
     int* scnt[2];
     ulonglong2* table[2];
-    int2* items;
     int* parent;
     int* sroot;                  // per sorted position: root hint during the union
                                  // (-1: not core), then the root (-1: not core)

@@ -1105,7 +1105,6 @@ __device__ __forceinline__ void merge_body(const View& v, int j, int c, int init
         v.ctl->nitems = 0;
         v.ctl->ncells = 0;
         v.ctl->union_next = 0;
-        v.ctl->label_next = 0;
     }
     // Table generations wrap every kGenMod builds of a table: clear it then.
     if (b >= 2 && ((b >> 1) % (long long)kGenMod) == 0) {
@@ -1257,21 +1256,21 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge(View v, int j, int c, i
     merge_body(v, j, c, init, blockIdx.x, gridDim.x, sm);
 }
 
-// Cell table and work list of the new sorted window.  A work item is a
-// maximal run of one cell inside a 32-aligned block of sorted positions.
-// Item and cell counters are reserved once per block.
+// Cell table of the new sorted window.  A cell that starts and ends in one
+// warp's positions is entered once, by its first point; otherwise its first
+// point enters the start, its last the end.  Cells and cell runs (within 32
+// positions) are counted once per block.  Bound by the latency of the inserts
+// (a read, a CAS and a store to a random slot): 1M walkers, 275k cells, 25 us
+// (29 with a work list of cell runs for the union and the label pass, which
+// now take blocks of positions).
 struct BuildSmem {
-    int wcount[kBuildThreads / 32];
-    int wbase[kBuildThreads / 32];
-    int bcells;
+    int cells, runs;
 };
 
-// (pooled: a pool launch, whose many streams fill the GPU: 32-point items)
-__device__ __forceinline__ void build_body(const View& v, int bx, BuildSmem& sm, bool pooled) {
-    int* wcount = sm.wcount;
-    int* wbase = sm.wbase;
-    int& bcells = sm.bcells;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+__device__ __forceinline__ void build_body(const View& v, int bx, BuildSmem& sm) {
+    if (threadIdx.x == 0) sm.cells = sm.runs = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
     const int gw = (bx * blockDim.x + threadIdx.x) >> 5;
     const long long b = v.ctl->b;
     const int cur = (int)(b & 1);
@@ -1287,13 +1286,16 @@ __device__ __forceinline__ void build_body(const View& v, int bx, BuildSmem& sm,
     if (lane == 31) kn = (i + 1 < n) ? skey[i + 1] : ~0ull;
     const bool first = valid && (i == 0 || kp != k);
     const bool last = valid && (i == n - 1 || kn != k);
+    const unsigned firsts = __ballot_sync(kFull, first);
+    const unsigned lasts = __ballot_sync(kFull, last);
+    if (lane == 0) {
+        const int runs = __popc(firsts | (valid ? 1u : 0u));
+        if (firsts) atomicAdd(&sm.cells, __popc(firsts));
+        if (runs) atomicAdd(&sm.runs, runs);
+    }
     int err = 0;
     ulonglong2* T = v.table[cur];
     const unsigned long long tag = tag_of(k & kKeyMask, gen);
-    // A cell that starts and ends in this warp is entered once, by its first
-    // point; otherwise its first point enters the start, its last the end.
-    const unsigned firsts = __ballot_sync(kFull, first);
-    const unsigned lasts = __ballot_sync(kFull, last);
     if (first) {
         const unsigned ends = lasts & ~((1u << lane) - 1u);  // my cell's last is the lowest
         const bool ok = ends ? table_set(T, v.pmask, v.pbits, tag, 2, i, gw * 32 + __ffs(ends))
@@ -1302,43 +1304,19 @@ __device__ __forceinline__ void build_body(const View& v, int bx, BuildSmem& sm,
     }
     if (last && !(firsts & ((2u << lane) - 1u)) && !table_set(T, v.pmask, v.pbits, tag, 1, i + 1))
         err |= kErrHashFull;
-    const int ip = (!pooled && v.item_pts > 0) ? v.item_pts : 32;
-    const unsigned starts = __ballot_sync(kFull, valid && (first || (lane & (ip - 1)) == 0));
-    const int nfirst = __popc(__ballot_sync(kFull, first));
-    if (threadIdx.x == 0) bcells = 0;
-    if (lane == 0) wcount[wib] = __popc(starts);
-    __syncthreads();
-    if (lane == 0 && nfirst) atomicAdd(&bcells, nfirst);
-    if (threadIdx.x == 0) {
-        int tot = 0;
-        for (int w = 0; w < kBuildThreads / 32; ++w) {
-            wbase[w] = tot;
-            tot += wcount[w];
-        }
-        const int base = tot ? atomicAdd(&v.ctl->nitems, tot) : 0;
-        for (int w = 0; w < kBuildThreads / 32; ++w) wbase[w] += base;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0 && bcells) atomicAdd(&v.ctl->ncells, bcells);
-    if (bx == 0 && threadIdx.x == 0) v.ctl->b_done = b;  // not read here
-    if (valid && (first || (lane & (ip - 1)) == 0)) {
-        const int rank = __popc(starts & lanemask_lt(lane));
-        const unsigned above = starts & ~((2u << lane) - 1u);
-        const int next = above ? gw * 32 + __ffs(above) - 1 : gw * 32 + 32;
-        const int end = min(next, n);
-        const int slot = wbase[wib] + rank;
-        if (slot < v.max_items)
-            v.items[slot] = make_int2(i, end - i);
-        else
-            err |= kErrItems;
-    }
     if (err) atomicOr(&v.ctl->err, err);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (sm.cells) atomicAdd(&v.ctl->ncells, sm.cells);
+        if (sm.runs) atomicAdd(&v.ctl->nitems, sm.runs);
+        if (bx == 0) v.ctl->b_done = b;  // not read here
+    }
 }
 
 __global__ void __launch_bounds__(kBuildThreads) k_build(View v) {
     pdl_wait();
     __shared__ BuildSmem sm;
-    build_body(v, blockIdx.x, sm, false);
+    build_body(v, blockIdx.x, sm);
 }
 
 // Full count of each new point and +1 on every older neighbour (new grid).
@@ -1662,7 +1640,6 @@ __global__ void k_fill(View v, int ob, int passes) {
         v.ctl->nitems = 0;
         v.ctl->ncells = 0;
         v.ctl->union_next = 0;
-        v.ctl->label_next = 0;
     }
     // table generations wrap every kGenMod builds of a table, as in the merge
     if (b >= 2 && ((b >> 1) % (long long)kGenMod) == 0) {
@@ -1975,22 +1952,6 @@ __global__ void __launch_bounds__(kLinkThreads) k_link(View v) {
     link_body<MODE, DK>(v, blockIdx.x, sm);
 }
 
-struct ClusterSmem {
-    float4 home_pt[kClusterThreads / 32][32];
-    int rstart[kClusterThreads / 32][kMaxRows], rpre[kClusterThreads / 32][kMaxRows + 1];
-};
-
-// Work items the label scan's warps take at a time: the stream's setting, or
-// by default 8 in a pool launch (many streams share the GPU); for a single
-// stream up to 8 on large windows, fewer on small ones (a 10k-point window has
-// a few hundred to a few thousand items: 8 per grab would leave them to a few
-// dozen warps).
-__device__ __forceinline__ int work_grab(const View& v, bool pooled) {
-    if (v.grab > 0) return v.grab;
-    if (pooled) return kBatch;
-    return max(1, min(kBatch, v.W >> 14));
-}
-
 // Blocks of positions a union warp takes at a time: one, as a block holds
 // about 8 cell runs (2 blocks: walkers 168 -> 178 us, trajectories 79 -> 109);
 // the stream's setting counts cell runs.
@@ -2262,7 +2223,6 @@ __device__ __forceinline__ void rebuild_list(const View& v, int at, int cur, uns
 template <int MODE, int DK>
 __device__ __forceinline__ void flatten_body(const View& v, int bx, int nbx, StreamSmem& sm) {
     constexpr int DIM = DK & 3, K = (DK >> 2) + 1;  // dimension, cells per Eps
-    if (bx == 0 && threadIdx.x == 0) v.ctl->label_next = 0;  // k_label's queue; not read here
     const long long b = v.ctl->b;
     const int cur = (int)(b & 1);
     const int n = v.ctl->nocc[cur];
@@ -2332,89 +2292,136 @@ __global__ void __launch_bounds__(256, 6) k_flatten(View v) {
 }
 
 // Labels and ids by slot: core -> 0 and its root; non-core -> 1 and the
-// minimum root over adjacent cores, or 2 and its own slot.
-template <int MODE, int DK>
-__device__ __forceinline__ void label_body(const View& v, int advance, int bx, ClusterSmem& sm, int grab) {
+// minimum root over adjacent cores, or 2 and its own slot.  As in the count, a
+// warp takes a block of consecutive sorted positions, whose non-core points
+// with neighbours are its home points, and walks the whole stencil of their
+// cells as one candidate stream; a core candidate is tested against those
+// home points of its segment whose minimum it would lower.  Bound by load
+// latency.
+template <int DIM, int K>
+struct LabelSmem {
+    using C = CountShape<DIM, K>;
+    static constexpr int kWarps = kClusterThreads / 32;
+    float4 pt[kWarps][C::kBlock];
+    unsigned long long skey[kWarps][C::kBlock];
+    unsigned segm[kWarps][C::kBlock];  // home points of a segment
+    int best[kWarps][C::kBlock];       // minimum root near a home point
+    int tstart[kWarps][C::kTasks];
+    int tpre[kWarps][C::kTasks + 1];
+    unsigned char tseg[kWarps][C::kTasks];
+};
+
+template <int MODE, int DK, class Smem>
+__device__ __forceinline__ void label_body(const View& v, int advance, int bx, int nbx, Smem& sm, int P) {
     constexpr int DIM = DK & 3, K = (DK >> 2) + 1;  // dimension, cells per Eps
-    int(&rstart)[kClusterThreads / 32][kMaxRows] = sm.rstart;
-    int(&rpre)[kClusterThreads / 32][kMaxRows + 1] = sm.rpre;
-    float4(&home_pt)[kClusterThreads / 32][32] = sm.home_pt;
+    constexpr int R = CountShape<DIM, K>::kRows;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const float4* hpt = home_pt[wib];
+    float4* hpt = sm.pt[wib];
+    unsigned* segm = sm.segm[wib];
+    int* best = sm.best[wib];
+    int* tstart = sm.tstart[wib];
+    int* tpre = sm.tpre[wib];
+    unsigned char* tseg = sm.tseg[wib];
     const long long b = v.ctl->b;
     const int cur = (int)(b & 1);
     const unsigned gen = gen_of_build(b);
-    const int nitems = min(v.ctl->nitems, v.max_items);
+    const int n = v.ctl->nocc[cur];
+    const int nblk = (n + P - 1) / P, step = nbx * (kClusterThreads / 32);
     const float4* spt = v.spt[cur];
     const int* sroot = v.sroot;
-    const unsigned long long* skey = v.skey[cur];
-    const ulonglong2* T = v.table[cur];
     Tally tally;
-    int it1 = 0;
-    for (int itx = nitems;;) {
-        if (itx >= it1) {
-            int got = 0;
-            if (lane == 0) got = atomicAdd(&v.ctl->label_next, grab);
-            itx = __shfl_sync(kFull, got, 0);
-            if (itx >= nitems) break;
-            it1 = min(itx + grab, nitems);
-        }
-        const int2 item = v.items[itx++];
-        const int start = item.x, len = item.y;
-        const bool hv = lane < len;
+    for (int bk = bx * (kClusterThreads / 32) + wib; bk < nblk; bk += step) {
+        const int i = bk * P + lane;
+        const bool hv = lane < P && i < n;
         float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
-        int hslot = -1, hr = -1;
-        bool lonely = false;
+        bool home = false;
+        unsigned long long key = 0;
+        int hslot = -1;
         if (hv) {
-            h = spt[start + lane];
+            h = spt[i];
             hslot = slot_of(h);
-            hr = sroot[start + lane];
-            if (hr >= 0) {
-                v.label[hslot] = 0;
-                v.cid[hslot] = hr;
-            } else if (v.scnt[cur][start + lane] <= 1) {
-                // no neighbour but itself: noise without a scan
-                lonely = true;
-                v.label[hslot] = 2;
-                v.cid[hslot] = hslot;
+            const int hr = sroot[i];
+            // (a point with no neighbour but itself is noise without a scan)
+            home = hr < 0 && v.scnt[cur][i] > 1;
+            if (!home) {
+                v.label[hslot] = hr >= 0 ? 0 : 2;
+                v.cid[hslot] = hr >= 0 ? hr : hslot;
+            } else {
+                key = v.skey[cur][i];
             }
         }
-        const unsigned nmask = __ballot_sync(kFull, hv && hr < 0 && !lonely);
-        if (!nmask) continue;
+        const unsigned hmask = __ballot_sync(kFull, home);
+        if (!hmask) continue;
+        // segments: the home points of one cell
+        const unsigned below = hmask & lanemask_lt(lane);
+        const unsigned long long kprev = __shfl_sync(kFull, key, below ? 31 - __clz(below) : lane);
+        const unsigned leaders = __ballot_sync(kFull, home && (!below || kprev != key));
+        const int ns = __popc(leaders);
+        if (home) {
+            hpt[lane] = h;
+            best[lane] = INT_MAX;
+        }
+        if ((leaders >> lane) & 1u) {
+            const unsigned later = leaders & ~((2u << lane) - 1u);
+            const int at = __popc(leaders & lanemask_lt(lane));
+            segm[at] = hmask & ~lanemask_lt(lane) & (later ? lanemask_lt(__ffs(later) - 1) : kFull);
+            sm.skey[wib][at] = key;
+        }
         __syncwarp();
-        home_pt[wib][lane] = h;
-        int rs, re;
-        row_ranges<DIM, false, K>(v, T, gen, skey[start], lane, rs, re);
-        const int total = candidate_stream<Stencil<DIM, false, K>::kRows>(rs, re, 0, lane, rstart[wib], rpre[wib]);
-        int best = INT_MAX, r = 0;
+        int nt = 0, total = 0;
+        for (int t0 = 0; t0 < ns * R; t0 += 32) {
+            const int t = t0 + lane, seg = t / R;
+            int a = 0, len = 0;
+            if (t < ns * R) {
+                const int2 rr = row_range_lane<DIM, false, K>(v, v.table[cur], gen, sm.skey[wib][seg], t - seg * R);
+                a = rr.x;
+                len = rr.y - rr.x;
+            }
+            int incl = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int x = __shfl_up_sync(kFull, incl, o);
+                if (lane >= o) incl += x;
+            }
+            const unsigned some = __ballot_sync(kFull, len > 0);
+            if (len > 0) {
+                const int at = nt + __popc(some & lanemask_lt(lane));
+                tstart[at] = a;
+                tpre[at] = total + incl - len;
+                tseg[at] = (unsigned char)seg;
+            }
+            nt += __popc(some);
+            total += __shfl_sync(kFull, incl, 31);
+        }
+        if (lane == 0) tpre[nt] = total;
+        __syncwarp();
+        int r = 0;
         for (int base = 0; base < total; base += 32) {
             const int idx = base + lane;
-            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+            unsigned mm = 0;
             int qr = -1;
+            float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
             if (idx < total) {
-                const int pos = stream_pos(idx, r, rstart[wib], rpre[wib]);
+                while (idx >= tpre[r + 1]) ++r;
+                const int pos = tstart[r] + idx - tpre[r];
                 qr = sroot[pos];
                 q = spt[pos];
+                if (qr >= 0) mm = segm[tseg[r]];
             }
-            if (!__any_sync(kFull, qr >= 0)) continue;
-            unsigned mm = nmask;
             while (mm) {
                 const int hi = __ffs(mm) - 1;
                 mm &= mm - 1;
-                const int val = (qr >= 0 && is_nbr<MODE, DIM>(v, hpt[hi], q, tally)) ? qr : INT_MAX;
-                const int mn = (int)__reduce_min_sync(kFull, (unsigned)val);
-                if (lane == hi) best = min(best, mn);
+                if (qr < *(volatile int*)&best[hi] && is_nbr<MODE, DIM>(v, hpt[hi], q, tally))
+                    atomicMin(&best[hi], qr);
             }
         }
-        if (hv && hr < 0 && !lonely) {
-            if (best != INT_MAX) {
-                v.label[hslot] = 1;
-                v.cid[hslot] = best;
-            } else {
-                v.label[hslot] = 2;
-                v.cid[hslot] = hslot;
-            }
+        __syncwarp();
+        if (home) {
+            const int to = best[lane];
+            v.label[hslot] = to != INT_MAX ? 1 : 2;
+            v.cid[hslot] = to != INT_MAX ? to : hslot;
         }
+        __syncwarp();
     }
     flush_stats(v, tally, 0, lane, 1);
     if (bx == 0 && threadIdx.x == 0) {
@@ -2423,11 +2430,19 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, C
     }
 }
 
+// Positions a label warp takes as one block (at most CountShape's): short
+// chains on small windows (48k points, 4 / 8 / 16 / 32: 16 / 14 / 21 / 25 us; a
+// queue of single cells took 18).
+__host__ __device__ __forceinline__ int label_block(const View& v, bool pooled) {
+    const int most = v.dim == 3 && v.cell_mult == 2 ? 16 : 32;
+    return pooled ? most : min(most, v.W < 65536 ? 8 : 32);
+}
+
 template <int MODE, int DK>
-__global__ void __launch_bounds__(kClusterThreads, 6) k_label(View v, int advance) {
+__global__ void __launch_bounds__(kClusterThreads, 4) k_label(View v, int advance) {
     pdl_wait();
-    __shared__ ClusterSmem sm;
-    label_body<MODE, DK>(v, advance, blockIdx.x, sm, work_grab(v, false));
+    __shared__ LabelSmem<(DK & 3), (DK >> 2) + 1> sm;
+    label_body<MODE, DK>(v, advance, blockIdx.x, gridDim.x, sm, label_block(v, false));
 }
 
 // Outputs by slot from the roots and the lists: core -> 0 and its root; a
@@ -2501,7 +2516,7 @@ template <> struct PhaseShape<kBatchIncrement> { static constexpr int threads = 
 template <> struct PhaseShape<kBatchLink> { static constexpr int threads = kLinkThreads, min_blocks = 1; };
 template <> struct PhaseShape<kBatchUnion> { static constexpr int threads = kClusterThreads, min_blocks = kUnionBlocks; };
 template <> struct PhaseShape<kBatchFlatten> { static constexpr int threads = 256, min_blocks = 6; };
-template <> struct PhaseShape<kBatchLabel> { static constexpr int threads = kClusterThreads, min_blocks = 6; };
+template <> struct PhaseShape<kBatchLabel> { static constexpr int threads = kClusterThreads, min_blocks = 5; };
 
 // One phase over many streams.  The block finds its item, copies that
 // stream's View into shared memory and runs the stream's kernel body.
@@ -2554,7 +2569,7 @@ __global__ void __launch_bounds__(PhaseShape<PHASE>::threads, PhaseShape<PHASE>:
         merge_body(sv, it.j, it.c, 0, bx, nbx, sm);
     } else if constexpr (PHASE == kBatchBuild) {
         __shared__ BuildSmem sm;
-        build_body(sv, bx, sm, true);
+        build_body(sv, bx, sm);
     } else if constexpr (PHASE == kBatchIncrement) {
         __shared__ StreamSmem sm;
         incr_body<MODE, DK>(sv, it.j, it.c, 0, bx, sm);
@@ -2568,11 +2583,11 @@ __global__ void __launch_bounds__(PhaseShape<PHASE>::threads, PhaseShape<PHASE>:
         __shared__ StreamSmem sm;
         flatten_body<MODE, DK>(sv, bx, nbx, sm);
     } else {
-        __shared__ ClusterSmem sm;
+        __shared__ LabelSmem<(DK & 3), (DK >> 2) + 1> sm;
         if (sv.list_cap >= 0)
             border_body(sv, 1, bx, nbx);
         else
-            label_body<MODE, DK>(sv, 1, bx, sm, work_grab(sv, true));
+            label_body<MODE, DK>(sv, 1, bx, nbx, sm, label_block(sv, true));
     }
 }
 
@@ -2692,18 +2707,18 @@ cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, 
                 launch(k_border, max(1, min(sms * 8, (v.W + 255) / 256)), 256, 0, s, pdl, v, advance);
                 break;
             }
-            [[fallthrough]];
+            {
+                const int per = label_block(v, false) * (kClusterThreads / 32);  // positions per thread block
+                RTDBS_DISPATCH(precision, dk_of(v), k_label, (v.W + per - 1) / per, kClusterThreads, s, pdl, v, advance);
+            }
+            break;
         case kPhaseUnion: {
+            // queue-fed blocks, as many as the window has or the SMs hold
             const int sms = g_num_sms > 0 ? g_num_sms : 152;
-            // queue-fed blocks: one warp per ~12 window points (a few items
-            // each on sparse windows), all the SMs hold on large ones
-            const int need = (v.W + 95) / 96;
-            const int blocks = max(1, min(sms * 6, need));
-            if (phase == kPhaseUnion) {
-                RTDBS_DISPATCH(precision, dk_of(v), k_link, (v.W + kLinkThreads - 1) / kLinkThreads, kLinkThreads, s, pdl, v);
-                RTDBS_DISPATCH(precision, dk_of(v), k_union, max(1, min(sms * kUnionBlocks, (v.W + v.block_pts * 8 - 1) / (v.block_pts * 8))), kClusterThreads, s, pdl, v);
-            } else
-                RTDBS_DISPATCH(precision, dk_of(v), k_label, blocks, kClusterThreads, s, pdl, v, advance);
+            const int per = v.block_pts * (kClusterThreads / 32);
+            const int blocks = max(1, min(sms * kUnionBlocks, (v.W + per - 1) / per));
+            RTDBS_DISPATCH(precision, dk_of(v), k_link, (v.W + kLinkThreads - 1) / kLinkThreads, kLinkThreads, s, pdl, v);
+            RTDBS_DISPATCH(precision, dk_of(v), k_union, blocks, kClusterThreads, s, pdl, v);
             break;
         }
         case kPhaseFlatten: {
@@ -2886,7 +2901,7 @@ int batch_blocks(int phase, const View& v, int c) {
         case kBatchLabel:
             if (v.list_cap >= 0) return max(1, min(1024, (v.W + 1023) / 1024));  // k_border
             return max(1, min(1024, (v.W + 4095) / 4096));  // persistent, queue-fed
-        case kBatchFlatten: return max(1, min(1024, (v.W + 2047) / 2048));
+        case kBatchFlatten: return max(1, min(1024, (v.W + 1023) / 1024));  // (2,048 points a block: 74 us a round against 55)
         default: return 0;
     }
 }

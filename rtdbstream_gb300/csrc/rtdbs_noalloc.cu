@@ -30,7 +30,6 @@ constexpr int kMaxPoints = RTDBS_NOALLOC_MAX_POINTS;
 static_assert(kMaxPoints <= rtdbs::kChunkMax, "one grid-update chunk must hold the window");
 constexpr unsigned long long kTableSlots = 32768;  // power of two >= 2 * kMaxPoints
 static_assert(kTableSlots >= 2ull * kMaxPoints, "table capacity");
-constexpr int kMaxItems = kMaxPoints + kMaxPoints / 32 + 64;
 
 constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
@@ -45,8 +44,7 @@ constexpr size_t kOffScnt0 = kOffSpt1 + align256(sizeof(float4) * kMaxPoints);
 constexpr size_t kOffScnt1 = kOffScnt0 + align256(sizeof(int) * kMaxPoints);
 constexpr size_t kOffTable0 = kOffScnt1 + align256(sizeof(int) * kMaxPoints);
 constexpr size_t kOffTable1 = kOffTable0 + align256(sizeof(ulonglong2) * kTableSlots);
-constexpr size_t kOffItems = kOffTable1 + align256(sizeof(ulonglong2) * kTableSlots);
-constexpr size_t kOffParent = kOffItems + align256(sizeof(int2) * kMaxItems);
+constexpr size_t kOffParent = kOffTable1 + align256(sizeof(ulonglong2) * kTableSlots);
 constexpr size_t kOffSroot = kOffParent + align256(sizeof(int) * kMaxPoints);
 constexpr size_t kOffNsort = kOffSroot + align256(sizeof(int) * kMaxPoints);
 constexpr size_t kOffXsort = kOffNsort + align256(sizeof(unsigned long long) * kMaxPoints);
@@ -55,7 +53,7 @@ constexpr size_t kOffXword = kOffNword + align256(sizeof(unsigned long long) * k
 constexpr size_t kOffXpt = kOffXword + align256(sizeof(unsigned long long) * kMaxPoints);
 constexpr size_t kOffBox = kOffXpt + align256(sizeof(float4) * kMaxPoints);
 constexpr size_t kOffCtl = kOffBox + align256(sizeof(float) * 6);
-constexpr size_t kScratchBytes = kOffCtl + align256(sizeof(Ctl));  // about 3.4 MB
+constexpr size_t kScratchBytes = kOffCtl + align256(sizeof(Ctl));  // about 3.3 MB
 
 // The working memory.  In host code this name is only a host-side stand-in
 // for the device array: its device address comes from cudaGetSymbolAddress.
@@ -162,8 +160,6 @@ int window_view(View& v, unsigned char* base, const float* d_points, int n, int 
     if (rc != RTDBS_OK) return rc;
     v.pbits = 15;
     v.pmask = (unsigned)(kTableSlots - 1);
-    v.max_items = kMaxItems;
-    v.item_pts = 32;
     v.block_pts = 16;
     v.list_cap = -1;  // no neighbour lists: the label pass scans the grid
     v.list_stride = 0;
@@ -179,7 +175,6 @@ int window_view(View& v, unsigned char* base, const float* d_points, int n, int 
     v.scnt[1] = reinterpret_cast<int*>(base + kOffScnt1);
     v.table[0] = reinterpret_cast<ulonglong2*>(base + kOffTable0);
     v.table[1] = reinterpret_cast<ulonglong2*>(base + kOffTable1);
-    v.items = reinterpret_cast<int2*>(base + kOffItems);
     v.parent = reinterpret_cast<int*>(base + kOffParent);
     v.sroot = reinterpret_cast<int*>(base + kOffSroot);
     v.label = d_label;
@@ -257,7 +252,7 @@ extern "C" RTDBS_API int rtdbs_cluster_window_noalloc(const float* d_points, int
 #undef NOALLOC_TRY
     if (err)
         return set_error(RTDBS_ERR_DEVICE, "noalloc: device error bits 0x%x (1 table full, 2 union-find bound, "
-                         "4 work list full, 8 chunk bookkeeping)", err);
+                         "8 chunk bookkeeping)", err);
     return RTDBS_OK;
 }
 
