@@ -187,6 +187,9 @@ RTDBS_API int rtdbs_slide(rtdbs_engine* engine, const float* new_points, int32_t
                 int32_t* cluster_id);
 
 /* Same slide with device pointers, stream-ordered, no host synchronisation.
+ * d_new_points is read, and label/cluster_id are written, by the slide's own
+ * kernels where they are 4-byte aligned memory of the engine's device, and
+ * through copies otherwise; all three stay in use until the slide has run.
  * label/cluster_id may be NULL: the result then stays in the engine's own
  * buffers (rtdbs_device_outputs). */
 RTDBS_API int rtdbs_slide_async(rtdbs_engine* engine, const float* d_new_points, int32_t* d_label,

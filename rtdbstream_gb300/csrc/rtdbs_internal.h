@@ -79,7 +79,20 @@ struct Ctl {
     int reuse_skip;            // slides left without forest reuse (it paid off too little)
     long long last_reused;     // `reused` of the last clustering
     long long kept_from;       // first slide since when every slide kept its chunks' orders
+    const float* input;        // new points of this slide
+    int* out_label;            // caller's outputs of this slide or clustering, written beside
+    int* out_cid;              // label and cid (null: none)
     long long b_done;          // builds whose table is in place (b, while no build is under way)
+};
+
+// What a slide or a clustering exchanges with its caller: the kernels read the
+// new points and write the results there, so no copies run around them.  All
+// pointers are accessible to the kernels (device memory, or pinned host
+// memory); label / cid may be null.
+struct SlideIO {
+    const float* input;
+    int* label;
+    int* cid;
 };
 
 // Everything a kernel needs for one stream, passed by value.
@@ -166,20 +179,26 @@ constexpr int kChunkPhases = 6;  // ingest .. increment, once per chunk
 // Launchers (rtdbs_kernels.cu).  j = chunk index within the slide (or the
 // load), c = points in the chunk, init = 1 while loading the first window,
 // advance = 1 when the label phase ends a slide.
+// io: for the ingest (input null: the one that the slide's first ingest left in
+// the control block).
 cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, int init,
-                         int staging_offset, int advance, cudaStream_t s, bool pdl = false);
+                         int staging_offset, int advance, cudaStream_t s, bool pdl = false,
+                         const SlideIO& io = SlideIO{});
 // With a side stream and two events, the decrement pass (which needs only
 // the ingest) runs on `side` beside the sort, joined before the merge.  pdl:
 // programmatic dependence on the kernel launched before on the same stream.
+// ingested: the chunk's ingest has been launched already (outside a captured
+// graph, as its arguments change from slide to slide).
 cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int init,
-                              int staging_offset, cudaStream_t s, cudaStream_t side = nullptr,
-                              cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
+                              int staging_offset, cudaStream_t s, const SlideIO& io, bool ingested = false,
+                              cudaStream_t side = nullptr, cudaEvent_t fork = nullptr,
+                              cudaEvent_t join = nullptr);
 // The grid of all W slots built at once (see the kernels): slots
-// [0, count) while loading (init), else the slide's slots, take the points at
-// `input` (device memory, count = S in a slide).
-cudaError_t launch_window_build(const View& v, int precision, const float* input, int count, int init,
-                                cudaStream_t s);
-cudaError_t launch_window_phase(int phase, const View& v, int precision, const float* input, int count, int init,
+// [0, count) while loading (init), else the slide's slots, take the new points
+// (count = S in a slide).
+cudaError_t launch_window_build(const View& v, int precision, const SlideIO& io, int count, int init,
+                                cudaStream_t s, bool ingested = false);
+cudaError_t launch_window_phase(int phase, const View& v, int precision, const SlideIO& io, int count, int init,
                                 cudaStream_t s, bool pdl = false);
 int window_build_launches(const View& v);
 // Bounding box of n points per axis as order-keeping unsigned keys: minima
@@ -195,11 +214,13 @@ inline bool window_build_fits(const View& v) {
     return v.W <= kChunkMax || v.key_bits + slot_bits(v.W) <= 64;
 }
 // fresh_hints: start the union from fresh hints and forest (no reuse), for a
-// clustering of the window as it stands rather than after a slide.
+// clustering of the window as it stands rather than after a slide, with its
+// outputs in io (a slide's io goes to its ingest).
 // outputs_free: an event the label pass (which rewrites label/cid) waits for
 // first, with wait_flags (cudaEventWaitExternal inside a stream capture).
 cudaError_t launch_cluster(const View& v, int precision, int advance, cudaStream_t s, bool fresh_hints = false,
-                           cudaEvent_t outputs_free = nullptr, unsigned wait_flags = 0);
+                           cudaEvent_t outputs_free = nullptr, unsigned wait_flags = 0,
+                           const SlideIO& io = SlideIO{});
 cudaError_t launch_counts_by_slot(const View& v, int* nn_by_slot, cudaStream_t s);
 cudaError_t configure_kernels();
 

@@ -710,9 +710,19 @@ __device__ __forceinline__ void mark_damage(const View& v, int slot) {
 
 // New points of chunk j -> ring slots [el, el+c): float4 + cell key; the
 // points they replace are kept for the decrement pass.
-__device__ __forceinline__ void ingest_body(const View& v, int j, int c, int init, int stg_off,
-                                            const float* input, int bx) {
-    if (bx == 0 && threadIdx.x == 0) v.ctl->b += 1;  // no reader in this kernel
+// The slide's first ingest (an input given) leaves the slide's pointers in the
+// control block for the later ones and the label pass.
+__device__ __forceinline__ void ingest_body(const View& v, int j, int c, int init, int stg_off, const SlideIO& io,
+                                            int bx) {
+    const float* input = io.input ? io.input : v.ctl->input;
+    if (bx == 0 && threadIdx.x == 0) {
+        v.ctl->b += 1;  // no reader in this kernel
+        if (io.input) {
+            v.ctl->input = io.input;  // (its readers here have the argument)
+            v.ctl->out_label = io.label;
+            v.ctl->out_cid = io.cid;
+        }
+    }
     const int k = bx * blockDim.x + threadIdx.x;
     if (k >= c) return;
     const int slot = chunk_base_slot(v, j, init) + k;
@@ -731,9 +741,9 @@ __device__ __forceinline__ void ingest_body(const View& v, int j, int c, int ini
     v.nsort[k] = (key << kOffBits) | (unsigned long long)k;
 }
 
-__global__ void k_ingest(View v, int j, int c, int init, int stg_off) {
+__global__ void k_ingest(View v, int j, int c, int init, int stg_off, SlideIO io) {
     pdl_wait();
-    ingest_body(v, j, c, init, stg_off, v.staging, blockIdx.x);
+    ingest_body(v, j, c, init, stg_off, io, blockIdx.x);
 }
 
 // Exclusive scan of one value per thread over a 1024-thread block.
@@ -1467,11 +1477,13 @@ __device__ __forceinline__ unsigned long long* rad_buffer(const View& v, int pas
 // Slots [base, base + count) take the new points (base by the slide's place
 // in the ring, 0 while loading); every slot's sort word goes to the first
 // pass's input (chunk < 0), or the new points' chunk words to nsort.
-__global__ void k_ingest_all(View v, const float* input, int count, int init, int ob, int passes) {
+__global__ void k_ingest_all(View v, SlideIO io, int count, int init, int ob, int passes) {
     pdl_wait();
     const long long b = v.ctl->b_done + 1;  // this build (k_build keeps b_done)
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         v.ctl->b = b;
+        v.ctl->out_label = io.label;
+        v.ctl->out_cid = io.cid;
         if (!init) {
             v.ctl->prev_ok = 0;     // no forest reuse in this clustering,
             v.ctl->reuse_skip = 2;  // no roots kept for the next,
@@ -1483,7 +1495,7 @@ __global__ void k_ingest_all(View v, const float* input, int count, int init, in
     const int base = chunk_base_slot(v, 0, init);
     unsigned long long key;
     if (s >= base && s < base + count) {
-        const float* p = input + (size_t)(s - base) * v.dim;
+        const float* p = io.input + (size_t)(s - base) * v.dim;
         const float x = p[0];
         const float y = v.dim > 1 ? p[1] : 0.0f;
         const float z = v.dim > 2 ? p[2] : 0.0f;
@@ -1854,13 +1866,17 @@ __global__ void __launch_bounds__(kCountThreads, 8) k_count(View v, int P) {
 // Fresh start hints without reuse (-1 for a non-core position, its own
 // slot for a core) and a fresh forest, for a clustering of the window as it
 // stands (rtdbs_cluster), whose hints may hold the last union's roots.
-__global__ void k_hints(View v) {
+__global__ void k_hints(View v, SlideIO io) {
     pdl_wait();
     const int cur = (int)(v.ctl->b & 1);
     const int n = v.ctl->nocc[cur];
     const int* scnt = v.scnt[cur];
     const int* sw = reinterpret_cast<const int*>(v.spt[cur]) + 3;
-    if (blockIdx.x == 0 && threadIdx.x == 0) v.ctl->prev_ok = 0;  // no reuse to judge (read by k_border)
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        v.ctl->prev_ok = 0;  // no reuse to judge (read by k_border)
+        v.ctl->out_label = io.label;
+        v.ctl->out_cid = io.cid;
+    }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int s = sw[4 * (size_t)i];
         v.sroot[i] = scnt[i] >= v.min_pts ? s : -1;
@@ -2311,6 +2327,13 @@ struct LabelSmem {
     unsigned char tseg[kWarps][C::kTasks];
 };
 
+__device__ __forceinline__ void put_result(const View& v, int* ol, int* oc, int slot, int lab, int id) {
+    v.label[slot] = lab;
+    v.cid[slot] = id;
+    if (ol) ol[slot] = lab;
+    if (oc) oc[slot] = id;
+}
+
 template <int MODE, int DK, class Smem>
 __device__ __forceinline__ void label_body(const View& v, int advance, int bx, int nbx, Smem& sm, int P) {
     constexpr int DIM = DK & 3, K = (DK >> 2) + 1;  // dimension, cells per Eps
@@ -2329,6 +2352,8 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, i
     const int nblk = (n + P - 1) / P, step = nbx * (kClusterThreads / 32);
     const float4* spt = v.spt[cur];
     const int* sroot = v.sroot;
+    int* ol = v.ctl->out_label;
+    int* oc = v.ctl->out_cid;
     Tally tally;
     for (int bk = bx * (kClusterThreads / 32) + wib; bk < nblk; bk += step) {
         const int i = bk * P + lane;
@@ -2344,8 +2369,7 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, i
             // (a point with no neighbour but itself is noise without a scan)
             home = hr < 0 && v.scnt[cur][i] > 1;
             if (!home) {
-                v.label[hslot] = hr >= 0 ? 0 : 2;
-                v.cid[hslot] = hr >= 0 ? hr : hslot;
+                put_result(v, ol, oc, hslot, hr >= 0 ? 0 : 2, hr >= 0 ? hr : hslot);
             } else {
                 key = v.skey[cur][i];
             }
@@ -2418,8 +2442,7 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, i
         __syncwarp();
         if (home) {
             const int to = best[lane];
-            v.label[hslot] = to != INT_MAX ? 1 : 2;
-            v.cid[hslot] = to != INT_MAX ? to : hslot;
+            put_result(v, ol, oc, hslot, to != INT_MAX ? 1 : 2, to != INT_MAX ? to : hslot);
         }
         __syncwarp();
     }
@@ -2451,6 +2474,8 @@ __global__ void __launch_bounds__(kClusterThreads, 4) k_label(View v, int advanc
 // forest for the next clustering (coalesced, by slot) and ends the slide
 // like k_label.
 __device__ __forceinline__ void border_body(const View& v, int advance, int bx, int nbx) {
+    int* ol = v.ctl->out_label;
+    int* oc = v.ctl->out_cid;
     for (int s = bx * blockDim.x + threadIdx.x; s < v.W; s += nbx * blockDim.x) {
         const int root = v.rslot[s];
         int lab = 0, id = root;
@@ -2474,6 +2499,8 @@ __device__ __forceinline__ void border_body(const View& v, int advance, int bx, 
         }
         v.label[s] = lab;
         v.cid[s] = id;
+        if (ol) ol[s] = lab;
+        if (oc) oc[s] = id;
         v.parent[s] = s;
         v.damaged[s] = 0;
     }
@@ -2552,7 +2579,7 @@ __global__ void __launch_bounds__(PhaseShape<PHASE>::threads, PhaseShape<PHASE>:
     __syncthreads();
     const int bx = s_bx, nbx = s_nbx;
     if constexpr (PHASE == kBatchIngest) {
-        ingest_body(sv, it.j, it.c, 0, it.stg_off, it.input, bx);
+        ingest_body(sv, it.j, it.c, 0, it.stg_off, SlideIO{it.input, nullptr, nullptr}, bx);
     } else if constexpr (PHASE == kBatchSort) {
         __shared__ SortSmem sm;
         const int nruns = (it.c + kSortRun - 1) / kSortRun;
@@ -2669,11 +2696,11 @@ constexpr int kPdlWindow = 131072;
 bool pdl_on(const View& v) { return v.W <= kPdlWindow; }
 
 cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, int init,
-                         int stg_off, int advance, cudaStream_t s, bool pdl) {
+                         int stg_off, int advance, cudaStream_t s, bool pdl, const SlideIO& io) {
     const int warp_blocks = (c * v.qlanes + 255) / 256;  // count passes
     switch (phase) {
         case kPhaseIngest:
-            launch(k_ingest, (c + 255) / 256, 256, 0, s, pdl, v, j, c, init, stg_off);
+            launch(k_ingest, (c + 255) / 256, 256, 0, s, pdl, v, j, c, init, stg_off, io);
             break;
         case kPhaseSort: {
             const int single = c <= kSortRun;  // one run: sorted straight into place, no run merge
@@ -2732,8 +2759,9 @@ cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int init, int stg_off,
-                              cudaStream_t s, cudaStream_t side, cudaEvent_t fork, cudaEvent_t join) {
+cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int init, int stg_off, cudaStream_t s,
+                              const SlideIO& io, bool ingested, cudaStream_t side, cudaEvent_t fork,
+                              cudaEvent_t join) {
     if (c <= 0 || c > kChunkMax) return cudaErrorInvalidValue;
     const bool beside = side && fork && join && !init;  // the decrement beside the sort
     for (int ph = 0; ph < kChunkPhases; ++ph) {
@@ -2741,9 +2769,13 @@ cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int in
         if (beside && ph == kPhaseDecrement) continue;  // launched on the side stream
         if (beside && ph == kPhaseMerge && (e = cudaStreamWaitEvent(s, join, 0)) != cudaSuccess) return e;
         // (the ingest follows a copy or another chunk's work, the merge two streams)
-        const bool pdl = pdl_on(v) && ph != kPhaseIngest && ph != kPhaseDecrement && ph != kPhaseMerge;
-        e = launch_phase(ph, v, precision, j, c, init, stg_off, 0, s, pdl);
-        if (e != cudaSuccess) return e;
+        // (a launch behind an ingest outside the graph is the graph's first node)
+        const bool pdl = pdl_on(v) && ph != kPhaseIngest && ph != kPhaseDecrement && ph != kPhaseMerge &&
+                         !(ingested && ph == kPhaseSort);
+        if (!(ingested && ph == kPhaseIngest)) {
+            e = launch_phase(ph, v, precision, j, c, init, stg_off, 0, s, pdl, io);
+            if (e != cudaSuccess) return e;
+        }
         // (after the ingest, but launched behind the sort, whose few large blocks
         // should not wait for the decrement's to leave: 500k points 174 -> 166 us
         // per slide, 1M 325 -> 318)
@@ -2758,7 +2790,7 @@ cudaError_t launch_chunk_step(const View& v, int precision, int j, int c, int in
     return cudaSuccess;
 }
 
-cudaError_t launch_window_phase(int phase, const View& v, int precision, const float* input, int count, int init,
+cudaError_t launch_window_phase(int phase, const View& v, int precision, const SlideIO& io, int count, int init,
                                 cudaStream_t s, bool pdl) {
     const int grid = (v.W + 255) / 256;
     const bool chunk = v.W <= kChunkMax;  // one chunk: its runs are sorted and ranked on chip
@@ -2766,7 +2798,7 @@ cudaError_t launch_window_phase(int phase, const View& v, int precision, const f
     const int passes = chunk ? -1 : (v.key_bits + 7) / 8;
     switch (phase) {
         case kPhaseIngest:
-            launch(k_ingest_all, grid, 256, 0, s, pdl, v, input, count, init, ob, passes);
+            launch(k_ingest_all, grid, 256, 0, s, pdl, v, io, count, init, ob, passes);
             break;
         case kPhaseSort:
             if (chunk) {
@@ -2807,14 +2839,15 @@ cudaError_t launch_window_phase(int phase, const View& v, int precision, const f
     return cudaGetLastError();
 }
 
-cudaError_t launch_window_build(const View& v, int precision, const float* input, int count, int init,
-                                cudaStream_t s) {
+cudaError_t launch_window_build(const View& v, int precision, const SlideIO& io, int count, int init,
+                                cudaStream_t s, bool ingested) {
     if (!window_build_fits(v)) return cudaErrorInvalidValue;
     cudaError_t e = cudaSuccess;
-    for (int ph = 0; ph < kChunkPhases && e == cudaSuccess; ++ph)
+    for (int ph = ingested ? kPhaseSort : kPhaseIngest; ph < kChunkPhases && e == cudaSuccess; ++ph)
         // (kernels that follow each other closely at any size: a first window of
         // 1M points 864 -> 820 us, of 20k 205 -> 179)
-        e = launch_window_phase(ph, v, precision, input, count, init, s, ph != kPhaseIngest);
+        e = launch_window_phase(ph, v, precision, io, count, init, s,
+                                ph != kPhaseIngest && !(ingested && ph == kPhaseSort));
     return e;
 }
 
@@ -2859,11 +2892,11 @@ cudaError_t launch_bbox(const float* pts, long long n, int dim, unsigned* box, c
 }
 
 cudaError_t launch_cluster(const View& v, int precision, int advance, cudaStream_t s, bool fresh_hints,
-                           cudaEvent_t outputs_free, unsigned wait_flags) {
+                           cudaEvent_t outputs_free, unsigned wait_flags, const SlideIO& io) {
     cudaError_t e = cudaSuccess;
     if (fresh_hints) {
         const int sms = g_num_sms > 0 ? g_num_sms : 152;
-        k_hints<<<max(1, min(sms * 8, (v.W + 255) / 256)), 256, 0, s>>>(v);
+        k_hints<<<max(1, min(sms * 8, (v.W + 255) / 256)), 256, 0, s>>>(v, io);
         e = cudaGetLastError();
     }
     for (int ph = kPhaseUnion; ph <= kPhaseLabel && e == cudaSuccess; ++ph) {

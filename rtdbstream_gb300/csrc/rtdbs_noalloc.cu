@@ -244,7 +244,7 @@ extern "C" RTDBS_API int rtdbs_cluster_window_noalloc(const float* d_points, int
                      d_cluster_id);
     if (rc != RTDBS_OK) return rc;  // nothing is queued after the wait above
 
-    NOALLOC_TRY(rtdbs::launch_window_build(v, precision, d_points, n, 1, s));
+    NOALLOC_TRY(rtdbs::launch_window_build(v, precision, rtdbs::SlideIO{d_points, nullptr, nullptr}, n, 1, s));
     NOALLOC_TRY(rtdbs::launch_cluster(v, precision, 0, s));
     int err = 0;
     NOALLOC_TRY(cudaMemcpyAsync(&err, &v.ctl->err, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -286,7 +286,7 @@ extern "C" RTDBS_API int rtdbs_cluster_window_noalloc_async(const float* d_point
         return RTDBS_OK;
     }
     NOALLOC_TRY(reset_scratch(base, s));
-    NOALLOC_TRY(rtdbs::launch_window_build(v, precision, d_points, n, 1, s));
+    NOALLOC_TRY(rtdbs::launch_window_build(v, precision, rtdbs::SlideIO{d_points, nullptr, nullptr}, n, 1, s));
     NOALLOC_TRY(rtdbs::launch_cluster(v, precision, 0, s));
     NOALLOC_TRY(cudaMemcpyAsync(d_status, &v.ctl->err, sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
 #undef NOALLOC_TRY

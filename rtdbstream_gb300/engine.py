@@ -179,8 +179,6 @@ class Engine:
         h = ctypes.c_void_p()
         _check(self._lib.rtdbs_create(ctypes.byref(p), ctypes.c_void_p(stream), ctypes.byref(h)))
         self._h = h
-        self._label = np.empty(self.window_size, np.int32)
-        self._cid = np.empty(self.window_size, np.int32)
 
     # -- lifecycle
     def close(self) -> None:
@@ -216,14 +214,12 @@ class Engine:
 
     def slide(self, new_points, label: Optional[np.ndarray] = None,
               cluster_id: Optional[np.ndarray] = None):
-        """One slide; returns (label, cluster_id) host arrays (copies)."""
+        """One slide; returns (label, cluster_id) host arrays (new ones unless given)."""
         a = self._host_points(new_points, self.stride_size)
-        lab = self._label if label is None else label
-        cid = self._cid if cluster_id is None else cluster_id
+        lab = np.empty(self.window_size, np.int32) if label is None else label
+        cid = np.empty(self.window_size, np.int32) if cluster_id is None else cluster_id
         _check(self._lib.rtdbs_slide(self._h, a.ctypes.data, lab.ctypes.data, cid.ctypes.data))
-        if label is None:
-            return lab.copy(), cid.copy()
-        return lab, cid
+        return lab, (cid.copy() if label is None and cluster_id is not None else cid)
 
     def slide_pipelined(self, new_points: np.ndarray, label: np.ndarray, cluster_id: np.ndarray) -> None:
         """One slide with host buffers, one slide in flight: returns once the
