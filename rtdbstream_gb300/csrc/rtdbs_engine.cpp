@@ -137,6 +137,21 @@ int set_geometry(View& v, int dim, double eps, int cells_per_eps, const float* b
     v.shift[0] = bits[1] + bits[2];
     const int kbits = bits[0] + bits[1] + bits[2];
     v.inv_cell = 1.0 / L;
+    // The single-precision quotient q32 = fl(fl(x - o32) * i32) of a coordinate
+    // x whose double quotient is q = (x - o) / L, with u = 2^-24: x - o32 is off
+    // by |o - o32| <= u |o| and one rounding of at most u |x - o32|; i32 and the
+    // product add a relative 2u.  For 0 <= q32 < ext + 1 (others are clamped or
+    // redone), |x - o32| <= (ext + 2) L, so |q32 - q| <= u (|o| / L + 4 (ext + 2)) in
+    // cells; doubled, which also covers the double evaluation's own rounding.
+    // Above half a cell, or where the single-precision values leave the normal
+    // range, the filter is off.
+    v.inv_cell32 = (float)v.inv_cell;
+    for (int a = 0; a < 3; ++a) {
+        v.origin32[a] = (float)v.origin[a];
+        const double err = 2.0 * std::ldexp(1.0, -24) * (std::fabs(v.origin[a]) / L + 4.0 * ((double)v.ext[a] + 2.0));
+        const bool normal = L > std::ldexp(1.0, -100) && L < std::ldexp(1.0, 100);
+        v.key_err[a] = normal && err < 0.4 ? std::nextafter((float)err, 1.0f) : 2.0f;
+    }
     v.key_bits = kbits;
     v.sort_passes = (kbits + 7) / 8;
     if (cell_side) *cell_side = L;
@@ -274,6 +289,7 @@ size_t plan_layout(rtdbs_engine* e, std::vector<Part>& parts) {
         {(void**)&v.sprev[1], sizeof(int) * track_ints},
         {(void**)&v.nsort, sizeof(unsigned long long) * C},
         {(void**)&v.xsort, sizeof(unsigned long long) * C},
+        {(void**)&v.xkey, sizeof(unsigned long long) * C},
         {(void**)&v.nword, sizeof(unsigned long long) * C},
         {(void**)&v.xword, sizeof(unsigned long long) * C},
         {(void**)&v.xpt, sizeof(float4) * C},

@@ -101,6 +101,8 @@ struct View {
     // key = i << shift[0] | j << shift[1] | k (bit fields, shift[2] = 0)
     double origin[3];
     double inv_cell;
+    float origin32[3], inv_cell32;  // the same in single precision, with the
+    float key_err[3];               // largest error of its quotient, in cells (> 1/2: not used)
     long long ext[3];
     int shift[3];
     int dim;
@@ -148,6 +150,7 @@ struct View {
                                  // reuse; null without neighbour lists
     unsigned long long* nsort;   // chunk sort words in (key << 14 | offset)
     unsigned long long* xsort;
+    unsigned long long* xkey;    // cell keys of the chunk's expired points by offset
     unsigned long long* nword;   // sorted
     unsigned long long* xword;
     float4* xpt;                 // expired points of the chunk by offset

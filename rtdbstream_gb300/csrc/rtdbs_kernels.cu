@@ -68,21 +68,33 @@ __device__ __forceinline__ unsigned lanemask_lt(int lane) { return (1u << lane) 
 
 // ------------------------------------------------------------------ geometry
 
-__device__ __forceinline__ unsigned long long cell_key(const View& v, float x, float y, float z) {
-    const float q[3] = {x, y, z};
-    unsigned long long key = 0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        long long c = 0;
-        if (a < v.dim) {
-            double t = floor(((double)q[a] - v.origin[a]) * v.inv_cell);
-            if (!(t >= 0.0)) t = 0.0;  // also maps NaN to cell 0
-            const double top = (double)(v.ext[a] - 1);
-            if (t > top) t = top;
-            c = (long long)t;
-        }
-        key |= (unsigned long long)c << v.shift[a];
+// Cell coordinate along axis a: clamp(floor((x - origin) * inv_cell), 0, ext - 1)
+// in double, NaN in cell 0.  The single-precision quotient differs from the
+// double one by at most key_err cells (see set_geometry), so its floor is the
+// double's wherever no cell edge lies within that; the others, and quotients
+// outside [0, 2^22), are redone in double.  (FP64 runs at 1/64 of the FP32
+// rate here: a first window of 1M points took 50 us longer all in double, and
+// the decrement, which recomputed its queries' keys, 7 us per slide.)
+__device__ __forceinline__ long long cell_coord(const View& v, int a, float x) {
+    const float t32 = __fmul_rn(__fsub_rn(x, v.origin32[a]), v.inv_cell32);
+    const float f = floorf(t32), in = __fsub_rn(t32, f);
+    long long c;
+    if (t32 >= 0.0f && t32 < 4194304.0f && in >= v.key_err[a] && in <= 1.0f - v.key_err[a]) {
+        c = (long long)(int)f;
+        const long long top = v.ext[a] - 1;
+        return c > top ? top : c;
     }
+    double t = floor(((double)x - v.origin[a]) * v.inv_cell);
+    if (!(t >= 0.0)) t = 0.0;  // also maps NaN to cell 0
+    const double top = (double)(v.ext[a] - 1);
+    if (t > top) t = top;
+    return (long long)t;
+}
+
+__device__ __forceinline__ unsigned long long cell_key(const View& v, float x, float y, float z) {
+    unsigned long long key = (unsigned long long)cell_coord(v, 0, x) << v.shift[0];
+    if (v.dim > 1) key |= (unsigned long long)cell_coord(v, 1, y) << v.shift[1];
+    if (v.dim > 2) key |= (unsigned long long)cell_coord(v, 2, z);
     return key;
 }
 
@@ -728,7 +740,9 @@ __device__ __forceinline__ void ingest_body(const View& v, int j, int c, int ini
     const int slot = chunk_base_slot(v, j, init) + k;
     if (!init) {
         v.xpt[k] = v.ring[slot];
-        v.xsort[k] = (v.kslot[slot] << kOffBits) | (unsigned long long)k;
+        const unsigned long long old = v.kslot[slot];
+        v.xkey[k] = old;
+        v.xsort[k] = (old << kOffBits) | (unsigned long long)k;
         if (damage_on(v)) mark_damage(v, slot);  // an expired core
     }
     const float* p = input + (size_t)(stg_off + k) * v.dim;
@@ -946,10 +960,10 @@ __device__ __forceinline__ void decr_g(const View& v, int j, int c, int bx, Stre
     const int old = (int)((b - 1) & 1);
     const unsigned gen = gen_of_build(b - 1);
     const int el = chunk_base_slot(v, j, 0);
-    // Expired points keyed from their saved coordinates (the same key they
-    // were sorted by when they arrived): the pass does not wait for the
-    // chunk's sort, and runs beside it.  Taken in their kept (key, slot)
-    // order where there is one, so neighbouring warps read the same cells.
+    // Expired points with their kept keys (the sort words are being sorted):
+    // the pass does not wait for the chunk's sort, and runs beside it.  Taken
+    // in their kept (key, slot) order where there is one, so neighbouring warps
+    // read the same cells.
     int k = qi;
     if (has && expired_presorted(v, 0)) {
         k = v.sorder[el + qi];
@@ -959,7 +973,7 @@ __device__ __forceinline__ void decr_g(const View& v, int j, int c, int bx, Stre
         }
     }
     const float4 xp = has ? v.xpt[k] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const unsigned long long key = has ? cell_key(v, xp.x, xp.y, xp.z) : 0ull;
+    const unsigned long long key = has ? v.xkey[k] : 0ull;
     int rs, re;
     row_ranges<DIM, false, K, G>(v, v.table[old], gen, key, gl, rs, re);
     int total = candidate_stream<Stencil<DIM, false, K>::kRows, G>(rs, re, 0, gl, rstart, rpre);
@@ -1451,7 +1465,7 @@ __global__ void __launch_bounds__(256, 5) k_incr(View v, int j, int c, int init)
 // word, a radix sort orders them, one pass lays the window out in that order,
 // the cell table is built once and every point's neighbours are counted once
 // (k_count), instead of W / 16384 chunk steps that each rewrite the window.
-// A 1M-point walker window: load 9.9 -> 0.5 ms (sort 97 us, count 276 us; the
+// A 1M-point walker window: load 9.9 -> 0.45 ms (sort 60 us, count 275 us; the
 // box of the points is taken on the device, not in a host loop over a copy);
 // 48k points replaced per slide: 327 -> 137 us for the grid.
 // Words are key << ob | slot (ob bits for the slots; the host takes the chunk
@@ -1463,10 +1477,18 @@ constexpr int kRadThreads = 512;
 constexpr int kRadItems = 8;                           // words per thread
 constexpr int kRadTile = kRadThreads * kRadItems;      // words per block
 constexpr int kRadWarps = kRadThreads / 32;
-// Up to this many tiles every scatter block sums the tiles' counters itself
-// (12 tiles: sort 52 -> 44 us without the scan's launches); above, a scan
-// kernel does it once.
-constexpr int kRadInline = 64;
+// Digits of up to 10 bits, as equal as the key's bits allow: a key of 18 or 20
+// bits takes two passes, one of 25 three, where 8-bit digits took three and
+// four (48k points 44 -> 27 us, 1M 97 -> 60).
+constexpr int kRadBits = 10;
+inline int rad_passes(const View& v) { return (v.key_bits + kRadBits - 1) / kRadBits; }
+inline int rad_bits(const View& v) {  // (at least 5: the scan takes 32 digits a block)
+    const int p = rad_passes(v);
+    return p ? max(5, (v.key_bits + p - 1) / p) : 5;
+}
+// Up to this many tiles every scatter block sums the tiles' counters itself;
+// above, a scan kernel does it once.
+constexpr int kRadInline = 32;
 
 // Input buffer of radix pass `pass` of `passes` (pass == passes: the sorted words).
 __device__ __forceinline__ unsigned long long* rad_buffer(const View& v, int pass, int passes) {
@@ -1514,12 +1536,13 @@ __global__ void k_ingest_all(View v, SlideIO io, int count, int init, int ob, in
     }
 }
 
-__global__ void __launch_bounds__(kRadThreads) k_rad_hist(View v, int pass, int passes, int shift) {
+__global__ void __launch_bounds__(kRadThreads) k_rad_hist(View v, int pass, int passes, int shift, int bits) {
     pdl_wait();
-    __shared__ int hist[256];
+    __shared__ int hist[1 << kRadBits];
+    const int bins = 1 << bits;
     const unsigned long long* in = rad_buffer(v, pass, passes);
     int* counts = v.scnt[(v.ctl->b & 1) ^ 1];
-    if (threadIdx.x < 256) hist[threadIdx.x] = 0;
+    for (int d = threadIdx.x; d < bins; d += kRadThreads) hist[d] = 0;
     __syncthreads();
     unsigned long long w[kRadItems];
 #pragma unroll
@@ -1530,16 +1553,16 @@ __global__ void __launch_bounds__(kRadThreads) k_rad_hist(View v, int pass, int 
 #pragma unroll
     for (int k = 0; k < kRadItems; ++k) {
         const int i = blockIdx.x * kRadTile + k * kRadThreads + threadIdx.x;
-        if (i < v.W) atomicAdd(&hist[(unsigned)(w[k] >> shift) & 255u], 1);
+        if (i < v.W) atomicAdd(&hist[(unsigned)(w[k] >> shift) & (bins - 1)], 1);
     }
     __syncthreads();
-    if (threadIdx.x < 256) counts[blockIdx.x * 256 + threadIdx.x] = hist[threadIdx.x];
+    for (int d = threadIdx.x; d < bins; d += kRadThreads) counts[blockIdx.x * bins + d] = hist[d];
 }
 
 // Exclusive scan over the tiles of 32 digits per block (a warp's lanes side by
 // side), 8 warps on an eighth of the tiles each; the digits' totals follow
 // the tiles' counters.  Only where there are many tiles (kRadInline).
-__global__ void __launch_bounds__(256) k_rad_scan(View v, int ntiles) {
+__global__ void __launch_bounds__(256) k_rad_scan(View v, int ntiles, int bins) {
     pdl_wait();
     __shared__ int part[8][32];
     int* counts = v.scnt[(v.ctl->b & 1) ^ 1];
@@ -1547,33 +1570,38 @@ __global__ void __launch_bounds__(256) k_rad_scan(View v, int ntiles) {
     const int per = (ntiles + 7) / 8, t0 = min(w * per, ntiles), t1 = min(t0 + per, ntiles);
     int sum = 0;
 #pragma unroll 8
-    for (int t = t0; t < t1; ++t) sum += counts[t * 256 + d];
+    for (int t = t0; t < t1; ++t) sum += counts[t * bins + d];
     part[w][lane] = sum;
     __syncthreads();
     int at = 0;
     for (int k = 0; k < w; ++k) at += part[k][lane];
 #pragma unroll 8
     for (int t = t0; t < t1; ++t) {
-        const int x = counts[t * 256 + d];
-        counts[t * 256 + d] = at;
+        const int x = counts[t * bins + d];
+        counts[t * bins + d] = at;
         at += x;
     }
-    if (w == 7) counts[(size_t)256 * ntiles + d] = at;
+    if (w == 7) counts[ntiles * bins + d] = at;
 }
 
 // Stable scatter of one tile by its digit: each warp ranks its 256
-// consecutive words in order (lanes with equal digits from eight ballots),
-// warp counters are scanned per digit, and every word goes to its place.
-__global__ void __launch_bounds__(kRadThreads) k_rad_scatter(View v, int pass, int passes, int shift, int scanned) {
+// consecutive words in order (lanes with equal digits from a ballot per
+// digit bit), warp counters are scanned per digit, and every word goes to its
+// place.
+__global__ void __launch_bounds__(kRadThreads) k_rad_scatter(View v, int pass, int passes, int shift, int bits,
+                                                             int scanned) {
     pdl_wait();
-    __shared__ int cnt[kRadWarps][256];
-    __shared__ int wsum[8];
+    __shared__ unsigned short cnt[kRadWarps][1 << kRadBits];  // of a warp, then before it in the tile
+    __shared__ int base[1 << kRadBits];                      // the tile's first place of a digit
+    __shared__ int wsum[kRadWarps];
+    const int bins = 1 << bits;
     const unsigned long long* in = rad_buffer(v, pass, passes);
     unsigned long long* out = rad_buffer(v, pass + 1, passes);
     const int* counts = v.scnt[(v.ctl->b & 1) ^ 1];
     const int ntiles = gridDim.x, tile = blockIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int k = threadIdx.x; k < kRadWarps * 256; k += kRadThreads) (&cnt[0][0])[k] = 0;
+    for (int k = threadIdx.x; k < kRadWarps * (1 << kRadBits) / 2; k += kRadThreads)
+        reinterpret_cast<unsigned*>(&cnt[0][0])[k] = 0;
     unsigned long long it[kRadItems];
     int rank[kRadItems];
     const int i0 = tile * kRadTile + w * (32 * kRadItems) + lane;
@@ -1583,57 +1611,66 @@ __global__ void __launch_bounds__(kRadThreads) k_rad_scatter(View v, int pass, i
 #pragma unroll
     for (int k = 0; k < kRadItems; ++k) {
         const bool has = i0 + 32 * k < v.W;
-        const unsigned d = (unsigned)(it[k] >> shift) & 255u;
+        const unsigned d = (unsigned)(it[k] >> shift) & (bins - 1);
         unsigned peers = __ballot_sync(kFull, has);
-#pragma unroll
-        for (int bit = 0; bit < 8; ++bit) {
+        for (int bit = 0; bit < bits; ++bit) {
             const unsigned bm = __ballot_sync(kFull, (d >> bit) & 1u);
             peers &= ((d >> bit) & 1u) ? bm : ~bm;
         }
         const int before = cnt[w][d];
         __syncwarp();
         rank[k] = before + __popc(peers & lanemask_lt(lane));
-        if (has && !(peers & lanemask_lt(lane))) cnt[w][d] = before + __popc(peers);
+        if (has && !(peers & lanemask_lt(lane))) cnt[w][d] = (unsigned short)(before + __popc(peers));
         __syncwarp();
     }
-    __syncthreads();
-    // digit totals -> digit bases, then every warp's first place per digit
-    int total = 0, incl = 0, mine = 0;  // the digit's words: all, running, before this tile
-    if (threadIdx.x < 256) {
+    // digit totals -> digit bases: each thread two neighbouring digits
+    int total[2] = {0, 0}, mine[2] = {0, 0};  // words of the digit: all, before this tile
+    const int d0 = 2 * threadIdx.x;
+    if (d0 < bins) {
         if (scanned) {
-            total = counts[(size_t)256 * ntiles + threadIdx.x];
-            mine = counts[tile * 256 + threadIdx.x];
+            for (int u = 0; u < 2; ++u) {
+                total[u] = counts[ntiles * bins + d0 + u];
+                mine[u] = counts[tile * bins + d0 + u];
+            }
         } else {
 #pragma unroll 8
             for (int t = 0; t < ntiles; ++t) {
-                const int x = counts[t * 256 + threadIdx.x];
-                total += x;
-                mine += t < tile ? x : 0;
+                const int2 x = *reinterpret_cast<const int2*>(&counts[t * bins + d0]);
+                total[0] += x.x;
+                total[1] += x.y;
+                mine[0] += t < tile ? x.x : 0;
+                mine[1] += t < tile ? x.y : 0;
             }
         }
-        incl = total;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += y;
-        }
-        if (lane == 31) wsum[w] = incl;
     }
-    __syncthreads();
-    if (threadIdx.x < 256) {
-        int at = incl - total + mine;
+    int incl = total[0] + total[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[w] = incl;
+    __syncthreads();  // (every warp's counts are in, too)
+    if (d0 < bins) {
+        int at = incl - total[0] - total[1];
         for (int k = 0; k < w; ++k) at += wsum[k];
-        for (int k = 0; k < kRadWarps; ++k) {
-            const int x = cnt[k][threadIdx.x];
-            cnt[k][threadIdx.x] = at;
-            at += x;
+        base[d0] = at + mine[0];
+        base[d0 + 1] = at + total[0] + mine[1];
+        for (int u = 0; u < 2; ++u) {
+            int before = 0;
+            for (int k = 0; k < kRadWarps; ++k) {
+                const int x = cnt[k][d0 + u];
+                cnt[k][d0 + u] = (unsigned short)before;
+                before += x;
+            }
         }
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < kRadItems; ++k) {
         if (i0 + 32 * k >= v.W) continue;
-        const int o = cnt[w][(unsigned)(it[k] >> shift) & 255u] + rank[k];
+        const unsigned d = (unsigned)(it[k] >> shift) & (bins - 1);
+        const int o = base[d] + cnt[w][d] + rank[k];
         if (o >= 0 && o < v.W)
             out[o] = it[k];
         else
@@ -2795,7 +2832,7 @@ cudaError_t launch_window_phase(int phase, const View& v, int precision, const S
     const int grid = (v.W + 255) / 256;
     const bool chunk = v.W <= kChunkMax;  // one chunk: its runs are sorted and ranked on chip
     const int ob = chunk ? kOffBits : slot_bits(v.W);
-    const int passes = chunk ? -1 : (v.key_bits + 7) / 8;
+    const int passes = chunk ? -1 : rad_passes(v), bits = rad_bits(v);
     switch (phase) {
         case kPhaseIngest:
             launch(k_ingest_all, grid, 256, 0, s, pdl, v, io, count, init, ob, passes);
@@ -2810,11 +2847,12 @@ cudaError_t launch_window_phase(int phase, const View& v, int precision, const S
                 break;
             }
             for (int p = 0; p < passes; ++p) {
-                const int tiles = (v.W + kRadTile - 1) / kRadTile;
-                launch(k_rad_hist, tiles, kRadThreads, 0, s, pdl, v, p, passes, ob + 8 * p);
+                const int tiles = (v.W + kRadTile - 1) / kRadTile, shift = ob + bits * p;
+                launch(k_rad_hist, tiles, kRadThreads, 0, s, pdl, v, p, passes, shift, bits);
                 const int scanned = tiles > kRadInline;
-                if (scanned) launch(k_rad_scan, 8, 256, 0, s, pdl, v, tiles);
-                launch(k_rad_scatter, tiles, kRadThreads, 0, s, pdl, v, p, passes, ob + 8 * p, scanned);
+                if (scanned) launch(k_rad_scan, (1 << bits) / 32, 256, 0, s, true, v, tiles, 1 << bits);
+                launch(k_rad_scatter, tiles, kRadThreads, 0, s, true, v, p, passes, shift, bits, scanned);
+                pdl = true;
             }
             break;
         case kPhaseDecrement: break;  // counted afresh
@@ -2853,7 +2891,7 @@ cudaError_t launch_window_build(const View& v, int precision, const SlideIO& io,
 
 int window_build_launches(const View& v) {
     const int per = (v.W + kRadTile - 1) / kRadTile > kRadInline ? 3 : 2;
-    const int sorts = v.W > kChunkMax ? per * ((v.key_bits + 7) / 8) : (v.W > kSortRun ? 2 : 1);
+    const int sorts = v.W > kChunkMax ? per * rad_passes(v) : (v.W > kSortRun ? 2 : 1);
     return 4 + sorts;
 }
 
