@@ -153,7 +153,8 @@ int set_geometry(View& v, int dim, double eps, int cells_per_eps, const float* b
         v.key_err[a] = normal && err < 0.4 ? std::nextafter((float)err, 1.0f) : 2.0f;
     }
     v.key_bits = kbits;
-    v.sort_passes = (kbits + 7) / 8;
+    v.sort_passes = (kbits + kSortBits - 1) / kSortBits;
+    v.sort_bits = v.sort_passes ? (kbits + v.sort_passes - 1) / v.sort_passes : 1;
     if (cell_side) *cell_side = L;
     return RTDBS_OK;
 }

@@ -41,6 +41,7 @@ constexpr unsigned kGenMod = 16383;  // table generations 1..16383 (tag = gen <<
 constexpr int kMergeTile = 1024;   // old entries per merge block
 constexpr int kMergeThreads = 256;
 constexpr int kSortRun = 1024;     // words per radix-sort CTA (one per thread)
+constexpr int kSortBits = 9;       // most digit bits of a chunk sort pass
 constexpr int kBuildThreads = 512;
 constexpr int kClusterThreads = 256;
 constexpr int kLinkThreads = 256;
@@ -120,7 +121,7 @@ struct View {
     double E;                   // FP64 mode: eps * eps
     int filter_ok;              // FP64 mode: band valid (else every test in FP64)
     int key_bits;
-    int sort_passes;
+    int sort_passes, sort_bits;  // radix passes over a chunk's keys, bits per pass
     int block_pts;              // sorted positions a union warp takes as one block (16 or 32;
                                 // pool launches take 32)
     int precision;              // RTDBS_PREC_* (batched launches dispatch on it)
