@@ -709,7 +709,7 @@ __device__ __forceinline__ bool slot_is_new(const View& v, int s) {
 __device__ __forceinline__ int start_hint(const View& v, int s, int cnt, int prev, bool reuse,
                                           unsigned& reused) {
     if (cnt < v.min_pts) return -1;
-    if (reuse && prev >= 0 && !v.damaged[prev]) {
+    if (reuse && prev >= 0 && !__ldg(&v.damaged[prev])) {
         ++reused;
         return prev;
     }
@@ -1229,8 +1229,12 @@ __device__ __forceinline__ void merge_body(const View& v, int j, int c, int init
     }
     __syncthreads();
 
-    // survivors (coalesced, item order i = tid + 256 k)
-    for (int i = tid; i < tlen; i += kMergeThreads) {
+    // survivors (coalesced, item order i = tid + 256 k; unrolled, with loads
+    // that may pass the stores: 1M points 24.6 -> 22.5 us)
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int i = tid + u * kMergeThreads;
+        if (i >= tlen) continue;
         const int s = tslot[i];
         if (!(init || s < el || s >= el + c)) continue;
         const int lessnew = m > 0 ? count_words_less(nw, m, el, tkey[i], s) : 0;
@@ -1240,10 +1244,10 @@ __device__ __forceinline__ void merge_body(const View& v, int j, int c, int init
             continue;
         }
         dkey[o] = tkey[i];
-        dpt[o] = opt[ts + i];
-        const int cnt = ocnt[ts + i];
+        dpt[o] = __ldg(&opt[ts + i]);
+        const int cnt = __ldg(&ocnt[ts + i]);
         dcnt[o] = cnt;
-        const int prev = oprev ? oprev[ts + i] : -1;
+        const int prev = oprev ? __ldg(&oprev[ts + i]) : -1;
         if (dprev) dprev[o] = prev;
         v.sroot[o] = start_hint(v, s, cnt, prev, reuse, reused);
         if (reset_parent) v.parent[s] = s;
@@ -2315,8 +2319,9 @@ __device__ __forceinline__ void flatten_body(const View& v, int bx, int nbx, Str
         bool need = false;
         if (i < n) {
             const int slot = sw[4 * (size_t)i];
-            if (scnt[i] >= v.min_pts) {
-                const int root = uf_find(v.parent, v.sroot[i]);
+            const int at = v.sroot[i];
+            if (at >= 0) {
+                const int root = uf_find(v.parent, at);
                 v.rslot[slot] = root;
                 if (keep_roots) v.sprev[cur][i] = root;  // the next slide's reuse reads it by position
             } else {
@@ -2582,10 +2587,10 @@ struct PhaseShape;
 template <> struct PhaseShape<kBatchIngest> { static constexpr int threads = 256, min_blocks = 1; };
 template <> struct PhaseShape<kBatchSort> { static constexpr int threads = kSortRun, min_blocks = 1; };
 template <> struct PhaseShape<kBatchRunmerge> { static constexpr int threads = kSortRun, min_blocks = 1; };
-template <> struct PhaseShape<kBatchDecrement> { static constexpr int threads = 256, min_blocks = 8; };
+template <> struct PhaseShape<kBatchDecrement> { static constexpr int threads = 256, min_blocks = 6; };
 template <> struct PhaseShape<kBatchMerge> { static constexpr int threads = kMergeThreads, min_blocks = 1; };
 template <> struct PhaseShape<kBatchBuild> { static constexpr int threads = kBuildThreads, min_blocks = 1; };
-template <> struct PhaseShape<kBatchIncrement> { static constexpr int threads = 256, min_blocks = 8; };
+template <> struct PhaseShape<kBatchIncrement> { static constexpr int threads = 256, min_blocks = 6; };
 template <> struct PhaseShape<kBatchLink> { static constexpr int threads = kLinkThreads, min_blocks = 1; };
 template <> struct PhaseShape<kBatchUnion> { static constexpr int threads = kClusterThreads, min_blocks = kUnionBlocks; };
 template <> struct PhaseShape<kBatchFlatten> { static constexpr int threads = 256, min_blocks = 6; };
