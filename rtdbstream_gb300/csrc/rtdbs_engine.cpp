@@ -174,7 +174,9 @@ void set_band(View& v, double eps) {
     v.lo = flo;
     v.hi = fhi;
     v.E = E;
-    v.filter_ok = (E >= std::ldexp(1.0, -100) && E <= std::ldexp(1.0, 100)) ? 1 : 0;
+    // outside the range where the analysis holds the filter is off: NaN bounds
+    // decide nothing, so every test is made in double
+    if (!(E >= std::ldexp(1.0, -100) && E <= std::ldexp(1.0, 100))) v.lo = v.hi = NAN;
     const float r = (float)eps;
     v.r2f = r * r;
 }

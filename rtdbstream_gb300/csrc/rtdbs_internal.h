@@ -117,9 +117,8 @@ struct View {
     int pbits;                  // log2 of table capacity
     unsigned pmask;
     float r2f;                  // FP32 mode: (float)eps * (float)eps
-    float lo, hi;               // FP64 mode: FP32 filter band
+    float lo, hi;               // FP64 mode: FP32 filter band (NaN: every test in FP64)
     double E;                   // FP64 mode: eps * eps
-    int filter_ok;              // FP64 mode: band valid (else every test in FP64)
     int key_bits;
     int sort_passes, sort_bits;  // radix passes over a chunk's keys, bits per pass
     int block_pts;              // sorted positions a union warp takes as one block (16 or 32;
@@ -233,7 +232,7 @@ cudaError_t configure_kernels();
 // Records the text rtdbs_last_error returns on this thread; returns status.
 int set_error(int status, const char* fmt, ...);
 // FP32 filter band of the FP64 predicate and the FP32 radius (View::lo, hi,
-// E, filter_ok, r2f) for this Eps.
+// E, r2f) for this Eps.
 void set_band(View& v, double eps);
 // Grid geometry of View v (origin, extents, key fields, inv_cell, key_bits,
 // sort_passes) for cells of side Eps (1 + 2^-12) / cells_per_eps over the

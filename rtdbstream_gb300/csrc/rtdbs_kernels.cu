@@ -166,9 +166,9 @@ __device__ __forceinline__ bool nbr_decide(const View& v, float d, const float4&
     bool nb;
     if (MODE == kPrecFp32) {
         nb = d < v.r2f;
-    } else if (v.filter_ok && d < v.lo) {
+    } else if (d < v.lo) {  // (lo and hi are NaN where the filter is off: all in double)
         nb = true;
-    } else if (v.filter_ok && d >= v.hi) {
+    } else if (d >= v.hi) {
         nb = false;
     } else {
         ++t.rechecks;
@@ -247,6 +247,24 @@ __device__ __forceinline__ int2 table_find_at(const ulonglong2* T, unsigned pmas
         const ulonglong2 e = T[s];
         if (e.x == tag) return make_int2((int)(unsigned)e.y, (int)(unsigned)(e.y >> 32));
         if ((e.x >> kKeyBitsMax) != gen) break;  // empty or stale slot ends the probe
+        s = (s + 1) & pmask;
+    }
+    return make_int2(0, 0);
+}
+
+// A table entry as four words: tag (low, high), start, end.  The 32-bit key
+// path compares words: the tag of a key below 2^32 is the key and gen << 18.
+__device__ __forceinline__ uint4 table_entry(const ulonglong2* T, unsigned s) {
+    return reinterpret_cast<const uint4*>(T)[s];
+}
+
+// table_find_at for a 32-bit key, from slot s on.
+__device__ __forceinline__ int2 table_find_from32(const ulonglong2* T, unsigned pmask, unsigned s, unsigned key,
+                                                  unsigned ghi) {
+    for (unsigned i = 0; i <= pmask; ++i) {
+        const uint4 e = table_entry(T, s);
+        if (e.x == key && e.y == ghi) return make_int2((int)e.z, (int)e.w);
+        if ((e.y ^ ghi) >> (kKeyBitsMax - 32)) break;  // empty or stale slot ends the probe
         s = (s + 1) & pmask;
     }
     return make_int2(0, 0);
@@ -332,7 +350,7 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
         const unsigned c1 = (k32 >> s1) & ((1u << (s0 - s1)) - 1u);
         const unsigned c0 = k32 >> s0;
         const unsigned e0 = (unsigned)v.ext[0], e1 = (unsigned)v.ext[1], e2 = (unsigned)v.ext[2];
-        const unsigned long long gtag = (unsigned long long)gen << kKeyBitsMax;
+        const unsigned ghi = gen << (kKeyBitsMax - 32);
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
             rg[k] = make_int2(0, 0);
@@ -353,7 +371,7 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
                 }
                 if (q0 < e0 && q1 < e1 && q2 < e2) {
                     const unsigned nk = (q0 << s0) | (q1 << s1) | q2;
-                    rg[k] = table_find_at(T, v.pmask, table_home32(nk, v.pbits), gtag | nk);
+                    rg[k] = table_find_from32(T, v.pmask, table_home32(nk, v.pbits), nk, ghi);
                 }
             }
         }
@@ -416,53 +434,88 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
 // One row of the stencil around a cell, looked up by one lane: kept row
 // `row` of Stencil<DIM, HALF, K> as a range of sorted positions (empty: 0, 0).
 // The first probes of the row's cells are issued together.
-template <int DIM, bool HALF, int K, bool SMALL>
-__device__ __forceinline__ int2 row_range_lane_t(const View& v, const ulonglong2* T, unsigned gen,
-                                                 unsigned long long key, int row) {
+template <int DIM, bool HALF, int K>
+__device__ __forceinline__ int2 row_range_lane32(const View& v, const ulonglong2* T, unsigned gen, unsigned key,
+                                                 int row) {
     using St = Stencil<DIM, HALF, K>;
-    using C = typename std::conditional<SMALL, int, long long>::type;  // cell coordinates
     constexpr int kW = St::kW;
     const int arow = St::kFirst + row;
     const bool centre = HALF && row == 0;  // its cells below the home cell are not kept
     const int s0 = v.shift[0], s1 = v.shift[1];
-    C q0 = (C)(key >> s0), q1 = (C)((key >> s1) & ((1ull << (s0 - s1)) - 1ull)), q2 = (C)(key & ((1ull << s1) - 1ull));
-    if (DIM == 2) {
-        q0 += arow - K;
-    } else if (DIM == 3) {
-        q0 += arow / kW - K;
-        q1 += arow % kW - K;
+    // coordinates wrap below zero, so one unsigned comparison bounds each axis
+    unsigned ql, el, rowkey;  // along the row: coordinate and extent; the rest of the key
+    int sl;
+    bool in = true;
+    if (DIM == 1) {
+        ql = key >> s0;
+        el = (unsigned)v.ext[0];
+        rowkey = 0;
+        sl = s0;
+    } else if (DIM == 2) {
+        const unsigned q0 = (key >> s0) + (unsigned)(arow - K);
+        in = q0 < (unsigned)v.ext[0];
+        ql = (key >> s1) & ((1u << (s0 - s1)) - 1u);
+        el = (unsigned)v.ext[1];
+        rowkey = q0 << s0;
+        sl = s1;
+    } else {
+        const unsigned q0 = (key >> s0) + (unsigned)(arow / kW - K);
+        const unsigned q1 = ((key >> s1) & ((1u << (s0 - s1)) - 1u)) + (unsigned)(arow % kW - K);
+        in = q0 < (unsigned)v.ext[0] && q1 < (unsigned)v.ext[1];
+        ql = key & ((1u << s1) - 1u);
+        el = (unsigned)v.ext[2];
+        rowkey = (q0 << s0) | (q1 << s1);
+        sl = 0;
     }
-    const C e0 = (C)v.ext[0], e1 = (C)v.ext[1], e2 = (C)v.ext[2];
-    C& ql = DIM == 1 ? q0 : (DIM == 2 ? q1 : q2);  // the axis along the row
-    const C el = DIM == 1 ? e0 : (DIM == 2 ? e1 : e2);
-    const bool in = (DIM == 1 || (q0 >= 0 && q0 < e0)) && (DIM < 3 || (q1 >= 0 && q1 < e1));
     if (!in) return make_int2(0, 0);
-    const C mid = ql;
-    ql = 0;
-    const unsigned long long rowkey =
-        ((unsigned long long)q0 << s0) | ((unsigned long long)q1 << s1) | (unsigned long long)q2;
-    const int sl = DIM == 1 ? s0 : (DIM == 2 ? s1 : 0);
-    const unsigned long long gtag = (unsigned long long)gen << kKeyBitsMax;
-    ulonglong2 e[kW];
-    unsigned home[kW];
+    const unsigned ghi = gen << (kKeyBitsMax - 32);
+    uint4 e[kW];
 #pragma unroll
     for (int k = 0; k < kW; ++k) {
-        const C q = mid + (k - K);
-        e[k].x = 0ull;  // no generation
-        home[k] = 0;
-        if (q >= 0 && q < el && !(centre && k < K)) {
-            const unsigned long long nk = rowkey | ((unsigned long long)q << sl);
-            home[k] = SMALL ? table_home32((unsigned)nk, v.pbits) : table_home(nk, v.pbits);
-            e[k] = T[home[k]];
-        }
+        const unsigned q = ql + (unsigned)(k - K);
+        e[k] = make_uint4(0, 0, 0, 0);  // no generation
+        if (q < el && !(centre && k < K)) e[k] = table_entry(T, table_home32(rowkey | (q << sl), v.pbits));
     }
     int rs = INT_MAX, re = 0;
 #pragma unroll
     for (int k = 0; k < kW; ++k) {
-        if ((e[k].x >> kKeyBitsMax) != gen) continue;  // out of the grid, or an empty or stale slot
-        const unsigned long long tag = gtag | rowkey | ((unsigned long long)(mid + (k - K)) << sl);
-        const int2 c = e[k].x == tag ? make_int2((int)(unsigned)e[k].y, (int)(unsigned)(e[k].y >> 32))
-                                     : table_find_at(T, v.pmask, (home[k] + 1) & v.pmask, tag);
+        if ((e[k].y ^ ghi) >> (kKeyBitsMax - 32)) continue;  // out of the grid, or an empty or stale slot
+        const unsigned nk = rowkey | ((ql + (unsigned)(k - K)) << sl);
+        int2 c = make_int2((int)e[k].z, (int)e[k].w);
+        if (e[k].x != nk)
+            c = table_find_from32(T, v.pmask, (table_home32(nk, v.pbits) + 1) & v.pmask, nk, ghi);
+        if (c.y > c.x) {
+            rs = min(rs, c.x);
+            re = max(re, c.y);
+        }
+    }
+    return re > 0 ? make_int2(rs, re) : make_int2(0, 0);
+}
+
+template <int DIM, bool HALF, int K>
+__device__ __noinline__ int2 row_range_lane64(const View& v, const ulonglong2* T, unsigned gen,
+                                              unsigned long long key, int row) {
+    using St = Stencil<DIM, HALF, K>;
+    constexpr int kW = St::kW;
+    const int arow = St::kFirst + row;
+    const int s0 = v.shift[0], s1 = v.shift[1];
+    long long q[3] = {(long long)(key >> s0), (long long)((key >> s1) & ((1ull << (s0 - s1)) - 1ull)),
+                      (long long)(key & ((1ull << s1) - 1ull))};
+    if (DIM == 2) q[0] += arow - K;
+    if (DIM == 3) {
+        q[0] += arow / kW - K;
+        q[1] += arow % kW - K;
+    }
+    const long long mid = q[DIM - 1];
+    int rs = INT_MAX, re = 0;
+    for (int k = HALF && row == 0 ? K : 0; k < kW; ++k) {
+        q[DIM - 1] = mid + (k - K);
+        bool in = true;
+        for (int a = 0; a < DIM; ++a) in = in && q[a] >= 0 && q[a] < v.ext[a];
+        if (!in) continue;
+        const unsigned long long nk = ((unsigned long long)q[0] << s0) | ((unsigned long long)q[1] << s1) |
+                                      (unsigned long long)q[2];
+        const int2 c = table_find(T, v.pmask, v.pbits, tag_of(nk, gen));
         if (c.y > c.x) {
             rs = min(rs, c.x);
             re = max(re, c.y);
@@ -474,8 +527,8 @@ __device__ __forceinline__ int2 row_range_lane_t(const View& v, const ulonglong2
 template <int DIM, bool HALF, int K>
 __device__ __forceinline__ int2 row_range_lane(const View& v, const ulonglong2* T, unsigned gen,
                                                unsigned long long key, int row) {
-    if (v.key_bits <= 31) return row_range_lane_t<DIM, HALF, K, true>(v, T, gen, key, row);
-    return row_range_lane_t<DIM, HALF, K, false>(v, T, gen, key, row);
+    if (v.key_bits <= 31) return row_range_lane32<DIM, HALF, K>(v, T, gen, (unsigned)key, row);
+    return row_range_lane64<DIM, HALF, K>(v, T, gen, key, row);
 }
 
 // The group's row ranges (group lanes 0..ROWS-1), clipped below at `lo`,
@@ -2041,12 +2094,16 @@ __device__ __forceinline__ int union_grab(const View& v) { return max(1, v.grab 
 // Bound by instruction issue and L2 latency (DRAM throughput 5%).  Against one
 // cell per warp, candidates looked up 14 cells at a time with shuffles, a find
 // and a hook per near pair: link and union 225 -> 168 us on the 1M-point
-// walker window (10.8 -> 4.4 M distance tests), 74 -> 41 us on the 500k precision stream, 297 -> 79 us on 200k trajectories, 520
-// -> 62 us on 100k prices, 606 -> 286 us per round of a 32-stream pool.
+// walker window (10.8 -> 4.4 M distance tests), 74 -> 41 us on the 500k
+// precision stream, 297 -> 79 us on 200k trajectories, 520 -> 62 us on 100k
+// prices, 606 -> 286 us per round of a 32-stream pool.
 // Without the root lookups before the tests: 204, 41, 129, 142, 430.
-// Thread blocks per SM 4 / 5 / 6: pool round 312 / 286 / 304 us, walkers at 5 /
-// 6 167 / 168 (registers against warps in flight).
-constexpr int kUnionBlocks = 5;
+// Row lookups in 32-bit words, and no filter flag beside the band, took its
+// register spills away (100-230 bytes a thread): walkers 168 -> 162, pool 288 ->
+// 278.  Thread blocks per SM 4 / 5 / 6: walkers 172 / 162 / 156 us, pool round
+// 298 / 278 / 287 (registers against warps in flight).
+constexpr int kUnionBlocks = 6;      // of a window slid alone
+constexpr int kPoolUnionBlocks = 5;
 
 template <int DIM, int K>
 struct UnionRows {
@@ -2592,7 +2649,7 @@ template <> struct PhaseShape<kBatchMerge> { static constexpr int threads = kMer
 template <> struct PhaseShape<kBatchBuild> { static constexpr int threads = kBuildThreads, min_blocks = 1; };
 template <> struct PhaseShape<kBatchIncrement> { static constexpr int threads = 256, min_blocks = 6; };
 template <> struct PhaseShape<kBatchLink> { static constexpr int threads = kLinkThreads, min_blocks = 1; };
-template <> struct PhaseShape<kBatchUnion> { static constexpr int threads = kClusterThreads, min_blocks = kUnionBlocks; };
+template <> struct PhaseShape<kBatchUnion> { static constexpr int threads = kClusterThreads, min_blocks = kPoolUnionBlocks; };
 template <> struct PhaseShape<kBatchFlatten> { static constexpr int threads = 256, min_blocks = 6; };
 template <> struct PhaseShape<kBatchLabel> { static constexpr int threads = kClusterThreads, min_blocks = 5; };
 
