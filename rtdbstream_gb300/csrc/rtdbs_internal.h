@@ -63,6 +63,7 @@ constexpr int kErrList = 16;
 struct Ctl {
     long long b;               // grid builds so far (merge + table build)
     long long slide;           // slides completed
+    int unit;                  // slide % units: the stride of ring slots that comes next
     int nocc[2];               // entries in sorted buffer 0 / 1
     int nitems;                // cell runs (within 32 sorted positions) of the current grid
     int ncells;                // cells of the current grid

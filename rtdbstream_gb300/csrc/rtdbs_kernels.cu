@@ -103,8 +103,13 @@ __device__ __forceinline__ unsigned gen_of_build(long long b) {
 }
 
 __device__ __forceinline__ int chunk_base_slot(const View& v, int j, int init) {
-    const int base = init ? 0 : (int)(v.ctl->slide % v.units) * v.S;
+    const int base = init ? 0 : v.ctl->unit * v.S;
     return base + j * v.chunk;
+}
+
+__device__ __forceinline__ void end_slide(const View& v) {
+    v.ctl->slide += 1;
+    v.ctl->unit = v.ctl->unit + 1 < v.units ? v.ctl->unit + 1 : 0;
 }
 
 // The expiring chunk's (key, slot) order is known from the slide that
@@ -351,9 +356,13 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
         const unsigned c0 = k32 >> s0;
         const unsigned e0 = (unsigned)v.ext[0], e1 = (unsigned)v.ext[1], e2 = (unsigned)v.ext[2];
         const unsigned ghi = gen << (kKeyBitsMax - 32);
+        uint4 e[kPer];  // first probes, issued together
+        unsigned nks[kPer];
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
             rg[k] = make_int2(0, 0);
+            e[k] = make_uint4(0, 0, 0, 0);  // no generation
+            nks[k] = 0;
             const int cs = lane + k * G;
             const int row = St::kFirst + cs / kW, d_last = cs % kW - K;
             const bool skip = HALF && cs < kW && d_last < 0;
@@ -370,10 +379,17 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
                     q2 += (unsigned)d_last;
                 }
                 if (q0 < e0 && q1 < e1 && q2 < e2) {
-                    const unsigned nk = (q0 << s0) | (q1 << s1) | q2;
-                    rg[k] = table_find_from32(T, v.pmask, table_home32(nk, v.pbits), nk, ghi);
+                    nks[k] = (q0 << s0) | (q1 << s1) | q2;
+                    e[k] = table_entry(T, table_home32(nks[k], v.pbits));
                 }
             }
+        }
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) {
+            if ((e[k].y ^ ghi) >> (kKeyBitsMax - 32)) continue;
+            rg[k] = e[k].x == nks[k]
+                        ? make_int2((int)e[k].z, (int)e[k].w)
+                        : table_find_from32(T, v.pmask, (table_home32(nks[k], v.pbits) + 1) & v.pmask, nks[k], ghi);
         }
     } else {
     const long long c2 = (long long)(key & ((1ull << v.shift[1]) - 1ull));
@@ -748,7 +764,7 @@ __device__ __forceinline__ bool damage_on(const View& v) {
 
 // The slide's new slots: [base, base + S).
 __device__ __forceinline__ bool slot_is_new(const View& v, int s) {
-    const int base = (int)(v.ctl->slide % v.units) * v.S;
+    const int base = v.ctl->unit * v.S;
     return s >= base && s < base + v.S;
 }
 
@@ -990,6 +1006,17 @@ __global__ void __launch_bounds__(kSortRun) k_runmerge(View v, int j, int c, int
     runmerge_body(v, j, c, init, blockIdx.x, blockIdx.y, words);
 }
 
+// Count passes of a stream slid alone: blocks of 128 threads, 9 per SM (56
+// registers), so that the 5,000 warps of 10,000 queries are resident at once.
+// They are one wave of dependent loads, bound by latency.  With 256-thread
+// blocks, 5 per SM, a candidate pair's loads only when it was worked on and the
+// table probes of a lane one after the other, decrement and increment took 31 +
+// 39 us on 200k trajectories (now 26 + 35), 30 + 35 on 100k prices (26 + 29),
+// 24 + 23 on 1M walkers (21 + 25); 8 and 10 blocks per SM: walkers 27 + 27 and 22
+// + 25, trajectories 26 + 33 and 32 + 41.
+constexpr int kQueryThreads = 128;
+constexpr int kQueryBlocks = 9;
+
 // -1 on the count of every surviving neighbour of each expired point (old grid).
 // G lanes scan one query point's neighbourhood (View::qlanes): 16 (two points
 // per warp, so two queries' dependent loads overlap) or 32; the 25 rows of the
@@ -1006,7 +1033,7 @@ struct StreamSmem {
     int nq;
 };
 
-template <int MODE, int DK, int G>
+template <int MODE, int DK, int G, bool AHEAD>
 __device__ __forceinline__ void decr_g(const View& v, int j, int c, int bx, StreamSmem& sm) {
     constexpr int DIM = DK & 3, K = (DK >> 2) + 1;  // dimension, cells per Eps
     constexpr int kPerWarp = 32 / G;
@@ -1048,14 +1075,27 @@ __device__ __forceinline__ void decr_g(const View& v, int j, int c, int bx, Stre
     Tally tally;
     int r = 0;
     // Two candidates per lane and trip (idx and idx + G): their loads are in
-    // flight together and one paired distance evaluation serves both.
+    // flight together and one paired distance evaluation serves both.  AHEAD
+    // (streams slid alone, whose passes are one wave of dependent loads): the
+    // next trip's loads are issued before this one is worked on.
+    int npos0 = 0, npos1 = 0, ncnt0 = 0, ncnt1 = 0;
+    float4 nq0 = make_float4(0.f, 0.f, 0.f, 0.f), nq1 = nq0;
+    auto fetch = [&](int at) {
+        npos0 = stream_pos(at, r, rstart, rpre);
+        npos1 = at + G < total ? stream_pos(at + G, r, rstart, rpre) : npos0;
+        nq0 = spt[npos0];
+        nq1 = spt[npos1];
+        // counts only fall here: >= MinPts means no list kept
+        ncnt0 = scnt[npos0];
+        ncnt1 = scnt[npos1];
+    };
+    if (AHEAD && gl < total) fetch(gl);
     for (int idx = gl; idx < total; idx += 2 * G) {
         const bool two = idx + G < total;
-        const int pos0 = stream_pos(idx, r, rstart, rpre);
-        const int pos1 = two ? stream_pos(idx + G, r, rstart, rpre) : pos0;
-        const float4 q0 = spt[pos0], q1 = spt[pos1];
-        // counts only fall here: >= MinPts means no list kept
-        const int cnt0 = scnt[pos0], cnt1 = scnt[pos1];
+        if (!AHEAD) fetch(idx);
+        const int pos0 = npos0, pos1 = npos1, cnt0 = ncnt0, cnt1 = ncnt1;
+        const float4 q0 = nq0, q1 = nq1;
+        if (AHEAD && idx + 2 * G < total) fetch(idx + 2 * G);
         const int qs0 = slot_of(q0), qs1 = slot_of(q1);
         float d0, d1;
         sqdist32x2<DIM>(xp, q0, q1, d0, d1);
@@ -1082,22 +1122,22 @@ __device__ __forceinline__ void decr_g(const View& v, int j, int c, int bx, Stre
 
 // The count passes' lane group, chosen per stream at run time (uniform per
 // launch): 16 or 32 lanes with one cell per Eps, 32 with two.
-template <int MODE, int DK>
+template <int MODE, int DK, bool AHEAD>
 __device__ __forceinline__ void decr_body(const View& v, int j, int c, int bx, StreamSmem& sm) {
     if constexpr ((DK >> 2) == 0) {
         if (v.qlanes == 16) {
-            decr_g<MODE, DK, 16>(v, j, c, bx, sm);
+            decr_g<MODE, DK, 16, AHEAD>(v, j, c, bx, sm);
             return;
         }
     }
-    decr_g<MODE, DK, 32>(v, j, c, bx, sm);
+    decr_g<MODE, DK, 32, AHEAD>(v, j, c, bx, sm);
 }
 
 template <int MODE, int DK>
-__global__ void __launch_bounds__(256) k_decr(View v, int j, int c) {
+__global__ void __launch_bounds__(kQueryThreads, kQueryBlocks) k_decr(View v, int j, int c) {
     pdl_wait();
     __shared__ StreamSmem sm;
-    decr_body<MODE, DK>(v, j, c, blockIdx.x, sm);
+    decr_body<MODE, DK, true>(v, j, c, blockIdx.x, sm);
 }
 
 __device__ __forceinline__ bool tuple_less(unsigned long long ka, int sa, unsigned long long kb,
@@ -1410,7 +1450,7 @@ __global__ void __launch_bounds__(kBuildThreads) k_build(View v) {
 }
 
 // Full count of each new point and +1 on every older neighbour (new grid).
-template <int MODE, int DK, int G>
+template <int MODE, int DK, int G, bool AHEAD>
 __device__ __forceinline__ void incr_g(const View& v, int j, int c, int init, int bx, StreamSmem& sm) {
     constexpr int DIM = DK & 3, K = (DK >> 2) + 1;  // dimension, cells per Eps
     constexpr int kPerWarp = 32 / G;
@@ -1444,20 +1484,33 @@ __device__ __forceinline__ void incr_g(const View& v, int j, int c, int init, in
     Tally tally;
     int count = 0, mypos = -1, r = 0, nfound = 0;
     // Two candidates per lane and trip (idx and idx + G), as in the decrement.
+    int npos[2] = {0, 0}, ncnt[2] = {0, 0};
+    float4 nq[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    auto fetch = [&](int at, int* p, int* n, float4* c4) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (at + u * G >= total) continue;
+            p[u] = stream_pos(at + u * G, r, rstart, rpre);
+            c4[u] = spt[p[u]];
+            n[u] = scnt[p[u]];  // counts only rise here: >= MinPts means no list kept
+        }
+    };
+    if (AHEAD) fetch(gl, npos, ncnt, nq);
     for (int base = 0; base < tmax; base += 2 * G) {
         const int idx = base + gl;
         const bool h0 = idx < total, h1 = idx + G < total;
         int pos[2] = {0, 0}, cnt[2] = {0, 0}, qs[2] = {-1, -1};
         float4 q[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
-        if (h0) {
-            pos[0] = stream_pos(idx, r, rstart, rpre);
-            q[0] = spt[pos[0]];
-            cnt[0] = scnt[pos[0]];  // counts only rise here: >= MinPts means no list kept
-        }
-        if (h1) {
-            pos[1] = stream_pos(idx + G, r, rstart, rpre);
-            q[1] = spt[pos[1]];
-            cnt[1] = scnt[pos[1]];
+        if (AHEAD) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                pos[u] = npos[u];
+                cnt[u] = ncnt[u];
+                q[u] = nq[u];
+            }
+            fetch(idx + 2 * G, npos, ncnt, nq);
+        } else {
+            fetch(idx, pos, cnt, q);
         }
         float d[2];
         sqdist32x2<DIM>(ap, q[0], q[1], d[0], d[1]);
@@ -1507,22 +1560,22 @@ __device__ __forceinline__ void incr_g(const View& v, int j, int c, int init, in
     flush_stats(v, tally, err, lane, 0);
 }
 
-template <int MODE, int DK>
+template <int MODE, int DK, bool AHEAD>
 __device__ __forceinline__ void incr_body(const View& v, int j, int c, int init, int bx, StreamSmem& sm) {
     if constexpr ((DK >> 2) == 0) {
         if (v.qlanes == 16) {
-            incr_g<MODE, DK, 16>(v, j, c, init, bx, sm);
+            incr_g<MODE, DK, 16, AHEAD>(v, j, c, init, bx, sm);
             return;
         }
     }
-    incr_g<MODE, DK, 32>(v, j, c, init, bx, sm);
+    incr_g<MODE, DK, 32, AHEAD>(v, j, c, init, bx, sm);
 }
 
 template <int MODE, int DK>
-__global__ void __launch_bounds__(256, 5) k_incr(View v, int j, int c, int init) {
+__global__ void __launch_bounds__(kQueryThreads, kQueryBlocks) k_incr(View v, int j, int c, int init) {
     pdl_wait();
     __shared__ StreamSmem sm;
-    incr_body<MODE, DK>(v, j, c, init, blockIdx.x, sm);
+    incr_body<MODE, DK, true>(v, j, c, init, blockIdx.x, sm);
 }
 
 // ------------------------------------------------------ whole-window build
@@ -2557,7 +2610,7 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, i
     flush_stats(v, tally, 0, lane, 1);
     if (bx == 0 && threadIdx.x == 0) {
         v.ctl->union_next = 0;                // the next clustering's queue; not read here
-        if (advance) v.ctl->slide += 1;       // no reader here
+        if (advance) end_slide(v);            // no reader here
     }
 }
 
@@ -2623,7 +2676,7 @@ __device__ __forceinline__ void border_body(const View& v, int advance, int bx, 
         v.ctl->last_reused = v.ctl->reused;
         v.ctl->reused = 0;
         v.ctl->prev_ok = 1;                   // the forest of this clustering can be reused
-        if (advance) v.ctl->slide += 1;       // no reader here
+        if (advance) end_slide(v);            // no reader here
     }
 }
 
@@ -2698,7 +2751,7 @@ __global__ void __launch_bounds__(PhaseShape<PHASE>::threads, PhaseShape<PHASE>:
         runmerge_body(sv, it.j, it.c, 0, bx % nruns, bx / nruns, words);
     } else if constexpr (PHASE == kBatchDecrement) {
         __shared__ StreamSmem sm;
-        decr_body<MODE, DK>(sv, it.j, it.c, bx, sm);
+        decr_body<MODE, DK, false>(sv, it.j, it.c, bx, sm);
     } else if constexpr (PHASE == kBatchMerge) {
         __shared__ MergeSmem<kMergeTile> sm;
         merge_body(sv, it.j, it.c, 0, bx, nbx, sm);
@@ -2707,7 +2760,7 @@ __global__ void __launch_bounds__(PhaseShape<PHASE>::threads, PhaseShape<PHASE>:
         build_body(sv, bx, sm);
     } else if constexpr (PHASE == kBatchIncrement) {
         __shared__ StreamSmem sm;
-        incr_body<MODE, DK>(sv, it.j, it.c, 0, bx, sm);
+        incr_body<MODE, DK, false>(sv, it.j, it.c, 0, bx, sm);
     } else if constexpr (PHASE == kBatchLink) {
         __shared__ LinkSmem sm;
         link_body<MODE, DK>(sv, bx, sm);
@@ -2807,7 +2860,7 @@ bool pdl_on(const View& v) { return v.W <= kPdlWindow; }
 
 cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, int init,
                          int stg_off, int advance, cudaStream_t s, bool pdl, const SlideIO& io) {
-    const int warp_blocks = (c * v.qlanes + 255) / 256;  // count passes
+    const int warp_blocks = (c * v.qlanes + kQueryThreads - 1) / kQueryThreads;  // count passes
     switch (phase) {
         case kPhaseIngest:
             launch(k_ingest, (c + 255) / 256, 256, 0, s, pdl, v, j, c, init, stg_off, io);
@@ -2822,7 +2875,7 @@ cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, 
             break;
         }
         case kPhaseDecrement:
-            if (!init) RTDBS_DISPATCH(precision, dk_of(v), k_decr, warp_blocks, 256, s, pdl, v, j, c);
+            if (!init) RTDBS_DISPATCH(precision, dk_of(v), k_decr, warp_blocks, kQueryThreads, s, pdl, v, j, c);
             break;
         case kPhaseMerge:
             // short tiles where the blocks are few (10k points 14 -> 10 us, 200k
@@ -2836,7 +2889,7 @@ cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, 
             launch(k_build, (v.W + kBuildThreads - 1) / kBuildThreads, kBuildThreads, 0, s, pdl, v);
             break;
         case kPhaseIncrement:
-            RTDBS_DISPATCH(precision, dk_of(v), k_incr, warp_blocks, 256, s, pdl, v, j, c, init);
+            RTDBS_DISPATCH(precision, dk_of(v), k_incr, warp_blocks, kQueryThreads, s, pdl, v, j, c, init);
             break;
         case kPhaseLabel:
             if (v.list_cap >= 0) {
