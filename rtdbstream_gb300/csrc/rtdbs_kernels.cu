@@ -1584,7 +1584,7 @@ __global__ void __launch_bounds__(kQueryThreads, kQueryBlocks) k_incr(View v, in
 // word, a radix sort orders them, one pass lays the window out in that order,
 // the cell table is built once and every point's neighbours are counted once
 // (k_count), instead of W / 16384 chunk steps that each rewrite the window.
-// A 1M-point walker window: load 9.9 -> 0.45 ms (sort 60 us, count 275 us; the
+// A 1M-point walker window: load 9.9 -> 0.40 ms (sort 52 us, count 240 us; the
 // box of the points is taken on the device, not in a host loop over a copy);
 // 48k points replaced per slide: 327 -> 137 us for the grid.
 // Words are key << ob | slot (ob bits for the slots; the host takes the chunk
@@ -1598,7 +1598,7 @@ constexpr int kRadTile = kRadThreads * kRadItems;      // words per block
 constexpr int kRadWarps = kRadThreads / 32;
 // Digits of up to 10 bits, as equal as the key's bits allow: a key of 18 or 20
 // bits takes two passes, one of 25 three, where 8-bit digits took three and
-// four (48k points 44 -> 27 us, 1M 97 -> 60).
+// four (48k points 44 -> 25 us, 1M 97 -> 52).
 constexpr int kRadBits = 10;
 inline int rad_passes(const View& v) { return (v.key_bits + kRadBits - 1) / kRadBits; }
 inline int rad_bits(const View& v) {  // (at least 5: the scan takes 32 digits a block)
@@ -1679,14 +1679,14 @@ __global__ void __launch_bounds__(kRadThreads) k_rad_hist(View v, int pass, int 
 }
 
 // Exclusive scan over the tiles of 32 digits per block (a warp's lanes side by
-// side), 8 warps on an eighth of the tiles each; the digits' totals follow
-// the tiles' counters.  Only where there are many tiles (kRadInline).
-__global__ void __launch_bounds__(256) k_rad_scan(View v, int ntiles, int bins) {
+// side), 32 warps on a part of the tiles each; the digits' totals follow the
+// tiles' counters.  Only where there are many tiles (kRadInline).
+__global__ void __launch_bounds__(1024) k_rad_scan(View v, int ntiles, int bins) {
     pdl_wait();
-    __shared__ int part[8][32];
+    __shared__ int part[32][32];
     int* counts = v.scnt[(v.ctl->b & 1) ^ 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, d = blockIdx.x * 32 + lane;
-    const int per = (ntiles + 7) / 8, t0 = min(w * per, ntiles), t1 = min(t0 + per, ntiles);
+    const int per = (ntiles + 31) / 32, t0 = min(w * per, ntiles), t1 = min(t0 + per, ntiles);
     int sum = 0;
 #pragma unroll 8
     for (int t = t0; t < t1; ++t) sum += counts[t * bins + d];
@@ -1700,7 +1700,7 @@ __global__ void __launch_bounds__(256) k_rad_scan(View v, int ntiles, int bins) 
         counts[t * bins + d] = at;
         at += x;
     }
-    if (w == 7) counts[ntiles * bins + d] = at;
+    if (w == 31) counts[ntiles * bins + d] = at;
 }
 
 // Stable scatter of one tile by its digit: each warp ranks its 256
@@ -1839,7 +1839,9 @@ __global__ void k_fill(View v, int ob, int passes) {
 // rank and a store per test: 1M walkers 349 us against 276, 200k dense
 // trajectories 263 against 136).  Bound by instruction issue; against one
 // whole-stencil query per point with atomics on its neighbours, as the chunk
-// steps count, 1M walkers take 0.28 ms instead of 1.8.
+// steps count, 1M walkers take 0.24 ms instead of 1.8.
+// Blocks per SM 8 / 10 / 12: 1M walkers 268 / 245 / 240 us; two cells per Eps
+// spill above 8 (48k points replaced per slide 115 / 125 / 122).
 constexpr int kCountThreads = 128;
 
 template <int DIM, int K>
@@ -1869,7 +1871,7 @@ __device__ __forceinline__ unsigned lane_range(int lo, int hi) {  // lanes [lo, 
 }
 
 template <int MODE, int DK>
-__global__ void __launch_bounds__(kCountThreads, 8) k_count(View v, int P) {
+__global__ void __launch_bounds__(kCountThreads, (DK >> 2) == 0 ? 12 : 8) k_count(View v, int P) {
     pdl_wait();
     constexpr int DIM = DK & 3, K = (DK >> 2) + 1;
     using C = CountShape<DIM, K>;
@@ -2976,7 +2978,7 @@ cudaError_t launch_window_phase(int phase, const View& v, int precision, const S
                 const int tiles = (v.W + kRadTile - 1) / kRadTile, shift = ob + bits * p;
                 launch(k_rad_hist, tiles, kRadThreads, 0, s, pdl, v, p, passes, shift, bits);
                 const int scanned = tiles > kRadInline;
-                if (scanned) launch(k_rad_scan, (1 << bits) / 32, 256, 0, s, true, v, tiles, 1 << bits);
+                if (scanned) launch(k_rad_scan, (1 << bits) / 32, 1024, 0, s, true, v, tiles, 1 << bits);
                 launch(k_rad_scatter, tiles, kRadThreads, 0, s, true, v, p, passes, shift, bits, scanned);
                 pdl = true;
             }
@@ -2992,7 +2994,7 @@ cudaError_t launch_window_phase(int phase, const View& v, int precision, const S
             // positions per warp (at most CountShape's): short chains while the
             // blocks are few, fuller lookups above.  us with 8 / 16 / 32: 20k
             // points 14 / 20 / 28, 48k 39 / 43 / 66, 200k trajectories 141 / 136
-            // / 152, 1M walkers 358 / 300 / 276
+            // / 152, 1M walkers 358 / 300 / 276 (at 8 blocks per SM)
             const int block = v.W < 65536 ? 8 : (v.W < 524288 || (v.dim == 3 && v.cell_mult == 2) ? 16 : 32);
             const int per = block * (kCountThreads / 32);
             RTDBS_DISPATCH(precision, dk_of(v), k_count, (v.W + per - 1) / per, kCountThreads, s, pdl, v, block);
@@ -3023,10 +3025,15 @@ int window_build_launches(const View& v) {
 
 // Finite bounding box of n points per axis, as order-keeping unsigned keys
 // (box[0..2] minima from ~0, box[3..5] maxima from 0).
-__global__ void k_bbox(const float* pts, long long n, int dim, unsigned* box) {
+__global__ void __launch_bounds__(256) k_bbox(const float* pts, long long n, int dim, unsigned* box) {
+    __shared__ unsigned sbox[6];  // (one global atomic per block and bound)
+    if (threadIdx.x < 6) sbox[threadIdx.x] = threadIdx.x < 3 ? ~0u : 0u;
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     unsigned lo[3] = {~0u, ~0u, ~0u}, hi[3] = {0u, 0u, 0u};
+#pragma unroll 4
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+#pragma unroll
         for (int a = 0; a < 3; ++a) {
             if (a >= dim) break;
             const float x = pts[i * dim + a];
@@ -3036,13 +3043,18 @@ __global__ void k_bbox(const float* pts, long long n, int dim, unsigned* box) {
             lo[a] = min(lo[a], k);
             hi[a] = max(hi[a], k);
         }
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
-        if (a >= dim) break;
         const unsigned l = __reduce_min_sync(kFull, lo[a]), h = __reduce_max_sync(kFull, hi[a]);
         if (lane == 0 && l <= h) {
-            atomicMin(&box[a], l);
-            atomicMax(&box[3 + a], h);
+            atomicMin(&sbox[a], l);
+            atomicMax(&sbox[3 + a], h);
         }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3 && sbox[threadIdx.x] <= sbox[3 + threadIdx.x]) {
+        atomicMin(&box[threadIdx.x], sbox[threadIdx.x]);
+        atomicMax(&box[3 + threadIdx.x], sbox[3 + threadIdx.x]);
     }
 }
 
