@@ -3,12 +3,11 @@
 Three knobs change how the engine works without changing its results:
 - ``cell_mult`` (K): grid cells per Eps along each axis.  K = 2 scans the
   (2K+1)^d = 5^d cells of side Eps/2 around a point, which tests fewer pairs
-  where cells are dense, but costs more cells, table lookups and work items
-  where they are sparse.
-- ``work_grab``: work items (cell runs) a clustering warp takes from the
-  shared queue at a time -- the work split between warps.  Small grabs balance
-  uneven items; large ones keep consecutive cells on one warp and cost fewer
-  queue atomics.
+  where cells are dense, but costs more cells and table lookups where they are
+  sparse.
+- ``work_grab``: cell runs a union warp takes from the shared queue at a time,
+  in whole blocks of sorted positions (one block up to 31 runs) -- the work
+  split between warps.
 - ``query_lanes``: the block shape of the count passes -- 16 lanes per expired
   or new point (two points per warp, 16 per 256-thread block, their dependent
   loads overlapping) or 32 (one point per warp, half the loop trips where
@@ -22,7 +21,7 @@ of the bucket, and later runs, reuse it.  A stream slid alone is latency-bound
 and one slid in a pool round is throughput-bound, so the two are tuned
 apart: `choose` times a single engine (its first window, then a few slides),
 `choose_batched` times pool rounds over up to 16 streams of each bucket
-together.  The default (one cell per Eps, 8 items per grab) is kept unless a
+together.  The default (one cell per Eps, 8 runs per grab) is kept unless a
 candidate is at least 3% faster, so timing noise does not pick a
 configuration.  Candidates are (cell_mult, work_grab, query_lanes) triples.
 """

@@ -278,7 +278,7 @@ def make_params(dim: int, window_size: int, stride_size: int, radius: float, min
                 use_graph: bool = True, cell_mult: int = 1, work_grab: int = 0,
                 query_lanes: int = 0) -> Params:
     """rtdbs_params for one stream; cell_mult = grid cells per Eps (1 or 2),
-    work_grab = work items per queue grab of the clustering warps (0: 8),
+    work_grab = cell runs per queue grab of the union warps (0: one block),
     query_lanes = lanes per query point in the count passes (0: 16 with one
     cell per Eps in a pool or at strides above 6,080 points, else 32; 16 or 32)."""
     L = load_library()
