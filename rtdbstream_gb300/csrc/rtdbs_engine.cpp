@@ -458,6 +458,18 @@ bool direct_access(const rtdbs_engine* e, const void* p) {
     return a.type == cudaMemoryTypeDevice && a.device == e->device;
 }
 
+// Whether the host may read and write the caller's array as it is (device
+// memory given to a host-buffer call goes through a copy, which checks it).
+bool host_access(const void* p) {
+    cudaPointerAttributes a;
+    if (!p) return true;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type != cudaMemoryTypeDevice;
+}
+
 int copy_in(rtdbs_engine* e, const float* src, size_t npts, int on_device) {
     const size_t bytes = sizeof(float) * npts * e->p.dim;
     CUDA_TRY(cudaMemcpyAsync((void*)e->v.staging, src, bytes,
@@ -482,6 +494,15 @@ int fetch_ctl_and_sync(rtdbs_engine* e) {
     return check_device_error(e);
 }
 
+// Orders the legacy default stream after the work queued on the engine's stream.
+int wait_on_default_stream(rtdbs_engine* e) {
+    const int rc = ensure_side(e);
+    if (rc != RTDBS_OK) return rc;
+    CUDA_TRY(cudaEventRecord(e->ev_fork, e->stream));
+    CUDA_TRY(cudaStreamWaitEvent(cudaStreamLegacy, e->ev_fork, 0));
+    return RTDBS_OK;
+}
+
 // Finite bounding box of the window's points, from the device; per axis 0 to
 // 0 where no coordinate is finite.  Device points of the caller are read on
 // the legacy default stream, after all work queued there and on the engine's
@@ -489,11 +510,9 @@ int fetch_ctl_and_sync(rtdbs_engine* e) {
 int device_bbox(rtdbs_engine* e, const float* d_points, int callers, float* mn, float* mx) {
     cudaStream_t s = e->stream;
     if (callers) {
-        const int rc = ensure_side(e);
+        const int rc = wait_on_default_stream(e);
         if (rc != RTDBS_OK) return rc;
         s = cudaStreamLegacy;
-        CUDA_TRY(cudaEventRecord(e->ev_fork, e->stream));
-        CUDA_TRY(cudaStreamWaitEvent(s, e->ev_fork, 0));
     }
     unsigned box[6];
     unsigned* d_box = reinterpret_cast<unsigned*>(e->d_box);
@@ -649,12 +668,19 @@ int rtdbs_load_window(rtdbs_engine* e, const float* points, int points_on_device
     CUDA_TRY(guard.err);
     const int W = e->p.window, dim = e->p.dim;
     // Host points go to the device once (the sorted points of the side that
-    // this build does not lay out hold them); device points are read in place.
+    // this build does not lay out hold them); device points are read in place
+    // where the kernels may, and else copied the same way.
     const float* d_points = points;
-    if (!points_on_device) {
+    if (!points_on_device || !direct_access(e, points)) {
         d_points = reinterpret_cast<const float*>(e->v.spt[0]);
-        CUDA_TRY(cudaMemcpyAsync(e->v.spt[0], points, sizeof(float) * (size_t)W * dim, cudaMemcpyHostToDevice,
-                                 e->stream));
+        cudaStream_t s = e->stream;
+        if (points_on_device && !e->p.has_bbox) {  // as the box reads the caller's points, see device_bbox
+            const int rc = wait_on_default_stream(e);
+            if (rc != RTDBS_OK) return rc;
+            s = cudaStreamLegacy;
+        }
+        CUDA_TRY(cudaMemcpyAsync(e->v.spt[0], points, sizeof(float) * (size_t)W * dim,
+                                 points_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
     }
     if (!e->p.has_bbox) {
         float mn[3] = {0, 0, 0}, mx[3] = {0, 0, 0};
@@ -716,7 +742,8 @@ int rtdbs_slide(rtdbs_engine* e, const float* new_points, int32_t* label, int32_
     if (!e->loaded) return fail(RTDBS_ERR_STATE, "rtdbs_load_window must come first");
     DeviceGuard guard(e->device);
     CUDA_TRY(guard.err);
-    if (e->h_points) {  // through pinned buffers that the kernels read and write themselves
+    // through pinned buffers that the kernels read and write themselves
+    if (e->h_points && host_access(new_points) && host_access(label) && host_access(cluster_id)) {
         const size_t W = (size_t)e->p.window;
         std::memcpy(e->h_points, new_points, sizeof(float) * (size_t)e->p.stride * e->p.dim);
         int rc = run_slide(e, SlideIO{e->h_points, label ? e->h_label : nullptr, cluster_id ? e->h_cid : nullptr});
@@ -800,7 +827,7 @@ int rtdbs_cluster(rtdbs_engine* e, int32_t* label, int32_t* cluster_id, int on_d
     CUDA_TRY(guard.err);
     const int rc0 = wait_outputs_free(e);
     if (rc0 != RTDBS_OK) return rc0;
-    if (e->h_points && !on_device) {
+    if (e->h_points && !on_device && host_access(label) && host_access(cluster_id)) {
         const SlideIO io{nullptr, label ? e->h_label : nullptr, cluster_id ? e->h_cid : nullptr};
         CUDA_TRY(rtdbs::launch_cluster(e->v, e->p.precision, 0, e->stream, true, nullptr, 0, io));
         const int rc = fetch_ctl_and_sync(e);

@@ -16,24 +16,28 @@
 //     k_merge   old sorted window minus expired plus new, one pass, merge-path
 //               tiles (reference: merge_by_cell_id_and_idx,
 //               src/dbscan/thrust_helper.cu:31-51)
-//     k_build   cell table (tagged open addressing) + work list of cell runs
-//               (replaces compute_offsets_of_cells / set_hybrid_spheres_info /
+//     k_build   cell table (tagged open addressing; replaces
+//               compute_offsets_of_cells / set_hybrid_spheres_info /
 //               optixAccelBuild, src/dbscan/aabb.cu:377-544,
 //               src/dbscan/optix.cpp:438-483)
 //     k_incr    full count of every new point and exact +1 on its neighbours
 //               on the new grid (reference: __raygen__grid/__intersection__grid,
 //               src/dbscan/dbscan.cu:155-194,250-270, which recounts all W)
+//   or, for first windows and large slides, one build from all W slots:
+//     k_ingest_all, k_rad_* (or k_sort), k_fill, k_build, k_count
 //   clustering step
-//     k_union   union-find over core-core pairs, each unordered pair once
+//     k_link    cores joined within 32 sorted positions
+//     k_union   union-find over core-core pairs by blocks of positions
 //               (reference: __raygen__cluster/__intersection__hybrid_radius_sphere,
 //               src/dbscan/dbscan.cu:279-321,354-394; find_repres/unite 9-43)
-//     k_label   labels and ids by slot; border = minimum id of the adjacent
-//               clusters (reference: set_label_kernel + post_cluster_t,
+//     k_flatten, k_border (neighbour lists) or k_flatten, k_label (grid scan)
+//               labels and ids by slot; border = minimum id of the
+//               adjacent clusters (reference: set_label_kernel + post_cluster_t,
 //               src/dbscan/aabb.cu:173-196,575-587)
 //
 // Neighbour predicate: a warp holds 32 candidates in lanes (coalesced float4
 // loads of the cell-sorted window) and tests them against home points
-// broadcast by shuffle.  Squared distances use explicitly rounded IEEE
+// kept in shared memory.  Squared distances use explicitly rounded IEEE
 // operations (no FMA contraction; the count passes evaluate two candidates'
 // differences and squares with paired FP32 instructions, each half rounded
 // the same way), so FP32 mode is bit-identical to the reference's CPU checker

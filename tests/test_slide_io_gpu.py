@@ -102,3 +102,20 @@ def test_host_arrays_at_the_staging_limit(n_w, n_s):
         win[: 2 * n_s] = pts[n_w:]
         _, elab, ecid, _ = O.window_grid(win, 0.4, 6, O.MODE_FP64)
         assert np.array_equal(lab, elab) and np.array_equal(cid[elab != 2], ecid[elab != 2])
+
+
+@pytest.mark.parametrize("bbox", [None, ([-5.0, -5.0], [25.0, 25.0])])
+@pytest.mark.parametrize("odd", [0, 3])
+def test_first_window_from_device_bytes(stream, bbox, odd):
+    """Device points at any byte: read in place where aligned, copied otherwise."""
+    import torch
+
+    pts = stream[0][:W]
+    raw = torch.zeros(8 * W + 64, dtype=torch.uint8, device="cuda")
+    raw[odd: odd + 8 * W].copy_(torch.from_numpy(np.ascontiguousarray(pts)).cuda().reshape(-1).view(torch.uint8))
+    torch.cuda.synchronize()
+    with Engine(2, W, S, EPS, MP, bbox=bbox) as eng:
+        assert load_library().rtdbs_load_window(eng._h, ctypes.c_void_p(raw.data_ptr() + odd), 1) == 0
+        lab, cid = eng.cluster()
+        _, elab, ecid, _ = O.window_grid(pts, EPS, MP, O.MODE_FP64)
+        assert np.array_equal(lab, elab) and np.array_equal(cid[elab != 2], ecid[elab != 2])
