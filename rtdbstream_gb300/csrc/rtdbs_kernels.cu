@@ -340,10 +340,10 @@ constexpr int kMaxRows = 25;  // (2K+1)^2 rows for K = 2 in 3-D
 // (the whole warp, or each 16-lane half for its own key; `lane` counts within
 // the group; a lane looks up one to four cells).  On return group lane
 // r < kRows holds row r as [rs, re) (empty rows: rs == re).
-template <int DIM, bool HALF, int K = 1, int G = 32>
+template <int DIM, int K = 1, int G = 32>
 __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, unsigned gen,
                                            unsigned long long key, int lane, int& rs, int& re) {
-    using St = Stencil<DIM, HALF, K>;
+    using St = Stencil<DIM, false, K>;
     constexpr int kW = St::kW;
     constexpr int kSlots = kW * St::kRows;           // cell slots, kept row by kept row
     constexpr int kPer = (kSlots + G - 1) / G;       // cells per lane
@@ -369,8 +369,7 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
             nks[k] = 0;
             const int cs = lane + k * G;
             const int row = St::kFirst + cs / kW, d_last = cs % kW - K;
-            const bool skip = HALF && cs < kW && d_last < 0;
-            if (cs < kSlots && !skip) {
+            if (cs < kSlots) {
                 unsigned q0 = c0, q1 = c1, q2 = c2;
                 if (DIM == 1) {
                     q0 += (unsigned)d_last;
@@ -404,8 +403,7 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
         rg[k] = make_int2(0, 0);
         const int cs = lane + k * G;                                  // = kW * kept row + cell
         const int row = St::kFirst + cs / kW, d_last = cs % kW - K;
-        const bool skip = HALF && cs < kW && d_last < 0;             // centre row, negative cells
-        if (cs < kSlots && !skip) {
+        if (cs < kSlots) {
             long long q0 = c0, q1 = c1, q2 = c2;
             if (DIM == 1) {
                 q0 += d_last;
@@ -766,12 +764,6 @@ __device__ __forceinline__ bool damage_on(const View& v) {
     return v.list_cap >= 0 && v.ctl->prev_ok && v.ctl->reuse_skip <= 0;
 }
 
-// The slide's new slots: [base, base + S).
-__device__ __forceinline__ bool slot_is_new(const View& v, int s) {
-    const int base = v.ctl->unit * v.S;
-    return s >= base && s < base + v.S;
-}
-
 // Root hint a position starts the union with: -1 for a non-core point; the
 // old root `prev` of a core of an intact component (the root the point had
 // at the last clustering, carried with it by the merges; -1 for a point that
@@ -1068,7 +1060,7 @@ __device__ __forceinline__ void decr_g(const View& v, int j, int c, int bx, Stre
     const float4 xp = has ? v.xpt[k] : make_float4(0.f, 0.f, 0.f, 0.f);
     const unsigned long long key = has ? v.xkey[k] : 0ull;
     int rs, re;
-    row_ranges<DIM, false, K, G>(v, v.table[old], gen, key, gl, rs, re);
+    row_ranges<DIM, K, G>(v, v.table[old], gen, key, gl, rs, re);
     int total = candidate_stream<Stencil<DIM, false, K>::kRows, G>(rs, re, 0, gl, rstart, rpre);
     if (!has) total = 0;
     const float4* spt = v.spt[old];
@@ -1475,7 +1467,7 @@ __device__ __forceinline__ void incr_g(const View& v, int j, int c, int init, in
     const int aslot = el + (int)(word & ((1u << kOffBits) - 1));
     const float4 ap = has ? v.ring[aslot] : make_float4(0.f, 0.f, 0.f, 0.f);
     int rs, re;
-    row_ranges<DIM, false, K, G>(v, v.table[cur], gen, key, gl, rs, re);
+    row_ranges<DIM, K, G>(v, v.table[cur], gen, key, gl, rs, re);
     int total = candidate_stream<Stencil<DIM, false, K>::kRows, G>(rs, re, 0, gl, rstart, rpre);
     if (!has) total = 0;
     int tmax = total;
@@ -2379,7 +2371,7 @@ __device__ __forceinline__ void rebuild_list(const View& v, int at, int cur, uns
     const float4 ap = spt[at];
     const int a = slot_of(ap);
     int rs, re;
-    row_ranges<DIM, false, K>(v, v.table[cur], gen, v.skey[cur][at], lane, rs, re);
+    row_ranges<DIM, K>(v, v.table[cur], gen, v.skey[cur][at], lane, rs, re);
     const int total = candidate_stream<Stencil<DIM, false, K>::kRows>(rs, re, 0, lane, rstart, rpre);
     int r = 0, nfound = 0;
     for (int base = 0; base < total; base += 32) {
