@@ -179,7 +179,8 @@ RTDBS_API int rtdbs_load_window(rtdbs_engine* engine, const float* points, int p
 /* One slide with host buffers: new_points[S][dim] replace slots
  * [u*S, u*S+S) (u = slides done mod W/S), then label[W] and cluster_id[W]
  * (host memory; pinned memory avoids a staging copy) receive the window's
- * result.  Replaces one iteration of the reference's slide loop
+ * result.  Pinned or managed new_points are read in the stream's order, after
+ * work queued before that may still write them.  Replaces one iteration of the reference's slide loop
  * (src/dbscan/dbscan.cpp:2276-2362: H2D at 2289, grid update 2293, core
  * identification 2300-2322, clustering 2331-2336, D2H 2344-2345).
  * Synchronous; returns RTDBS_ERR_DEVICE if a device bound was hit. */

@@ -79,6 +79,7 @@ cudaError_t configure_device(int dev) {
 
 constexpr int kFlagPooled = 1 << 30;  // of rtdbs_params.flags: an engine of a pool
 constexpr int kHostStage = 131072;    // largest window whose host-buffer calls go through pinned buffers
+constexpr size_t kCopiedAtOnce = 65536;  // bytes of plain host memory that cudaMemcpyAsync takes when called
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
@@ -458,16 +459,17 @@ bool direct_access(const rtdbs_engine* e, const void* p) {
     return a.type == cudaMemoryTypeDevice && a.device == e->device;
 }
 
-// Whether the host may read and write the caller's array as it is (device
-// memory given to a host-buffer call goes through a copy, which checks it).
-bool host_access(const void* p) {
+// Whether a host-buffer call may take the caller's array through the engine's
+// pinned buffers: plain host memory.  Pinned, managed and device memory may be
+// in use by work queued on the stream, so it is copied in the stream's order.
+bool through_staging(const rtdbs_engine* e, const void* p) {
     cudaPointerAttributes a;
-    if (!p) return true;
+    if (!p || !e->h_points) return false;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return a.type != cudaMemoryTypeDevice;
+    return a.type == cudaMemoryTypeUnregistered;
 }
 
 int copy_in(rtdbs_engine* e, const float* src, size_t npts, int on_device) {
@@ -492,6 +494,19 @@ int fetch_ctl_and_sync(rtdbs_engine* e) {
     if (e->copy) CUDA_TRY(cudaStreamSynchronize(e->copy));
     e->pipe_pending = false;  // everything queued, pipelined slides included, is done
     return check_device_error(e);
+}
+
+// Ends a host-buffer call: results to the caller's arrays, those that the
+// label pass wrote to the pinned buffers (io) once it is done.
+int finish_host_call(rtdbs_engine* e, const SlideIO& io, int32_t* label, int32_t* cluster_id) {
+    const size_t bytes = sizeof(int) * (size_t)e->p.window;
+    int rc = copy_out(e, io.label ? nullptr : label, io.cid ? nullptr : cluster_id, 0);
+    const int done = fetch_ctl_and_sync(e);  // (the pinned buffers are free again in any case)
+    if (rc == RTDBS_OK) rc = done;
+    if (rc != RTDBS_OK && rc != RTDBS_ERR_DEVICE) return rc;
+    if (io.label) std::memcpy(label, io.label, bytes);
+    if (io.cid) std::memcpy(cluster_id, io.cid, bytes);
+    return rc;
 }
 
 // Orders the legacy default stream after the work queued on the engine's stream.
@@ -742,22 +757,23 @@ int rtdbs_slide(rtdbs_engine* e, const float* new_points, int32_t* label, int32_
     if (!e->loaded) return fail(RTDBS_ERR_STATE, "rtdbs_load_window must come first");
     DeviceGuard guard(e->device);
     CUDA_TRY(guard.err);
-    // through pinned buffers that the kernels read and write themselves
-    if (e->h_points && host_access(new_points) && host_access(label) && host_access(cluster_id)) {
-        const size_t W = (size_t)e->p.window;
-        std::memcpy(e->h_points, new_points, sizeof(float) * (size_t)e->p.stride * e->p.dim);
-        int rc = run_slide(e, SlideIO{e->h_points, label ? e->h_label : nullptr, cluster_id ? e->h_cid : nullptr});
-        if (rc == RTDBS_OK) rc = fetch_ctl_and_sync(e);
-        if (rc != RTDBS_OK && rc != RTDBS_ERR_DEVICE) return rc;
-        if (label) std::memcpy(label, e->h_label, sizeof(int) * W);
-        if (cluster_id) std::memcpy(cluster_id, e->h_cid, sizeof(int) * W);
-        return rc;
+    // plain arrays through pinned buffers that the kernels read and write
+    // themselves, the others by copies
+    int rc = RTDBS_OK;
+    SlideIO io{e->v.staging, through_staging(e, label) ? e->h_label : nullptr,
+               through_staging(e, cluster_id) ? e->h_cid : nullptr};
+    if (through_staging(e, new_points)) {
+        const size_t bytes = sizeof(float) * (size_t)e->p.stride * e->p.dim;
+        // (a copy takes small plain arrays when it is called, larger ones after
+        // the work queued before; the wait costs 2 us of a 74 us slide)
+        if (bytes > kCopiedAtOnce) CUDA_TRY(cudaStreamSynchronize(e->stream));
+        std::memcpy(e->h_points, new_points, bytes);
+        io.input = e->h_points;
+    } else {
+        rc = copy_in(e, new_points, e->p.stride, 0);
     }
-    int rc = copy_in(e, new_points, e->p.stride, 0);
-    if (rc == RTDBS_OK) rc = run_slide(e, SlideIO{e->v.staging, nullptr, nullptr});
-    if (rc == RTDBS_OK) rc = copy_out(e, label, cluster_id, 0);
-    if (rc == RTDBS_OK) rc = fetch_ctl_and_sync(e);
-    return rc;
+    if (rc == RTDBS_OK) rc = run_slide(e, io);
+    return rc == RTDBS_OK ? finish_host_call(e, io, label, cluster_id) : rc;
 }
 
 int rtdbs_slide_async(rtdbs_engine* e, const float* d_new_points, int32_t* d_label,
@@ -827,14 +843,11 @@ int rtdbs_cluster(rtdbs_engine* e, int32_t* label, int32_t* cluster_id, int on_d
     CUDA_TRY(guard.err);
     const int rc0 = wait_outputs_free(e);
     if (rc0 != RTDBS_OK) return rc0;
-    if (e->h_points && !on_device && host_access(label) && host_access(cluster_id)) {
-        const SlideIO io{nullptr, label ? e->h_label : nullptr, cluster_id ? e->h_cid : nullptr};
+    if (!on_device) {
+        const SlideIO io{nullptr, through_staging(e, label) ? e->h_label : nullptr,
+                         through_staging(e, cluster_id) ? e->h_cid : nullptr};
         CUDA_TRY(rtdbs::launch_cluster(e->v, e->p.precision, 0, e->stream, true, nullptr, 0, io));
-        const int rc = fetch_ctl_and_sync(e);
-        if (rc != RTDBS_OK && rc != RTDBS_ERR_DEVICE) return rc;
-        if (label) std::memcpy(label, e->h_label, sizeof(int) * (size_t)e->p.window);
-        if (cluster_id) std::memcpy(cluster_id, e->h_cid, sizeof(int) * (size_t)e->p.window);
-        return rc;
+        return finish_host_call(e, io, label, cluster_id);
     }
     CUDA_TRY(rtdbs::launch_cluster(e->v, e->p.precision, 0, e->stream, true));
     int rc = copy_out(e, label, cluster_id, on_device);
