@@ -79,6 +79,7 @@ cudaError_t configure_device(int dev) {
 
 constexpr int kFlagPooled = 1 << 30;  // of rtdbs_params.flags: an engine of a pool
 constexpr int kHostStage = 131072;    // largest window whose host-buffer calls go through pinned buffers
+constexpr int kScatterStage = 24576;  // ... and whose labels the grid scan may store there (see host_outputs)
 constexpr size_t kCopiedAtOnce = 65536;  // bytes of plain host memory that cudaMemcpyAsync takes when called
 
 size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
@@ -496,6 +497,19 @@ int fetch_ctl_and_sync(rtdbs_engine* e) {
     return check_device_error(e);
 }
 
+// What the label pass of a host-buffer call writes itself: the pinned buffers
+// of plain arrays where it goes by slot (neighbour lists) or the window is
+// small.  The grid scan writes in sorted order, 4 bytes here and there across
+// the host link; two copies behind the pass take 10 to 15 us whatever the size.
+// Slides with MinPts 40, us, stores / copies: 2.5k points 62 / 77, 12k 70 / 79,
+// 20k 94 / 102, 24k 108 / 104 (3-D 97 / 103), 28k 111 / 106 (111 / 107), 100k
+// 251 / 173, 130k 348 / 240.
+SlideIO host_outputs(const rtdbs_engine* e, const float* input, const int32_t* label, const int32_t* cluster_id) {
+    const bool direct = e->v.list_cap >= 0 || e->p.window <= kScatterStage;
+    return SlideIO{input, direct && through_staging(e, label) ? e->h_label : nullptr,
+                   direct && through_staging(e, cluster_id) ? e->h_cid : nullptr};
+}
+
 // Ends a host-buffer call: results to the caller's arrays, those that the
 // label pass wrote to the pinned buffers (io) once it is done.
 int finish_host_call(rtdbs_engine* e, const SlideIO& io, int32_t* label, int32_t* cluster_id) {
@@ -760,8 +774,7 @@ int rtdbs_slide(rtdbs_engine* e, const float* new_points, int32_t* label, int32_
     // plain arrays through pinned buffers that the kernels read and write
     // themselves, the others by copies
     int rc = RTDBS_OK;
-    SlideIO io{e->v.staging, through_staging(e, label) ? e->h_label : nullptr,
-               through_staging(e, cluster_id) ? e->h_cid : nullptr};
+    SlideIO io = host_outputs(e, e->v.staging, label, cluster_id);
     if (through_staging(e, new_points)) {
         const size_t bytes = sizeof(float) * (size_t)e->p.stride * e->p.dim;
         // (a copy takes small plain arrays when it is called, larger ones after
@@ -844,8 +857,7 @@ int rtdbs_cluster(rtdbs_engine* e, int32_t* label, int32_t* cluster_id, int on_d
     const int rc0 = wait_outputs_free(e);
     if (rc0 != RTDBS_OK) return rc0;
     if (!on_device) {
-        const SlideIO io{nullptr, through_staging(e, label) ? e->h_label : nullptr,
-                         through_staging(e, cluster_id) ? e->h_cid : nullptr};
+        const SlideIO io = host_outputs(e, nullptr, label, cluster_id);
         CUDA_TRY(rtdbs::launch_cluster(e->v, e->p.precision, 0, e->stream, true, nullptr, 0, io));
         return finish_host_call(e, io, label, cluster_id);
     }

@@ -142,3 +142,17 @@ def test_results_reach_every_kind_of_array(rt, W, S, mp, points, label, ids):
             exp = expected(win, mp)
             assert lab is None or np.array_equal(lab.get(), exp[0])
             assert cid is None or np.array_equal(cid.get(), exp[1])
+
+
+# lists off: the grid scan stores to the engine's pinned buffers up to 24,576
+# points, copies follow it above
+@pytest.mark.parametrize("W,S", [(24_576, 1_024), (24_577, 3_511), (131_072, 4_096)])
+@pytest.mark.parametrize("mp", [1, 40])
+def test_grid_scan_results_reach_plain_arrays(W, S, mp):
+    pts = wl.gaussian_mixture(W + S, dim=2, k=20, seed=5)
+    with Engine(2, W, S, EPS, mp) as eng:
+        eng.load_window(pts[:W])
+        assert same(*eng.cluster(), expected(pts[:W], mp))
+        win = pts[:W].copy()
+        win[:S] = pts[W:]
+        assert same(*eng.slide(pts[W:]), expected(win, mp))
