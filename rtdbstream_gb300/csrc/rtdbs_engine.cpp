@@ -210,6 +210,7 @@ struct rtdbs_engine {
     // side stream for the decrement pass beside the sort (made on the first slide)
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_order = nullptr;  // the engine's work before the default stream's (made by a load)
     double cell_side = 0.0;
     // rtdbs_slide_pipelined: the outputs go to the host on their own stream
     // (`copy`) while the next slide runs; ev_done marks a slide's end on the
@@ -525,10 +526,9 @@ int finish_host_call(rtdbs_engine* e, const SlideIO& io, int32_t* label, int32_t
 
 // Orders the legacy default stream after the work queued on the engine's stream.
 int wait_on_default_stream(rtdbs_engine* e) {
-    const int rc = ensure_side(e);
-    if (rc != RTDBS_OK) return rc;
-    CUDA_TRY(cudaEventRecord(e->ev_fork, e->stream));
-    CUDA_TRY(cudaStreamWaitEvent(cudaStreamLegacy, e->ev_fork, 0));
+    if (!e->ev_order) CUDA_TRY(cudaEventCreateWithFlags(&e->ev_order, cudaEventDisableTiming));
+    CUDA_TRY(cudaEventRecord(e->ev_order, e->stream));
+    CUDA_TRY(cudaStreamWaitEvent(cudaStreamLegacy, e->ev_order, 0));
     return RTDBS_OK;
 }
 
@@ -683,6 +683,7 @@ int rtdbs_destroy(rtdbs_engine* e) {
     if (e->ev_done) cudaEventDestroy(e->ev_done);
     if (e->ev_free) cudaEventDestroy(e->ev_free);
     if (e->ev_fork) cudaEventDestroy(e->ev_fork);
+    if (e->ev_order) cudaEventDestroy(e->ev_order);
     for (auto& ev : e->ev_pipe)
         if (ev) cudaEventDestroy(ev);
     if (e->ev_join) cudaEventDestroy(e->ev_join);

@@ -1,0 +1,71 @@
+"""The host side of the C ABI (rtdbs_engine.cpp) against a stand-in for the
+CUDA runtime (cuda_stub/stub.cpp): which resources its calls make, and which
+arrays of the caller the kernels are given."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from rtdbstream_gb300 import build as B
+from rtdbstream_gb300 import engine as E
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    cxx = shutil.which("g++")
+    inc = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(B.nvcc()))), "include")
+    if not cxx or not os.path.exists(os.path.join(inc, "cuda_runtime.h")):
+        pytest.skip("no host compiler or CUDA headers")
+    out = str(tmp_path_factory.mktemp("stub") / "librtdbs_stub.so")
+    subprocess.run([cxx, "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", inc, "-I", B.CSRC,
+                    "-I", os.path.join(B.ROOT, "include"), os.path.join(B.CSRC, "rtdbs_engine.cpp"),
+                    os.path.join(HERE, "cuda_stub", "stub.cpp"), "-o", out], check=True)
+    L = ctypes.CDLL(out)
+    vp = ctypes.c_void_p
+    L.stub_memory.restype = vp
+    L.stub_memory.argtypes = [ctypes.c_size_t, ctypes.c_int]
+    L.stub_io.restype = vp
+    L.stub_pinned_limit.argtypes = [ctypes.c_size_t]
+    L.stub_calls.argtypes = [ctypes.c_char_p]
+    L.rtdbs_create.argtypes = [ctypes.POINTER(E.Params), vp, ctypes.POINTER(vp)]
+    for name in ("rtdbs_load_window", "rtdbs_pool_load_window", "rtdbs_slide_async", "rtdbs_destroy",
+                 "rtdbs_pool_destroy"):
+        getattr(L, name).argtypes = {"rtdbs_load_window": [vp, vp, ctypes.c_int],
+                                     "rtdbs_pool_load_window": [vp, ctypes.c_int32, vp, ctypes.c_int],
+                                     "rtdbs_slide_async": [vp, vp, vp, vp]}.get(name, [vp])
+    return L
+
+
+DEVICE = 2  # cudaMemoryTypeDevice
+
+
+def params(W, S, dim=2, **kw):
+    p = E.Params()
+    p.dim, p.window, p.stride, p.min_pts, p.eps = dim, W, S, 5, 0.5
+    for k, v in kw.items():
+        setattr(p, k, v)
+    return p
+
+
+def test_pool_streams_loaded_from_the_device_make_no_cuda_streams(lib):
+    """A first window from device points without a box needs one event for the
+    order between the streams, not a slide's side streams."""
+    pp, pool = E.PoolParams(), ctypes.c_void_p()
+    assert lib.rtdbs_pool_params_init(ctypes.byref(pp)) == 0
+    assert lib.rtdbs_pool_create(ctypes.byref(pp), None, ctypes.byref(pool)) == 0
+    pts = lib.stub_memory(1_000 * 8, DEVICE)
+    lib.stub_reset()
+    for _ in range(5):
+        sid, p = ctypes.c_int32(), params(1_000, 100)
+        assert lib.rtdbs_pool_add_stream(pool, ctypes.byref(p), ctypes.byref(sid)) == 0
+        for _ in range(2):
+            assert lib.rtdbs_pool_load_window(pool, sid.value, pts, 1) == 0
+    assert lib.stub_calls(b"launch_bbox") == 10
+    assert lib.stub_calls(b"cudaStreamCreate") == 0
+    assert lib.stub_calls(b"cudaEventCreate") == 5
+    assert lib.rtdbs_pool_destroy(pool) == 0
+    assert lib.stub_calls(b"cudaEventDestroy") >= 5
