@@ -448,17 +448,35 @@ int run_slide(rtdbs_engine* e, const SlideIO& io, bool pipelined = false) {
     return RTDBS_OK;
 }
 
-// Whether kernels on the engine's device may take the caller's array as it is:
-// this device's own memory, aligned to its elements (anything else goes
-// through a copy, which checks it).
-bool direct_access(const rtdbs_engine* e, const void* p) {
+// Whether one device allocation holds `bytes` bytes from p on (false where the
+// driver cannot tell).
+bool in_one_allocation(const void* p, size_t bytes) {
+    using AddressRange = int (*)(unsigned long long*, size_t*, unsigned long long);
+    static const AddressRange range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault, &found) !=
+            cudaSuccess)
+            cudaGetLastError();
+        return found == cudaDriverEntryPointSuccess ? reinterpret_cast<AddressRange>(f) : nullptr;
+    }();
+    const unsigned long long at = reinterpret_cast<uintptr_t>(p);
+    unsigned long long base = 0;
+    size_t size = 0;
+    return range && range(&base, &size, at) == 0 && at >= base && at - base <= size && bytes <= size - (at - base);
+}
+
+// Whether kernels on the engine's device may take the caller's array of
+// `bytes` bytes as it is: this device's own memory, aligned to its elements,
+// within its allocation (anything else goes through a copy, which checks it).
+bool direct_access(const rtdbs_engine* e, const void* p, size_t bytes) {
     cudaPointerAttributes a;
     if (reinterpret_cast<uintptr_t>(p) % sizeof(int) != 0) return false;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return a.type == cudaMemoryTypeDevice && a.device == e->device;
+    return a.type == cudaMemoryTypeDevice && a.device == e->device && in_one_allocation(p, bytes);
 }
 
 // Whether a host-buffer call may take the caller's array through the engine's
@@ -701,7 +719,7 @@ int rtdbs_load_window(rtdbs_engine* e, const float* points, int points_on_device
     // this build does not lay out hold them); device points are read in place
     // where the kernels may, and else copied the same way.
     const float* d_points = points;
-    if (!points_on_device || !direct_access(e, points)) {
+    if (!points_on_device || !direct_access(e, points, sizeof(float) * (size_t)W * dim)) {
         d_points = reinterpret_cast<const float*>(e->v.spt[0]);
         cudaStream_t s = e->stream;
         if (points_on_device && !e->p.has_bbox) {  // as the box reads the caller's points, see device_bbox
@@ -799,13 +817,14 @@ int rtdbs_slide_async(rtdbs_engine* e, const float* d_new_points, int32_t* d_lab
     int rc = RTDBS_OK;
     SlideIO io{d_new_points, d_label, d_cluster_id};
     const int W = e->p.window;
-    if (!direct_access(e, d_new_points)) {
+    const size_t out = sizeof(int) * (size_t)W;
+    if (!direct_access(e, d_new_points, sizeof(float) * (size_t)e->p.stride * e->p.dim)) {
         rc = copy_in(e, d_new_points, e->p.stride, 1);
         io.input = e->v.staging;
     }
     const bool apart = !d_label || !d_cluster_id || d_label + W <= d_cluster_id || d_cluster_id + W <= d_label;
-    if (d_label && (d_label == e->v.label || !apart || !direct_access(e, d_label))) io.label = nullptr;
-    if (d_cluster_id && (d_cluster_id == e->v.cid || !apart || !direct_access(e, d_cluster_id))) io.cid = nullptr;
+    if (d_label && (d_label == e->v.label || !apart || !direct_access(e, d_label, out))) io.label = nullptr;
+    if (d_cluster_id && (d_cluster_id == e->v.cid || !apart || !direct_access(e, d_cluster_id, out))) io.cid = nullptr;
     if (rc == RTDBS_OK) rc = run_slide(e, io);
     if (rc == RTDBS_OK)  // what the label pass did not write itself
         rc = copy_out(e, io.label || d_label == e->v.label ? nullptr : d_label,

@@ -69,3 +69,27 @@ def test_pool_streams_loaded_from_the_device_make_no_cuda_streams(lib):
     assert lib.stub_calls(b"cudaEventCreate") == 5
     assert lib.rtdbs_pool_destroy(pool) == 0
     assert lib.stub_calls(b"cudaEventDestroy") >= 5
+
+
+def test_device_arrays_shorter_than_the_call_are_refused(lib):
+    """Kernels are given a caller's device array only where its allocation
+    holds all of it; a shorter one goes to the copy, which refuses it."""
+    W, S = 1_000, 100
+    h, p = ctypes.c_void_p(), params(W, S)
+    assert lib.rtdbs_create(ctypes.byref(p), None, ctypes.byref(h)) == 0
+    full = lib.stub_memory(8 * W, DEVICE)
+    assert lib.rtdbs_load_window(h, full, 1) == 0
+    assert lib.stub_io(0) == full
+    assert lib.rtdbs_load_window(h, lib.stub_memory(8 * W - 4, DEVICE), 1) == E.RTDBS_ERR_CUDA
+    assert lib.rtdbs_load_window(h, full + 4, 1) == E.RTDBS_ERR_CUDA
+    new, lab, cid = lib.stub_memory(8 * S, DEVICE), lib.stub_memory(8 * W, DEVICE), lib.stub_memory(4 * W, DEVICE)
+    assert lib.rtdbs_slide_async(h, new, lab + 4 * W, cid) == 0  # the second half of lab
+    assert (lib.stub_io(0), lib.stub_io(1), lib.stub_io(2)) == (new, lab + 4 * W, cid)
+    launched = lib.stub_calls(b"launch")
+    assert lib.rtdbs_slide_async(h, new + 4, lab, cid) == E.RTDBS_ERR_CUDA
+    assert lib.stub_calls(b"launch") == launched  # nothing ran
+    assert lib.rtdbs_slide_async(h, new, lab + 4 * W + 4, cid) == E.RTDBS_ERR_CUDA
+    assert (lib.stub_io(1), lib.stub_io(2)) == (None, cid)  # the label pass was not given it
+    assert lib.rtdbs_slide_async(h, new, lab, cid + 8) == E.RTDBS_ERR_CUDA
+    assert (lib.stub_io(1), lib.stub_io(2)) == (lab, None)
+    assert lib.rtdbs_destroy(h) == 0
