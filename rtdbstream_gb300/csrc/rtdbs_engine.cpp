@@ -325,12 +325,17 @@ int allocate(rtdbs_engine* e) {
     CUDA_TRY(cudaMemsetAsync(v.table[1], 0, sizeof(ulonglong2) * P, e->stream));
     CUDA_TRY(cudaMemsetAsync(v.ctl, 0, sizeof(Ctl), e->stream));
     // Pinned memory: the control block's mirror, and on windows up to
-    // kHostStage the new points and results of host-buffer calls.
-    const bool stage = e->p.window <= kHostStage && !(e->p.flags & kFlagPooled);
+    // kHostStage the new points and results of host-buffer calls (which copy
+    // where these cannot be had).
+    bool stage = e->p.window <= kHostStage && !(e->p.flags & kFlagPooled);
     const size_t at_points = align_up(sizeof(Ctl), 256);
     const size_t at_label = at_points + align_up(sizeof(float) * (size_t)e->p.stride * e->p.dim, 256);
     const size_t out = align_up(sizeof(int) * (size_t)e->p.window, 256);
-    CUDA_TRY(cudaMallocHost((void**)&e->h_ctl, stage ? at_label + 2 * out : sizeof(Ctl)));
+    if (stage && cudaMallocHost((void**)&e->h_ctl, at_label + 2 * out) != cudaSuccess) {
+        cudaGetLastError();
+        stage = false;
+    }
+    if (!stage) CUDA_TRY(cudaMallocHost((void**)&e->h_ctl, sizeof(Ctl)));
     std::memset(e->h_ctl, 0, sizeof(Ctl));
     if (stage) {
         char* h = reinterpret_cast<char*>(e->h_ctl);

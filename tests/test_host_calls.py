@@ -32,11 +32,11 @@ def lib(tmp_path_factory):
     L.stub_pinned_limit.argtypes = [ctypes.c_size_t]
     L.stub_calls.argtypes = [ctypes.c_char_p]
     L.rtdbs_create.argtypes = [ctypes.POINTER(E.Params), vp, ctypes.POINTER(vp)]
-    for name in ("rtdbs_load_window", "rtdbs_pool_load_window", "rtdbs_slide_async", "rtdbs_destroy",
+    for name in ("rtdbs_load_window", "rtdbs_pool_load_window", "rtdbs_slide_async", "rtdbs_slide", "rtdbs_destroy",
                  "rtdbs_pool_destroy"):
         getattr(L, name).argtypes = {"rtdbs_load_window": [vp, vp, ctypes.c_int],
                                      "rtdbs_pool_load_window": [vp, ctypes.c_int32, vp, ctypes.c_int],
-                                     "rtdbs_slide_async": [vp, vp, vp, vp]}.get(name, [vp])
+                                     "rtdbs_slide_async": [vp, vp, vp, vp], "rtdbs_slide": [vp, vp, vp, vp]}.get(name, [vp])
     return L
 
 
@@ -92,4 +92,25 @@ def test_device_arrays_shorter_than_the_call_are_refused(lib):
     assert (lib.stub_io(1), lib.stub_io(2)) == (None, cid)  # the label pass was not given it
     assert lib.rtdbs_slide_async(h, new, lab, cid + 8) == E.RTDBS_ERR_CUDA
     assert (lib.stub_io(1), lib.stub_io(2)) == (lab, None)
+    assert lib.rtdbs_destroy(h) == 0
+
+
+def test_engine_without_pinned_staging_still_runs(lib):
+    """Where the pinned buffers of host calls cannot be had, an engine keeps
+    the control block's mirror alone, and host calls copy."""
+    W, S = 1_000, 100
+    h, p = ctypes.c_void_p(), params(W, S)
+    lib.stub_pinned_limit(4_096)
+    try:
+        assert lib.rtdbs_create(ctypes.byref(p), None, ctypes.byref(h)) == 0
+    finally:
+        lib.stub_pinned_limit(1 << 62)
+    pts = (ctypes.c_float * (2 * W))()
+    out = [(ctypes.c_int32 * W)() for _ in range(2)]
+    at = [ctypes.c_void_p(ctypes.addressof(x)) for x in (pts, *out)]
+    assert lib.rtdbs_load_window(h, at[0], 0) == 0
+    copies = lib.stub_calls(b"cudaMemcpyAsync")
+    assert lib.rtdbs_slide(h, *at) == 0
+    assert lib.stub_calls(b"cudaMemcpyAsync") == copies + 4  # points, label, ids, control block
+    assert (lib.stub_io(1), lib.stub_io(2)) == (None, None)
     assert lib.rtdbs_destroy(h) == 0
