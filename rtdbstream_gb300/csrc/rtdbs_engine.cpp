@@ -263,6 +263,12 @@ size_t plan_layout(rtdbs_engine* e, std::vector<Part>& parts) {
     // union 45 -> 37 us, 2-D 33 -> 31), 32 above (48k points 51 -> 45 us, 1M
     // walkers 186 -> 168)
     v.block_pts = W < 32768 ? 16 : 32;
+    // with two cells per Eps in 3-D a cell looks up 13 rows of 5 cells instead
+    // of 5 of 3, so a block's chain is as long with a fraction of the positions.
+    // us per slide with 8 / 16 / 32 (3-D mixture, MinPts 2; Eps 0.3): 10k points
+    // 88 / 99 / -, 50k 150 / 194 / 242, 80k 184 / 187 / 260, 200k 372 / 343 / 338;
+    // Eps 1.2: 50k 162 / 163 / 193, 200k 434 / 394 / 407
+    if (e->p.cell_mult == 2 && dim == 3) v.block_pts = W < 65536 ? 8 : 16;
     // Neighbour lists of non-core points (MinPts - 2 entries each) replace the
     // label pass's grid scan up to kListCap entries; above that the scan stays.
     const int mp = e->p.min_pts;

@@ -122,7 +122,7 @@ struct View {
     double E;                   // FP64 mode: eps * eps
     int key_bits;
     int sort_passes, sort_bits;  // radix passes over a chunk's keys, bits per pass
-    int block_pts;              // sorted positions a union warp takes as one block (16 or 32;
+    int block_pts;              // sorted positions a union warp takes as one block (8, 16 or 32;
                                 // pool launches take 32)
     int precision;              // RTDBS_PREC_* (batched launches dispatch on it)
     int list_cap;               // entries per neighbour list; -1: no lists (the
