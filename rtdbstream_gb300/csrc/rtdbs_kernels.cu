@@ -2853,8 +2853,14 @@ cudaError_t configure_kernels() {
 // to show (slides of 2.5k / 10k / 100k points 112 -> 106, 98 -> 95, 312 -> 291
 // us); on larger ones the waiting blocks take SM slots from the running kernel
 // (500k points 168 -> 186 us, 1M 324 -> 342).
+// With two cells per Eps in 3-D the clustering kernels are several times as long
+// and want the slots earlier.  us with it / without (3-D mixture): Eps 0.3,
+// MinPts 2, 10k points 88 / 90, 32k 168 / 160, 80k 189 / 176, MinPts 40, 130k 432
+// / 393; Eps 0.6, MinPts 8, 50k 164 / 170, 80k 181 / 168; mean gain of a mixture
+// and walkers at 32k to 130k points 2.5%.
 constexpr int kPdlWindow = 131072;
-bool pdl_on(const View& v) { return v.W <= kPdlWindow; }
+constexpr int kPdlWindowRows = 16384;  // two cells per Eps in 3-D
+bool pdl_on(const View& v) { return v.W <= (v.dim == 3 && v.cell_mult == 2 ? kPdlWindowRows : kPdlWindow); }
 
 cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, int init,
                          int stg_off, int advance, cudaStream_t s, bool pdl, const SlideIO& io) {
