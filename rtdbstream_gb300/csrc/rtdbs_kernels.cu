@@ -495,6 +495,36 @@ __device__ __forceinline__ int2 row_range_lane32(const View& v, const ulonglong2
         if (q < el && !(centre && k < K)) e[k] = table_entry(T, table_home32(rowkey | (q << sl), v.pbits));
     }
     int rs = INT_MAX, re = 0;
+    if (DIM == 3 && K == 2) {
+        // the probes past the first slots side by side as well.  One cell's
+        // after the other, in a table half full, held up the label pass and
+        // the union (130k points, MinPts 40: label 286 -> 184 us with blocks of
+        // 16; pools of such streams 643 -> 478 and 2845 -> 1682 us a round).  In 1-D
+        // and 2-D, with fewer rows and fuller cells, nothing is gained
+        unsigned open = 0;  // cells whose first slot holds another cell
+#pragma unroll
+        for (int k = 0; k < kW; ++k)
+            if (!((e[k].y ^ ghi) >> (kKeyBitsMax - 32)) && e[k].x != (rowkey | ((ql + (unsigned)(k - K)) << sl)))
+                open |= 1u << k;
+        for (unsigned step = 1; open && step <= v.pmask; ++step) {
+#pragma unroll
+            for (int k = 0; k < kW; ++k)
+                if ((open >> k) & 1u)
+                    e[k] = table_entry(T, (table_home32(rowkey | ((ql + (unsigned)(k - K)) << sl), v.pbits) + step) &
+                                              v.pmask);
+#pragma unroll
+            for (int k = 0; k < kW; ++k)
+                if (((e[k].y ^ ghi) >> (kKeyBitsMax - 32)) || e[k].x == (rowkey | ((ql + (unsigned)(k - K)) << sl)))
+                    open &= ~(1u << k);
+        }
+#pragma unroll
+        for (int k = 0; k < kW; ++k) {
+            if (((open >> k) & 1u) || ((e[k].y ^ ghi) >> (kKeyBitsMax - 32)) || (int)e[k].w <= (int)e[k].z) continue;
+            rs = min(rs, (int)e[k].z);
+            re = max(re, (int)e[k].w);
+        }
+        return re > 0 ? make_int2(rs, re) : make_int2(0, 0);
+    }
 #pragma unroll
     for (int k = 0; k < kW; ++k) {
         if ((e[k].y ^ ghi) >> (kKeyBitsMax - 32)) continue;  // out of the grid, or an empty or stale slot
@@ -2614,10 +2644,13 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, i
 
 // Positions a label warp takes as one block (at most CountShape's): short
 // chains on small windows (48k points, 4 / 8 / 16 / 32: 16 / 14 / 21 / 25 us; a
-// queue of single cells took 18).
+// queue of single cells took 18), and at any size for the 25 rows of two cells
+// per Eps in 3-D (8 / 16, mixture and walkers: 80k points 78 / 88, 72 / 78,
+// 130k 167 / 184, 127 / 131, 200k 180 / 186, 158 / 158; single cells 98, 94,
+// 201, 159, 227, 205).
 __host__ __device__ __forceinline__ int label_block(const View& v, bool pooled) {
-    const int most = v.dim == 3 && v.cell_mult == 2 ? 16 : 32;
-    return pooled ? most : min(most, v.W < 65536 ? 8 : 32);
+    const bool rows = v.dim == 3 && v.cell_mult == 2;
+    return pooled ? (rows ? 16 : 32) : (rows || v.W < 65536 ? 8 : 32);
 }
 
 template <int MODE, int DK>
