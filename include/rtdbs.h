@@ -99,9 +99,10 @@ typedef struct rtdbs_params {
                              rtdbstream_gb300/autotune.py.  No reference counterpart */
     int32_t query_lanes;  /* lanes that scan one expired or new point's neighbourhood in the
                              count passes, 16 or 32 (0 = 16 with one cell per Eps in a pool
-                             or at strides above 6,080 points, else 32; two cells per Eps
-                             needs 32): the block shape of those passes (a 256-thread
-                             block takes 16 or 8 points), picked by
+                             or at strides of more points than the GPU holds warps of these
+                             passes, 5,472 on 152 SMs, else 32; two cells per Eps needs 32):
+                             the block shape of those passes (4 or 8 points a 128-thread
+                             block, twice as many in a pool's), picked by
                              rtdbstream_gb300/autotune.py.  No reference counterpart */
     int32_t reserved[3];
 } rtdbs_params;

@@ -669,14 +669,14 @@ int rtdbs_create(const rtdbs_params* params, void* cuda_stream, rtdbs_engine** o
     View& v = e->v;
     v.dim = p.dim;
     v.cell_mult = p.cell_mult > 0 ? p.cell_mult : 1;
-    v.grab = p.work_grab;  // 0: by launch kind and window size (work_grab in the kernels)
+    v.grab = p.work_grab;  // 0: one block of positions (union_grab in the kernels)
     // a stride of few points leaves the count passes short of warps: the whole
-    // warp for one query while all fit the GPU at once (152 SMs of 40 warps).
-    // Decrement and increment, us, with 16 / 32 lanes: 500 points 16 + 16 / 12 +
-    // 12, 1k 14 + 14 / 10 + 10, 5k 52 + 67 / 32 + 35, 10k (1M walkers) 31 + 24 /
-    // 36 + 31
+    // warp for one query while all of a stride's are resident at once.  Geometric
+    // mean over five streams (1-D, 2-D and 3-D mixtures, walkers at two Eps) of a
+    // slide with 16 lanes against one with 32: 500 points 1.02, 2k 1.03, 4k 1.01;
+    // 5,473 points 0.96, 6k 0.95, 7k 0.95 (5k 0.97, for want of a finer rule)
     v.qlanes = p.query_lanes > 0 ? p.query_lanes
-                                 : (v.cell_mult == 1 && p.stride > 6080 ? rtdbs::kQueryLanes : 32);
+                                 : (v.cell_mult == 1 && p.stride > rtdbs::count_pass_warps() ? rtdbs::kQueryLanes : 32);
     v.W = p.window;
     v.S = p.stride;
     v.min_pts = p.min_pts;

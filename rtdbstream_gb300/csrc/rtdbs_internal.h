@@ -227,6 +227,8 @@ cudaError_t launch_cluster(const View& v, int precision, int advance, cudaStream
                            const SlideIO& io = SlideIO{});
 cudaError_t launch_counts_by_slot(const View& v, int* nn_by_slot, cudaStream_t s);
 cudaError_t configure_kernels();
+// Warps of the count passes that the configured device holds at once.
+int count_pass_warps();
 
 // Host helpers shared by the engine and the allocation-free entry point
 // (rtdbs_engine.cpp).

@@ -2881,6 +2881,8 @@ cudaError_t configure_kernels() {
     return cudaSuccess;
 }
 
+int count_pass_warps() { return (g_num_sms > 0 ? g_num_sms : 152) * kQueryBlocks * (kQueryThreads / 32); }
+
 // Slides of windows up to this size launch their kernels with programmatic
 // dependence: they are short enough for the launch and the first instructions
 // to show (slides of 2.5k / 10k / 100k points 112 -> 106, 98 -> 95, 312 -> 291

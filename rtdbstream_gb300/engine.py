@@ -280,7 +280,8 @@ def make_params(dim: int, window_size: int, stride_size: int, radius: float, min
     """rtdbs_params for one stream; cell_mult = grid cells per Eps (1 or 2),
     work_grab = cell runs per queue grab of the union warps (0: one block),
     query_lanes = lanes per query point in the count passes (0: 16 with one
-    cell per Eps in a pool or at strides above 6,080 points, else 32; 16 or 32)."""
+    cell per Eps in a pool or at strides above 5,472 points on 152 SMs, else 32;
+    16 or 32)."""
     L = load_library()
     p = Params()
     _check(L.rtdbs_params_init(ctypes.byref(p)))

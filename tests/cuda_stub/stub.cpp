@@ -22,6 +22,8 @@ std::map<uintptr_t, Range> g_memory;  // by first byte
 std::map<std::string, int> g_calls;
 size_t g_pinned_limit = ~size_t(0);   // largest cudaMallocHost that succeeds
 rtdbs::SlideIO g_io;                  // of the last first kernel of a slide or load
+int g_lanes = 0;                      // lanes per query of the last launch
+int g_warps = 5472;                   // count_pass_warps()
 
 cudaError_t count(const char* name) {
     ++g_calls[name];
@@ -68,6 +70,8 @@ extern "C" {
 int stub_calls(const char* name) { return g_calls[name]; }
 void stub_reset() { g_calls.clear(); }
 void stub_pinned_limit(size_t bytes) { g_pinned_limit = bytes; }
+void stub_warps(int n) { g_warps = n; }
+int stub_lanes() { return g_lanes; }
 void* stub_memory(size_t bytes, int type) { return take(bytes, (cudaMemoryType)type); }
 const void* stub_io(int which) { return which == 0 ? g_io.input : which == 1 ? (void*)g_io.label : (void*)g_io.cid; }
 
@@ -148,7 +152,8 @@ cudaError_t launch_chunk_step(const View&, int, int, int, int, int, cudaStream_t
     if (!ingested && io.input) g_io = io;
     return count("launch");
 }
-cudaError_t launch_window_build(const View&, int, const SlideIO& io, int, int, cudaStream_t, bool ingested) {
+cudaError_t launch_window_build(const View& v, int, const SlideIO& io, int, int, cudaStream_t, bool ingested) {
+    g_lanes = v.qlanes;
     if (!ingested) g_io = io;
     return count("launch");
 }
@@ -167,6 +172,7 @@ cudaError_t launch_cluster(const View&, int, int, cudaStream_t, bool, cudaEvent_
 }
 cudaError_t launch_counts_by_slot(const View&, int*, cudaStream_t) { return count("launch"); }
 cudaError_t configure_kernels() { return cudaSuccess; }
+int count_pass_warps() { return g_warps; }
 int batch_blocks(int, const View&, int) { return 1; }
 int batch_threads(int) { return 256; }
 bool batch_phase_split(int) { return false; }

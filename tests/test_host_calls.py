@@ -114,3 +114,18 @@ def test_engine_without_pinned_staging_still_runs(lib):
     assert lib.stub_calls(b"cudaMemcpyAsync") == copies + 4  # points, label, ids, control block
     assert (lib.stub_io(1), lib.stub_io(2)) == (None, None)
     assert lib.rtdbs_destroy(h) == 0
+
+
+@pytest.mark.parametrize("warps,S,cells,lanes,want", [(5_472, 5_472, 1, 0, 32), (5_472, 5_473, 1, 0, 16),
+                                                      (4_752, 4_753, 1, 0, 16), (4_752, 4_752, 0, 0, 32),
+                                                      (5_472, 9_000, 2, 0, 32), (5_472, 9_000, 1, 32, 32),
+                                                      (5_472, 100, 1, 16, 16)])
+def test_lanes_per_query_by_resident_warps(lib, warps, S, cells, lanes, want):
+    """A whole warp per query while the device holds the warps of a stride at once."""
+    lib.stub_warps(warps)
+    h, p = ctypes.c_void_p(), params(2 * S, S, cell_mult=cells, query_lanes=lanes)
+    assert lib.rtdbs_create(ctypes.byref(p), None, ctypes.byref(h)) == 0
+    assert lib.rtdbs_load_window(h, lib.stub_memory(16 * S, DEVICE), 1) == 0
+    assert lib.stub_lanes() == want
+    assert lib.rtdbs_destroy(h) == 0
+    lib.stub_warps(5_472)
