@@ -830,8 +830,8 @@ def run_batched(args, dev, stream, flush, world=1, rank=0, n_streams=256, rounds
     pool.close()
 
     # the plain path: the same streams, one engine each, slid one at a time
-    # (with the autotuner's single-engine choices, and with the default
-    # configuration for reference)
+    # (with the autotuner's single-engine choices, and with the engine's own
+    # defaults for reference)
     offsets, o = [], 0
     for st in streams:
         offsets.append(o)
@@ -860,7 +860,7 @@ def run_batched(args, dev, stream, flush, world=1, rank=0, n_streams=256, rounds
         return statistics.mean(ms)
 
     plain_ms = plain_round_ms(tuned_plain)
-    default_ms = plain_round_ms([{"cell_mult": 1, "work_grab": 8, "query_lanes": 16}] * len(streams))
+    default_ms = plain_round_ms([{"cell_mult": 1, "work_grab": 0, "query_lanes": 0}] * len(streams))
     plain_value, _, _ = combine_ranks(slid, plain_ms, world, f"cuda:{dev}")
     default_value, _, _ = combine_ranks(slid, default_ms, world, f"cuda:{dev}")
     # the tuner's per-bucket choices go to a file beside its cache, not on the line
@@ -881,7 +881,7 @@ def run_batched(args, dev, stream, flush, world=1, rank=0, n_streams=256, rounds
         "plain_one_at_a_time": {"value": plain_value, "round_ms": plain_ms,
                                 "config": "autotuned per stream bucket on single-engine slides"},
         "plain_one_at_a_time_default": {"value": default_value, "round_ms": default_ms,
-                                        "config": "1 cell per Eps, 8 items per grab, 16 lanes per count query"},
+                                        "config": "engine defaults: 1 cell per Eps, lanes per count query by stride"},
         "launches_per_round": stats["launches_per_round"], "graph_replays": stats["graph_replays"],
         "streams_exact_vs_fp64_oracle": f"{len(all_streams) - int(round(n_diff))}/{len(all_streams)}",
         "mean_neighbours_measured": {"min": round(float(mean_nn.min()), 1),

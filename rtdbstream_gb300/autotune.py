@@ -9,21 +9,24 @@ Three knobs change how the engine works without changing its results:
   in whole blocks of sorted positions (one block up to 31 runs) -- the work
   split between warps.
 - ``query_lanes``: the block shape of the count passes -- 16 lanes per expired
-  or new point (two points per warp, 16 per 256-thread block, their dependent
-  loads overlapping) or 32 (one point per warp, half the loop trips where
-  neighbourhoods are large).  Two cells per Eps always take 32.
+  or new point (two points per warp, their dependent loads overlapping) or 32
+  (one point per warp, half the loop trips where neighbourhoods are large).
+  Two cells per Eps always take 32.
 
-Streams are grouped into buckets by dimension, predicate, window size and
-density (mean points per occupied Eps-cell of a sample window).  For a
+Streams are grouped into buckets by dimension, predicate, window size, density
+(mean points per occupied Eps-cell of a sample window) and, for a stream slid
+alone, whose lanes depend on it, stride.  For a
 bucket seen for the first time the tuner times every candidate on the
 stream's own points and stores the choice in a JSON cache, so later streams
 of the bucket, and later runs, reuse it.  A stream slid alone is latency-bound
 and one slid in a pool round is throughput-bound, so the two are tuned
 apart: `choose` times a single engine (its first window, then a few slides),
 `choose_batched` times pool rounds over up to 16 streams of each bucket
-together.  The default (one cell per Eps, 8 runs per grab) is kept unless a
-candidate is at least 3% faster, so timing noise does not pick a
-configuration.  Candidates are (cell_mult, work_grab, query_lanes) triples.
+together.  The engine's own default is kept unless a candidate is at least 3%
+faster, so timing noise does not pick a configuration.  Candidates are
+(cell_mult, work_grab, query_lanes) triples; grabs below 32 are all one block,
+and more than one block lost wherever it was measured.  A cached choice holds
+for the kernels it was timed on (KERNELS).
 """
 from __future__ import annotations
 
@@ -37,9 +40,10 @@ import numpy as np
 
 from .engine import Engine, make_params
 
-# (cell_mult, work_grab, query_lanes); the first is the default
-CANDIDATES: Tuple[Tuple[int, int, int], ...] = ((1, 8, 16), (1, 5, 16), (1, 4, 16), (1, 16, 16), (1, 2, 16), (1, 1, 16),
-                                                (1, 8, 32), (2, 8, 32), (2, 4, 32), (2, 16, 32), (2, 1, 32))
+# (cell_mult, work_grab, query_lanes); the first is the engine's own choice
+# (0: by launch kind and stride), one of the two after it
+CANDIDATES: Tuple[Tuple[int, int, int], ...] = ((1, 0, 0), (1, 8, 16), (1, 8, 32), (2, 8, 32))
+KERNELS = 2             # raised when kernels change what is fastest: older choices are timed again
 MARGIN = 0.97           # a candidate replaces the default only when this much faster
 POOL_STREAMS = 16       # streams of a bucket timed together by choose_batched
 
@@ -57,11 +61,12 @@ def density(points: np.ndarray, eps: float, sample: int = 200_000) -> float:
     return float(len(pts) / max(1, len(counts)))
 
 
-def bucket_key(dim: int, window: int, precision: str, dens: float) -> str:
-    """Buckets: powers of two of the window and of the density."""
+def bucket_key(dim: int, window: int, precision: str, dens: float, stride: Optional[int] = None) -> str:
+    """Buckets: powers of two of the window, the density and (given one) the stride."""
     wb = int(round(math.log2(max(window, 1))))
     db = int(round(math.log2(max(dens, 1e-3))))
-    return f"d{dim}-{precision}-W2^{wb}-n2^{db}"
+    sb = "" if stride is None else f"-S2^{int(round(math.log2(max(stride, 1))))}"
+    return f"d{dim}-{precision}-W2^{wb}-n2^{db}{sb}"
 
 
 class Autotuner:
@@ -95,10 +100,9 @@ class Autotuner:
     def choose(self, points: np.ndarray, dim: int, window: int, stride: int, eps: float, min_pts: int,
                precision: str = "fp64") -> dict:
         """The bucket's configuration: {"cell_mult", "work_grab", "query_lanes", "ms"}."""
-        key = bucket_key(dim, window, precision, density(points[:window], eps))
-        hit = self.cache.get(key)
-        if hit is not None and "query_lanes" in hit:
-            return hit
+        key = bucket_key(dim, window, precision, density(points[:window], eps), stride)
+        if self._known(key):
+            return self.cache[key]
         return self._tune(key, lambda km, grab, ql: self.timer(points, dim, window, stride, eps, min_pts,
                                                                  precision, km, grab, ql))
 
@@ -112,10 +116,13 @@ class Autotuner:
         for k, st in zip(keys, streams):
             groups.setdefault(k, []).append(st)
         for k, members in groups.items():
-            if "query_lanes" not in self.cache.get(k, {}):
+            if not self._known(k):
                 sel = members[:POOL_STREAMS]
                 self._tune(k, lambda km, grab, ql: self.pool_timer(sel, km, grab, ql))
         return [self.cache[k] for k in keys]
+
+    def _known(self, key: str) -> bool:
+        return self.cache.get(key, {}).get("kernels") == KERNELS
 
     def _tune(self, key: str, run: Callable) -> dict:
         t0 = time.perf_counter()
@@ -132,7 +139,7 @@ class Autotuner:
         if default in ms and ms[best] > MARGIN * ms[default]:
             best = default
         km, grab, ql = (int(x) for x in best.split(","))
-        self.cache[key] = {"cell_mult": km, "work_grab": grab, "query_lanes": ql, "ms": ms}
+        self.cache[key] = {"cell_mult": km, "work_grab": grab, "query_lanes": ql, "ms": ms, "kernels": KERNELS}
         self.tuned += 1
         self.tune_seconds += time.perf_counter() - t0
         self._save()
