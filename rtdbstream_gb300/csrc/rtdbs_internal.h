@@ -29,6 +29,7 @@
 #pragma once
 
 #include <cstdint>
+#include <math.h>
 #include <cuda_runtime.h>
 
 namespace rtdbs {
@@ -161,6 +162,34 @@ struct View {
     const float* staging;        // new points [S][dim]
     Ctl* ctl;
 };
+
+// Cell coordinate along axis a: clamp(floor((x - origin) * inv_cell), 0, ext - 1)
+// in double, NaN in cell 0.  The single-precision quotient differs from the
+// double one by at most key_err cells (see set_geometry), so its floor is the
+// double's wherever no cell edge lies within that; the others, and quotients
+// outside [0, 2^22), are redone in double.  (FP64 runs at 1/64 of the FP32
+// rate here: a first window of 1M points took 50 us longer all in double, and
+// the decrement, which recomputed its queries' keys, 7 us per slide.)
+__host__ __device__ __forceinline__ long long cell_coord(const View& v, int a, float x) {
+#ifdef __CUDA_ARCH__  // (separate roundings; on the host by -ffp-contract=off)
+    const float t32 = __fmul_rn(__fsub_rn(x, v.origin32[a]), v.inv_cell32);
+    const float f = floorf(t32), in = __fsub_rn(t32, f);
+#else
+    const float t32 = (x - v.origin32[a]) * v.inv_cell32;
+    const float f = floorf(t32), in = t32 - f;
+#endif
+    long long c;
+    if (t32 >= 0.0f && t32 < 4194304.0f && in >= v.key_err[a] && in <= 1.0f - v.key_err[a]) {
+        c = (long long)(int)f;
+        const long long top = v.ext[a] - 1;
+        return c > top ? top : c;
+    }
+    double t = floor(((double)x - v.origin[a]) * v.inv_cell);
+    if (!(t >= 0.0)) t = 0.0;  // also maps NaN to cell 0
+    const double top = (double)(v.ext[a] - 1);
+    if (t > top) t = top;
+    return (long long)t;
+}
 
 // Combined template code of a stream's work kernels: dim + 4 (cells per Eps - 1).
 __host__ __device__ inline int dk_of(const View& v) { return v.dim + 4 * (v.cell_mult - 1); }

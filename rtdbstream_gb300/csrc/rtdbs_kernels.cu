@@ -72,29 +72,6 @@ __device__ __forceinline__ unsigned lanemask_lt(int lane) { return (1u << lane) 
 
 // ------------------------------------------------------------------ geometry
 
-// Cell coordinate along axis a: clamp(floor((x - origin) * inv_cell), 0, ext - 1)
-// in double, NaN in cell 0.  The single-precision quotient differs from the
-// double one by at most key_err cells (see set_geometry), so its floor is the
-// double's wherever no cell edge lies within that; the others, and quotients
-// outside [0, 2^22), are redone in double.  (FP64 runs at 1/64 of the FP32
-// rate here: a first window of 1M points took 50 us longer all in double, and
-// the decrement, which recomputed its queries' keys, 7 us per slide.)
-__device__ __forceinline__ long long cell_coord(const View& v, int a, float x) {
-    const float t32 = __fmul_rn(__fsub_rn(x, v.origin32[a]), v.inv_cell32);
-    const float f = floorf(t32), in = __fsub_rn(t32, f);
-    long long c;
-    if (t32 >= 0.0f && t32 < 4194304.0f && in >= v.key_err[a] && in <= 1.0f - v.key_err[a]) {
-        c = (long long)(int)f;
-        const long long top = v.ext[a] - 1;
-        return c > top ? top : c;
-    }
-    double t = floor(((double)x - v.origin[a]) * v.inv_cell);
-    if (!(t >= 0.0)) t = 0.0;  // also maps NaN to cell 0
-    const double top = (double)(v.ext[a] - 1);
-    if (t > top) t = top;
-    return (long long)t;
-}
-
 __device__ __forceinline__ unsigned long long cell_key(const View& v, float x, float y, float z) {
     unsigned long long key = (unsigned long long)cell_coord(v, 0, x) << v.shift[0];
     if (v.dim > 1) key |= (unsigned long long)cell_coord(v, 1, y) << v.shift[1];

@@ -10,6 +10,7 @@
 #include <map>
 #include <string>
 
+#include "rtdbs.h"
 #include "rtdbs_internal.h"
 
 namespace {
@@ -74,6 +75,20 @@ void stub_warps(int n) { g_warps = n; }
 int stub_lanes() { return g_lanes; }
 void* stub_memory(size_t bytes, int type) { return take(bytes, (cudaMemoryType)type); }
 const void* stub_io(int which) { return which == 0 ? g_io.input : which == 1 ? (void*)g_io.label : (void*)g_io.cid; }
+
+// Cells of n coordinates on axis 0 of the grid over [lo, hi]; also the grid's
+// extent there, its cell side and the largest error that the single-precision
+// quotient is trusted with.
+int stub_cells(double eps, int cells, float lo, float hi, const float* x, long long n, long long* cell,
+               long long* extent, double* side, float* key_err) {
+    rtdbs::View v{};
+    const int rc = rtdbs::set_geometry(v, 1, eps, cells, &lo, &hi, false, side);
+    if (rc != RTDBS_OK) return rc;
+    for (long long i = 0; i < n; ++i) cell[i] = rtdbs::cell_coord(v, 0, x[i]);
+    *extent = v.ext[0];
+    *key_err = v.key_err[0];
+    return RTDBS_OK;
+}
 
 cudaError_t cudaGetDeviceCount(int* n) { *n = 1; return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }

@@ -6,6 +6,7 @@ import os
 import shutil
 import subprocess
 
+import numpy as np
 import pytest
 
 from rtdbstream_gb300 import build as B
@@ -21,7 +22,7 @@ def lib(tmp_path_factory):
     if not cxx or not os.path.exists(os.path.join(inc, "cuda_runtime.h")):
         pytest.skip("no host compiler or CUDA headers")
     out = str(tmp_path_factory.mktemp("stub") / "librtdbs_stub.so")
-    subprocess.run([cxx, "-std=c++17", "-O1", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", inc, "-I", B.CSRC,
+    subprocess.run([cxx, "-std=c++17", "-O1", "-ffp-contract=off", "-fPIC", "-shared", "-Wl,-Bsymbolic", "-I", inc, "-I", B.CSRC,
                     "-I", os.path.join(B.ROOT, "include"), os.path.join(B.CSRC, "rtdbs_engine.cpp"),
                     os.path.join(HERE, "cuda_stub", "stub.cpp"), "-o", out], check=True)
     L = ctypes.CDLL(out)
@@ -129,3 +130,37 @@ def test_lanes_per_query_by_resident_warps(lib, warps, S, cells, lanes, want):
     assert lib.stub_lanes() == want
     assert lib.rtdbs_destroy(h) == 0
     lib.stub_warps(5_472)
+
+
+@pytest.mark.parametrize("cells", [1, 2])
+@pytest.mark.parametrize("lo,hi,eps", [(0.0, 100.0, 0.5), (-0.25, 1.25, 3.3e-3), (39.5, 40.5, 1e-3), (116.0, 117.0, 1e-3),
+                                       (-1e4, 1e4, 0.37), (0.0, 4.0e6, 1.0), (1e6, 1e6 + 10, 0.02), (0.0, 1e-3, 1e-9),
+                                       (-3e38, 3e38, 1e30), (0.0, 1e-36, 1e-38)])
+def test_cells_as_compiled_are_the_double_ones(lib, lo, hi, eps, cells):
+    """The cell coordinate (its single-precision shortcut and the geometry that
+    bounds it, as the library compiles them) against floor((x - lo) / side) in
+    double, clamped: on, next to, between and outside cell edges."""
+    lo, hi = float(np.float32(lo)), float(np.float32(hi))
+    ext, side, err = ctypes.c_longlong(), ctypes.c_double(), ctypes.c_float()
+
+    def run(x):
+        out = np.empty(len(x), np.int64)
+        assert lib.stub_cells(ctypes.c_double(eps), cells, ctypes.c_float(lo), ctypes.c_float(hi),
+                              x.ctypes.data_as(ctypes.c_void_p), ctypes.c_longlong(len(x)),
+                              out.ctypes.data_as(ctypes.c_void_p), ctypes.byref(ext), ctypes.byref(side),
+                              ctypes.byref(err)) == 0
+        return out
+
+    run(np.zeros(1, np.float32))
+    rng = np.random.default_rng(int(abs(lo) % 1e9) + cells)
+    with np.errstate(over="ignore"):
+        edges = (lo + rng.integers(-3, ext.value + 3, 200_000) * side.value).astype(np.float32)
+        span = hi - lo
+        x = np.concatenate([rng.uniform(lo - 0.1 * span, hi + 0.1 * span, 400_000).astype(np.float32), edges,
+                            np.nextafter(edges, np.float32(np.inf)), np.nextafter(edges, np.float32(-np.inf)),
+                            np.array([hi, lo, 3e38, -3e38, np.inf, -np.inf, np.nan], np.float32)])
+    with np.errstate(invalid="ignore", over="ignore"):
+        t = np.floor((x.astype(np.float64) - lo) * (1.0 / side.value))
+    want = np.clip(np.where(t >= 0, t, 0), 0, ext.value - 1).astype(np.int64)
+    assert np.array_equal(run(x), want)
+    assert err.value > 0
