@@ -2625,16 +2625,15 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, i
 // per Eps in 3-D (8 / 16, mixture and walkers: 80k points 78 / 88, 72 / 78,
 // 130k 167 / 184, 127 / 131, 200k 180 / 186, 158 / 158; single cells 98, 94,
 // 201, 159, 227, 205).
-__host__ __device__ __forceinline__ int label_block(const View& v, bool pooled) {
-    const bool rows = v.dim == 3 && v.cell_mult == 2;
-    return pooled ? (rows ? 16 : 32) : (rows || v.W < 65536 ? 8 : 32);
+__host__ __device__ __forceinline__ int label_block(int W, int dk, bool pooled) {
+    return pooled ? (dk == 7 ? 16 : 32) : (dk == 7 || W < 65536 ? 8 : 32);
 }
 
 template <int MODE, int DK>
 __global__ void __launch_bounds__(kClusterThreads, 4) k_label(View v, int advance) {
     pdl_wait();
     __shared__ LabelSmem<(DK & 3), (DK >> 2) + 1> sm;
-    label_body<MODE, DK>(v, advance, blockIdx.x, gridDim.x, sm, label_block(v, false));
+    label_body<MODE, DK>(v, advance, blockIdx.x, gridDim.x, sm, label_block(v.W, DK, false));
 }
 
 // Outputs by slot from the roots and the lists: core -> 0 and its root; a
@@ -2783,7 +2782,7 @@ __global__ void __launch_bounds__(PhaseShape<PHASE>::threads, PhaseShape<PHASE>:
         if (sv.list_cap >= 0)
             border_body(sv, 1, bx, nbx);
         else
-            label_body<MODE, DK>(sv, 1, bx, nbx, sm, label_block(sv, true));
+            label_body<MODE, DK>(sv, 1, bx, nbx, sm, label_block(sv.W, DK, true));
     }
 }
 
@@ -2914,7 +2913,7 @@ cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, 
                 break;
             }
             {
-                const int per = label_block(v, false) * (kClusterThreads / 32);  // positions per thread block
+                const int per = label_block(v.W, dk_of(v), false) * (kClusterThreads / 32);  // positions per thread block
                 RTDBS_DISPATCH(precision, dk_of(v), k_label, (v.W + per - 1) / per, kClusterThreads, s, pdl, v, advance);
             }
             break;
