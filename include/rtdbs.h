@@ -118,7 +118,8 @@ typedef struct rtdbs_stats {
     double  cell_side;       /* grid cell side (>= Eps) */
     int64_t device_bytes;    /* device memory owned by the engine */
     int32_t launches_per_slide; /* kernels launched by one slide */
-    int32_t chunks_per_slide;   /* grid-update chunks per slide (ceil(S / 16384)) */
+    int32_t chunks_per_slide;   /* grid-update chunks per slide: ceil(S / 16384), or 1
+                                   where slides build the grid from all slots */
     int64_t dist_tests;         /* distance tests evaluated, cumulative (the reference's
                                    DEBUG_INFO num_dist_calculations, src/dbscan/dbscan.cpp:145-212);
                                    query_tests + cluster_tests */

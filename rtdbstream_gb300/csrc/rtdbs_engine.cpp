@@ -205,6 +205,7 @@ struct rtdbs_engine {
     bool pooled = false;     // slid by a pool's rounds
     bool geometry_ready = false;
     bool loaded = false;
+    bool whole = false;      // slides build the grid anew from all slots (since the first window)
     cudaGraphExec_t slide_graph = nullptr;
     cudaGraphExec_t pipe_graph = nullptr;  // the slide of rtdbs_slide_pipelined
     // side stream for the decrement pass beside the sort (made on the first slide)
@@ -359,22 +360,20 @@ int check_device_error(rtdbs_engine* e) {
     return RTDBS_OK;
 }
 
-// Whether a slide builds the grid anew from all slots instead of by chunk
-// steps: where the new points make two chunks or more and at least a
-// twentieth of the window.  Device us per slide, chunk steps against a whole
-// build (2-D mixture / walkers): W = 50k, S = W 358 / 391 against 144 / 177,
-// S = W/2 207 / 236 against 144 / 175; W = 200k, S = 20k 257 / 232 against 223
-// / 232; W = 1M, S = 100k 1085 / 1077 against 613 / 699, S = 50k 720 / 706
-// against 597 / 697, S = 20k 492 / 450 against 565 / 693.  One chunk is always
-// better stepped (W = S = 10k: 102 against 107).
-bool slide_builds_window(const rtdbs_engine* e) {
-    return e->p.stride > e->chunk && 20ll * e->p.stride >= e->p.window && rtdbs::window_build_fits(e->v);
+// After a first window built from all slots (its counters in h_ctl): whether
+// slides are built so too.  One chunk is always better stepped (W = S = 10k: 102
+// us against 107).
+bool slides_build_window(const rtdbs_engine* e) {
+    double tests = 0.0;
+    for (unsigned long long t : e->h_ctl->ptests[0]) tests += (double)t;
+    return rtdbs::window_build_fits(e->v) &&
+           rtdbs::window_build_pays(e->p.window, e->p.stride, e->p.dim, e->v.cell_mult, e->h_ctl->nitems, tests);
 }
 
 // The slide's first kernel, with this slide's pointers.
 int start_slide(rtdbs_engine* e, const SlideIO& io) {
     const int S = e->p.stride;
-    if (slide_builds_window(e))
+    if (e->whole)
         CUDA_TRY(rtdbs::launch_window_phase(rtdbs::kPhaseIngest, e->v, e->p.precision, io, S, 0, e->stream));
     else
         CUDA_TRY(rtdbs::launch_phase(rtdbs::kPhaseIngest, e->v, e->p.precision, 0, std::min(e->chunk, S), 0, 0, 0,
@@ -388,7 +387,7 @@ int start_slide(rtdbs_engine* e, const SlideIO& io) {
 int enqueue_slide(rtdbs_engine* e, bool capturing, bool pipelined) {
     const int S = e->p.stride, C = e->chunk;
     const int nchunks = (S + C - 1) / C;
-    const bool whole = slide_builds_window(e);
+    const bool whole = e->whole;
     const SlideIO io{};  // as start_slide left it in the control block
     if (whole) CUDA_TRY(rtdbs::launch_window_build(e->v, e->p.precision, io, S, 0, e->stream, true));
     for (int j = 0; j < nchunks && !whole; ++j) {
@@ -792,6 +791,7 @@ int rtdbs_load_window(rtdbs_engine* e, const float* points, int points_on_device
     }
     int rc = fetch_ctl_and_sync(e);
     if (rc != RTDBS_OK) return rc;
+    e->whole = slides_build_window(e);
     e->loaded = true;
     return RTDBS_OK;
 }
@@ -950,7 +950,7 @@ int rtdbs_get_stats(rtdbs_engine* e, rtdbs_stats* s) {
     s->key_bits = e->v.key_bits;
     s->cell_side = e->cell_side;
     s->device_bytes = (int64_t)e->dev_bytes;
-    const bool whole = e->geometry_ready && !e->pooled && slide_builds_window(e);
+    const bool whole = e->whole && !e->pooled;
     const int nchunks = whole ? 1 : (e->p.stride + e->chunk - 1) / e->chunk;
     s->chunks_per_slide = nchunks;
     // per chunk 6 kernels, 7 when the sort phase needs a run merge (a chunk
@@ -972,7 +972,7 @@ int rtdbs_slide_profiled(rtdbs_engine* e, const float* d_new_points, rtdbs_phase
     CUDA_TRY(guard.err);
     const int S = e->p.stride, C = e->chunk;
     const SlideIO io{e->v.staging, nullptr, nullptr};
-    const bool whole = slide_builds_window(e);
+    const bool whole = e->whole;
     const int nchunks = whole ? 1 : (S + C - 1) / C;
     const int nev = nchunks * rtdbs::kChunkPhases + 4;
     std::vector<cudaEvent_t> ev(nev, nullptr);

@@ -23,6 +23,8 @@ std::map<uintptr_t, Range> g_memory;  // by first byte
 std::map<std::string, int> g_calls;
 size_t g_pinned_limit = ~size_t(0);   // largest cudaMallocHost that succeeds
 rtdbs::SlideIO g_io;                  // of the last first kernel of a slide or load
+int g_runs = 0;                       // cell runs and distance tests that a whole
+unsigned long long g_tests = 0;       // build reports
 int g_lanes = 0;                      // lanes per query of the last launch
 int g_warps = 5472;                   // count_pass_warps()
 
@@ -72,6 +74,7 @@ int stub_calls(const char* name) { return g_calls[name]; }
 void stub_reset() { g_calls.clear(); }
 void stub_pinned_limit(size_t bytes) { g_pinned_limit = bytes; }
 void stub_warps(int n) { g_warps = n; }
+void stub_window(int runs, unsigned long long tests) { g_runs = runs; g_tests = tests; }
 int stub_lanes() { return g_lanes; }
 void* stub_memory(size_t bytes, int type) { return take(bytes, (cudaMemoryType)type); }
 const void* stub_io(int which) { return which == 0 ? g_io.input : which == 1 ? (void*)g_io.label : (void*)g_io.cid; }
@@ -170,6 +173,9 @@ cudaError_t launch_chunk_step(const View&, int, int, int, int, int, cudaStream_t
 cudaError_t launch_window_build(const View& v, int, const SlideIO& io, int, int, cudaStream_t, bool ingested) {
     g_lanes = v.qlanes;
     if (!ingested) g_io = io;
+    v.ctl->nitems = g_runs;
+    v.ctl->ptests[0][0] = g_tests;
+    count("launch_window_build");
     return count("launch");
 }
 cudaError_t launch_window_phase(int phase, const View&, int, const SlideIO& io, int, int, cudaStream_t, bool) {

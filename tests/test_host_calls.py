@@ -34,10 +34,11 @@ def lib(tmp_path_factory):
     L.stub_calls.argtypes = [ctypes.c_char_p]
     L.rtdbs_create.argtypes = [ctypes.POINTER(E.Params), vp, ctypes.POINTER(vp)]
     for name in ("rtdbs_load_window", "rtdbs_pool_load_window", "rtdbs_slide_async", "rtdbs_slide", "rtdbs_destroy",
-                 "rtdbs_pool_destroy"):
+                 "rtdbs_pool_destroy", "rtdbs_get_stats"):
         getattr(L, name).argtypes = {"rtdbs_load_window": [vp, vp, ctypes.c_int],
                                      "rtdbs_pool_load_window": [vp, ctypes.c_int32, vp, ctypes.c_int],
-                                     "rtdbs_slide_async": [vp, vp, vp, vp], "rtdbs_slide": [vp, vp, vp, vp]}.get(name, [vp])
+                                     "rtdbs_slide_async": [vp, vp, vp, vp], "rtdbs_slide": [vp, vp, vp, vp],
+                                     "rtdbs_get_stats": [vp, vp]}.get(name, [vp])
     return L
 
 
@@ -164,3 +165,44 @@ def test_cells_as_compiled_are_the_double_ones(lib, lo, hi, eps, cells):
     want = np.clip(np.where(t >= 0, t, 0), 0, ext.value - 1).astype(np.int64)
     assert np.array_equal(run(x), want)
     assert err.value > 0
+
+
+# W, S, dim, cells per Eps, cell runs and distance tests of the first window, and
+# the slide's measured us by chunk steps and by a whole build
+PLANS = [(1_000_000, 50_000, 1, 1, 32_217, 13_389_424_178, 17_473, 73_530),  # many equal prices
+         (200_000, 40_000, 1, 2, 8_005, 472_327_967, 1_259, 3_539),
+         (1_000_000, 50_000, 3, 2, 998_791, 522_560, 733, 2_308),            # near-empty cells
+         (400_000, 20_000, 3, 2, 384_839, 6_766_817, 366, 925),
+         (100_000, 100_000, 3, 2, 99_987, 5_868, 689, 324),
+         (400_000, 80_000, 3, 1, 398_056, 124_137, 424, 252),
+         (100_000, 50_000, 2, 1, 27_762, 8_132_314, 292, 137),
+         (40_000, 40_000, 3, 1, 9_710, 2_947_298, 232, 127),
+         (1_000_000, 200_000, 1, 2, 78_762, 102_659_006, 1_496, 327),
+         (1_000_000, 500_000, 3, 1, 358_049, 173_499_013, 3_807, 850)]
+
+
+def test_slides_build_the_window_where_that_is_cheaper(lib):
+    """The plan of a slide of two chunks or more follows the window that was
+    loaded last; one chunk is always stepped."""
+    for W, S, dim, cells, runs, tests, steps, build in PLANS:
+        h, p, s = ctypes.c_void_p(), params(W, S, dim, cell_mult=cells), E.Stats()
+        assert lib.rtdbs_create(ctypes.byref(p), None, ctypes.byref(h)) == 0
+        pts, new = (lib.stub_memory(4 * dim * n, DEVICE) for n in (W, S))
+        chunks = -(-S // 16_384)
+        for r, t, want in ((runs, tests, 1 if build < steps else chunks), (100, 0, 1)):
+            lib.stub_window(r, ctypes.c_ulonglong(t))
+            assert lib.rtdbs_load_window(h, pts, 1) == 0
+            lib.stub_reset()
+            assert lib.rtdbs_slide_async(h, new, None, None) == 0
+            assert lib.stub_calls(b"launch_window_build") == (1 if want == 1 else 0), (W, S, dim, cells, r, t)
+            assert lib.rtdbs_get_stats(h, ctypes.byref(s)) == 0 and s.chunks_per_slide == want
+        assert lib.rtdbs_destroy(h) == 0
+    for S in (1_000, 16_384):
+        h, p = ctypes.c_void_p(), params(S, S)
+        lib.stub_window(100, ctypes.c_ulonglong(0))
+        assert lib.rtdbs_create(ctypes.byref(p), None, ctypes.byref(h)) == 0
+        assert lib.rtdbs_load_window(h, lib.stub_memory(8 * S, DEVICE), 1) == 0
+        lib.stub_reset()
+        assert lib.rtdbs_slide_async(h, lib.stub_memory(8 * S, DEVICE), None, None) == 0
+        assert lib.stub_calls(b"launch_window_build") == 0
+        assert lib.rtdbs_destroy(h) == 0
