@@ -2480,17 +2480,17 @@ __global__ void __launch_bounds__(256, 6) k_flatten(View v) {
 // cells as one candidate stream; a core candidate is tested against those
 // home points of its segment whose minimum it would lower.  Bound by load
 // latency.
-template <int DIM, int K>
+template <int DIM, int K, int THREADS, int BLOCK>
 struct LabelSmem {
-    using C = CountShape<DIM, K>;
-    static constexpr int kWarps = kClusterThreads / 32;
-    float4 pt[kWarps][C::kBlock];
-    unsigned long long skey[kWarps][C::kBlock];
-    unsigned segm[kWarps][C::kBlock];  // home points of a segment
-    int best[kWarps][C::kBlock];       // minimum root near a home point
-    int tstart[kWarps][C::kTasks];
-    int tpre[kWarps][C::kTasks + 1];
-    unsigned char tseg[kWarps][C::kTasks];
+    static constexpr int kWarps = THREADS / 32;
+    static constexpr int kTasks = BLOCK * CountShape<DIM, K>::kRows;
+    float4 pt[kWarps][BLOCK];
+    unsigned long long skey[kWarps][BLOCK];
+    unsigned segm[kWarps][BLOCK];  // home points of a segment
+    int best[kWarps][BLOCK];       // minimum root near a home point
+    int tstart[kWarps][kTasks];
+    int tpre[kWarps][kTasks + 1];
+    unsigned char tseg[kWarps][kTasks];
 };
 
 __device__ __forceinline__ void put_result(const View& v, int* ol, int* oc, int slot, int lab, int id) {
@@ -2515,13 +2515,13 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, i
     const int cur = (int)(b & 1);
     const unsigned gen = gen_of_build(b);
     const int n = v.ctl->nocc[cur];
-    const int nblk = (n + P - 1) / P, step = nbx * (kClusterThreads / 32);
+    const int nblk = (n + P - 1) / P, step = nbx * Smem::kWarps;
     const float4* spt = v.spt[cur];
     const int* sroot = v.sroot;
     int* ol = v.ctl->out_label;
     int* oc = v.ctl->out_cid;
     Tally tally;
-    for (int bk = bx * (kClusterThreads / 32) + wib; bk < nblk; bk += step) {
+    for (int bk = bx * Smem::kWarps + wib; bk < nblk; bk += step) {
         const int i = bk * P + lane;
         const bool hv = lane < P && i < n;
         float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -2625,14 +2625,24 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, i
 // per Eps in 3-D (8 / 16, mixture and walkers: 80k points 78 / 88, 72 / 78,
 // 130k 167 / 184, 127 / 131, 200k 180 / 186, 158 / 158; single cells 98, 94,
 // 201, 159, 227, 205).
-__host__ __device__ __forceinline__ int label_block(int W, int dk, bool pooled) {
+constexpr __host__ __device__ __forceinline__ int label_block(int W, int dk, bool pooled) {
     return pooled ? (dk == 7 ? 16 : 32) : (dk == 7 || W < 65536 ? 8 : 32);
 }
 
+// Thread blocks of the label pass of a stream slid alone.  With two cells per Eps
+// in 3-D the warps' work is so uneven that blocks of 8 warps, 4 per SM, kept 31%
+// of an SM's warps active: 300k points (3-D mixture, MinPts 40, 25 neighbours)
+// 357 us, where single cells from a queue had taken 250.  Blocks of 2 warps, 20
+// per SM (48 registers), slide in us with 8 x 4 / 2 x 16 / 2 x 20 / 2 x 24: 12k
+// points 96 / 95 / 97 / 106, 130k 277 / 261 / 262 / 300, 300k 581 / 513 / 480 /
+// 514, 1M 2201 / 1908 / 1750 / 1827; walkers 12k 88 / 89 / 90 / 98, 300k 343 / 317 /
+// 312 / 380, 1M 1270 / 1185 / 1165 / 1389.
+constexpr __host__ __device__ int label_threads(int dk) { return dk == 7 ? 64 : kClusterThreads; }
+
 template <int MODE, int DK>
-__global__ void __launch_bounds__(kClusterThreads, 4) k_label(View v, int advance) {
+__global__ void __launch_bounds__(label_threads(DK), DK == 7 ? 20 : 4) k_label(View v, int advance) {
     pdl_wait();
-    __shared__ LabelSmem<(DK & 3), (DK >> 2) + 1> sm;
+    __shared__ LabelSmem<(DK & 3), (DK >> 2) + 1, label_threads(DK), label_block(INT_MAX, DK, false)> sm;
     label_body<MODE, DK>(v, advance, blockIdx.x, gridDim.x, sm, label_block(v.W, DK, false));
 }
 
@@ -2778,7 +2788,7 @@ __global__ void __launch_bounds__(PhaseShape<PHASE>::threads, PhaseShape<PHASE>:
         __shared__ StreamSmem sm;
         flatten_body<MODE, DK>(sv, bx, nbx, sm);
     } else {
-        __shared__ LabelSmem<(DK & 3), (DK >> 2) + 1> sm;
+        __shared__ LabelSmem<(DK & 3), (DK >> 2) + 1, kClusterThreads, label_block(0, DK, true)> sm;
         if (sv.list_cap >= 0)
             border_body(sv, 1, bx, nbx);
         else
@@ -2913,8 +2923,9 @@ cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, 
                 break;
             }
             {
-                const int per = label_block(v.W, dk_of(v), false) * (kClusterThreads / 32);  // positions per thread block
-                RTDBS_DISPATCH(precision, dk_of(v), k_label, (v.W + per - 1) / per, kClusterThreads, s, pdl, v, advance);
+                const int threads = label_threads(dk_of(v));
+                const int per = label_block(v.W, dk_of(v), false) * (threads / 32);  // positions per thread block
+                RTDBS_DISPATCH(precision, dk_of(v), k_label, (v.W + per - 1) / per, threads, s, pdl, v, advance);
             }
             break;
         case kPhaseUnion: {
