@@ -265,14 +265,11 @@ size_t plan_layout(rtdbs_engine* e, std::vector<Part>& parts) {
     // walkers 186 -> 168)
     v.block_pts = W < 32768 ? 16 : 32;
     // with two cells per Eps in 3-D a cell looks up 13 rows of 5 cells instead
-    // of 5 of 3, so a block's chain is as long with a fraction of the positions.
-    // us per slide with 8 / 16 / 32 (3-D mixture with 10 neighbours and walkers,
-    // MinPts 2): 12k points 109 / 118 / 151 and 81 / 92 / 115, 50k 192 / 172 / 187
-    // and 108 / 116 / 137 (4 neighbours 170 / 178 / 241; one cell per warp 180), 80k
-    // 209 / 197 / 192 and 127 / 131 / 145, 250k 487 / 468 / 474 and 286 / 274 / 288,
-    // 400k 746 / 678 / 688 and 451 / 424 / 425, 500k 928 / 849 / 817 and 572 / 532 /
-    // 532, 1M 1876 / 1728 / 1678 and 1233 / 1124 / 1084 (one cell per warp 1690, 1202)
-    if (e->p.cell_mult == 2 && dim == 3) v.block_pts = W < 65536 ? 8 : (W < 400000 ? 16 : 32);
+    // of 5 of 3, so a block's chain is as long with half the positions (union_room
+    // in the kernels).  us per slide with 8 / 16 (3-D mixture with 10 neighbours
+    // and walkers, MinPts 3): 12k points 106 / 112 and 88 / 99, 50k 190 / 158 and 110
+    // / 117, 130k 251 / 252 and 179 / 182, 300k 398 / 351 and 254 / 239
+    if (e->p.cell_mult == 2 && dim == 3) v.block_pts = W < 32768 ? 8 : 16;
     // Neighbour lists of non-core points (MinPts - 2 entries each) replace the
     // label pass's grid scan up to kListCap entries; above that the scan stays.
     const int mp = e->p.min_pts;

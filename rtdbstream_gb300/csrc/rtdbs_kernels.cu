@@ -2163,26 +2163,31 @@ __device__ __forceinline__ int union_grab(const View& v) { return max(1, v.grab 
 constexpr int kUnionBlocks = 6;      // of a window slid alone
 constexpr int kPoolUnionBlocks = 5;
 
-template <int DIM, int K>
-struct UnionRows {
-    static constexpr int kRows = Stencil<DIM, true, K>::kRows;
-    static constexpr int kTasks = 32 * kRows;  // stencil rows of a block's segments, at most
-};
+// Most positions of a block (View::block_pts, a pool's blocks).  In a stream slid
+// alone the 13 rows of two cells per Eps in 3-D take 37 KB of shared memory a thread block for 32
+// positions, which leaves next to no L1 for the lookups, most of whose lines the
+// neighbouring cells share; 16 take half.  us per slide with room for 16 / 32, the
+// blocks 16 positions either way (3-D mixture, MinPts 3, 4 neighbours): 50k points
+// 162 / 172 (one cell per warp 165), 500k 508 / 587 (533), 2M 1847 / 2520 (2016);
+// walkers 500k 390 / 475 (512), 2M 1499 / 2217 (1884).  Pools of such streams lose by
+// blocks of 16 (walkers 4 x 300k points 628 -> 658 us a round, mixtures 988 -> 1005).
+constexpr __host__ __device__ int union_room(int dk, bool pooled) { return dk == 7 && !pooled ? 16 : 32; }
 
-template <int DIM, int K>
+template <int DIM, int K, int ROOM>
 struct UnionSmem {
+    static constexpr int kTasks = ROOM * Stencil<DIM, true, K>::kRows;  // stencil rows of a block's segments, at most
     float4 pt[kClusterThreads / 32][32];  // home points, .w = root known
     unsigned long long skey[kClusterThreads / 32][32];
     unsigned segm[kClusterThreads / 32][32];  // home cores of a segment
-    int tstart[kClusterThreads / 32][UnionRows<DIM, K>::kTasks];
-    int tpre[kClusterThreads / 32][UnionRows<DIM, K>::kTasks + 1];
-    unsigned char tseg[kClusterThreads / 32][UnionRows<DIM, K>::kTasks];
+    int tstart[kClusterThreads / 32][kTasks];
+    int tpre[kClusterThreads / 32][kTasks + 1];
+    unsigned char tseg[kClusterThreads / 32][kTasks];
 };
 
 template <int MODE, int DK, class Smem>
 __device__ __forceinline__ void union_body(const View& v, Smem& sm, int P, int grab) {
     constexpr int DIM = DK & 3, K = (DK >> 2) + 1;  // dimension, cells per Eps
-    constexpr int R = UnionRows<DIM, K>::kRows;
+    constexpr int R = Stencil<DIM, true, K>::kRows;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     float4* hpt = sm.pt[wib];
     int* tstart = sm.tstart[wib];
@@ -2365,7 +2370,7 @@ __device__ __forceinline__ void union_body(const View& v, Smem& sm, int P, int g
 template <int MODE, int DK>
 __global__ void __launch_bounds__(kClusterThreads, kUnionBlocks) k_union(View v) {
     pdl_wait();
-    __shared__ UnionSmem<(DK & 3), (DK >> 2) + 1> sm;
+    __shared__ UnionSmem<(DK & 3), (DK >> 2) + 1, union_room(DK, false)> sm;
     union_body<MODE, DK>(v, sm, v.block_pts, union_grab(v));
 }
 
@@ -2782,8 +2787,8 @@ __global__ void __launch_bounds__(PhaseShape<PHASE>::threads, PhaseShape<PHASE>:
         __shared__ LinkSmem sm;
         link_body<MODE, DK>(sv, bx, sm);
     } else if constexpr (PHASE == kBatchUnion) {
-        __shared__ UnionSmem<(DK & 3), (DK >> 2) + 1> sm;
-        union_body<MODE, DK>(sv, sm, 32, union_grab(sv));
+        __shared__ UnionSmem<(DK & 3), (DK >> 2) + 1, union_room(DK, true)> sm;
+        union_body<MODE, DK>(sv, sm, union_room(DK, true), union_grab(sv));
     } else if constexpr (PHASE == kBatchFlatten) {
         __shared__ StreamSmem sm;
         flatten_body<MODE, DK>(sv, bx, nbx, sm);

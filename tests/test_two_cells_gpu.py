@@ -1,6 +1,6 @@
 """Two cells per Eps in 3-D (13 and 25 stencil rows of five cells) against the
-oracle: windows around the union's and the label pass's blocks of 8, 16 and
-32 positions and around the switches between them, sparse and dense cells, labels
+oracle: windows around the union's and the label pass's blocks of 8 and 16
+positions and around the switches between them, sparse and dense cells, labels
 by neighbour lists and by grid scan, and a cell table half full, whose probes
 run on past the first slot.  Results are exact integers, so no tolerance."""
 import numpy as np
@@ -23,8 +23,8 @@ def _built():
 
 
 SMALL = [(W, W, 3.0, 0.4) for W in (1, 7, 8, 9, 15, 16, 17, 33)]
-LARGE = [(65_535, 4_369, 60.0, 0.6), (65_536, 4_096, 60.0, 0.6), (131_000, 6_550, 60.0, 0.3), (399_996, 12, 60.0, 0.2),
-         (400_000, 8_000, 60.0, 0.2), (16_384, 1_024, 60.0, 1.2),
+LARGE = [(65_535, 4_369, 60.0, 0.6), (65_536, 4_096, 60.0, 0.6), (131_000, 6_550, 60.0, 0.3), (32_767, 1_057, 60.0, 0.6),
+         (32_768, 2_048, 60.0, 0.6), (400_000, 8_000, 60.0, 0.2), (16_384, 1_024, 60.0, 1.2),
          (16_385, 565, 60.0, 1.2)]
 
 
