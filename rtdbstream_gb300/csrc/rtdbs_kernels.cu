@@ -2624,14 +2624,15 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, i
     }
 }
 
-// Positions a label warp takes as one block (at most CountShape's): short
+// Positions a label warp takes as one block: short
 // chains on small windows (48k points, 4 / 8 / 16 / 32: 16 / 14 / 21 / 25 us; a
 // queue of single cells took 18), and at any size for the 25 rows of two cells
 // per Eps in 3-D (8 / 16, mixture and walkers: 80k points 78 / 88, 72 / 78,
 // 130k 167 / 184, 127 / 131, 200k 180 / 186, 158 / 158; single cells 98, 94,
-// 201, 159, 227, 205).
+// 201, 159, 227, 205; pool rounds of mixtures, MinPts 40, 32 x 2k points 709 / 829,
+// 16 x 20k 1292 / 1363, 4 x 600k 4351 / 4404, single cells 4288).
 constexpr __host__ __device__ __forceinline__ int label_block(int W, int dk, bool pooled) {
-    return pooled ? (dk == 7 ? 16 : 32) : (dk == 7 || W < 65536 ? 8 : 32);
+    return dk == 7 ? 8 : (pooled || W >= 65536 ? 32 : 8);
 }
 
 // Thread blocks of the label pass of a stream slid alone.  With two cells per Eps
