@@ -669,6 +669,12 @@ int rtdbs_create(const rtdbs_params* params, void* cuda_stream, rtdbs_engine** o
     v.dim = p.dim;
     v.cell_mult = p.cell_mult > 0 ? p.cell_mult : 1;
     v.grab = p.work_grab;  // 0: one block of positions (union_grab in the kernels)
+    // with the shorter blocks of two cells per Eps in 3-D two of them, or large
+    // sparse windows wait for the queue.  us per slide with 1 / 2 (blocks of 32
+    // positions before): offset stream, MinPts 10, 200k points 91 / 87 (86), 500k 151 /
+    // 141 (139), 1M 274 / 254 (252); mixture with 60 neighbours 200k 248 / 235 (236),
+    // 1M 783 / 734 (860); walkers 200k 195 / 209 (245), 500k 384 / 398 (515)
+    if (p.work_grab == 0 && v.cell_mult == 2 && p.dim == 3 && p.window >= 131072) v.grab = 32;
     // a stride of few points leaves the count passes short of warps: the whole
     // warp for one query while all of a stride's are resident at once.  Geometric
     // mean over five streams (1-D, 2-D and 3-D mixtures, walkers at two Eps) of a
@@ -1400,7 +1406,9 @@ int rtdbs_pool_add_stream(rtdbs_pool* p, const rtdbs_params* params, int32_t* st
     // this stream's control block lives in the pool's contiguous array
     e->v.ctl = p->d_ctls + slot;
     e->pooled = true;
-    // a round's streams fill the GPU together: two queries per warp
+    // a round's streams fill the GPU together: blocks of 32 positions one by one, two
+    // queries per warp
+    e->v.grab = q.work_grab;
     if (q.query_lanes == 0 && e->v.cell_mult == 1) e->v.qlanes = rtdbs::kQueryLanes;
     {
         DeviceGuard guard(p->device);
