@@ -246,16 +246,16 @@ inline int slot_bits(int W) {
 inline bool window_build_fits(const View& v) {
     return v.W <= kChunkMax || v.key_bits + slot_bits(v.W) <= 64;
 }
-// Whether a slide of two chunks or more is cheaper built from all slots than
-// by chunk steps, by what the first window's build counted: its cell runs and
-// distance tests.  In units of a window position that a chunk step rewrites:
-// the steps rewrite W positions per chunk and, for every new and expired point
-// (both in one figure), look up its stencil (5/4 a cell) and test its candidates
-// (1/25 a test); the build orders W positions (3/4), looks up the stencil of
+// Whether a slide of two chunks or more, and at least a twentieth of the window,
+// is cheaper built from all slots than by chunk steps, by what the first window's
+// build counted: its cell runs and distance tests.  In units of a window position
+// that a chunk step rewrites: the steps rewrite W positions per chunk and, for
+// every new and expired point (both in one figure), look up its stencil (5/4 a
+// cell) and test its candidates (1/25 a test); the build orders W positions (3/4), looks up the stencil of
 // every cell run (3/10 a cell) and tests every point against its candidates (1/80
 // a test; 1/30 in 1-D, where steps keep most of the forest besides).  Fitted to
 // 990 pairs of times (W 40k to 2M, S W/100 to W, MinPts 3 to 30, streams from
-// near-empty cells to 13,000 tests a point, one and two cells per Eps): 0.8% over
+// near-empty cells to 13,000 tests a point, one and two cells per Eps): 0.7% over
 // the better of both in the geometric mean, 1.6 times at worst.  By S >= W/20 alone
 // it was 11% and 4.8 times (1-D prices with 13,000 tests a point, S = W/20, 1M points:
 // 17.5 ms stepped, 73.5 built; the offset stream with two cells per Eps 0.73 and
@@ -266,7 +266,7 @@ inline bool window_build_pays(int W, int S, int dim, int cells_per_eps, long lon
     const int chunks = (S + kChunkMax - 1) / kChunkMax;
     const double steps = (double)chunks * W + 1.25 * cells * S + 0.04 * tests * S / W;
     const double build = 0.75 * W + 0.3 * cells * (double)runs + tests / (dim == 1 ? 30.0 : 80.0);
-    return chunks > 1 && steps > build;
+    return chunks > 1 && 20ll * S >= W && steps > build;
 }
 // fresh_hints: start the union from fresh hints and forest (no reuse), for a
 // clustering of the window as it stands rather than after a slide, with its

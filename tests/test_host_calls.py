@@ -183,7 +183,7 @@ PLANS = [(1_000_000, 50_000, 1, 1, 32_217, 13_389_424_178, 17_473, 73_530),  # m
 
 def test_slides_build_the_window_where_that_is_cheaper(lib):
     """The plan of a slide of two chunks or more follows the window that was
-    loaded last; one chunk is always stepped."""
+    loaded last; one chunk, or less than a twentieth, is always stepped."""
     for W, S, dim, cells, runs, tests, steps, build in PLANS:
         h, p, s = ctypes.c_void_p(), params(W, S, dim, cell_mult=cells), E.Stats()
         assert lib.rtdbs_create(ctypes.byref(p), None, ctypes.byref(h)) == 0
@@ -197,11 +197,11 @@ def test_slides_build_the_window_where_that_is_cheaper(lib):
             assert lib.stub_calls(b"launch_window_build") == (1 if want == 1 else 0), (W, S, dim, cells, r, t)
             assert lib.rtdbs_get_stats(h, ctypes.byref(s)) == 0 and s.chunks_per_slide == want
         assert lib.rtdbs_destroy(h) == 0
-    for S in (1_000, 16_384):
-        h, p = ctypes.c_void_p(), params(S, S)
+    for W, S in ((1_000, 1_000), (16_384, 16_384), (357_000, 17_000)):
+        h, p = ctypes.c_void_p(), params(W, S)
         lib.stub_window(100, ctypes.c_ulonglong(0))
         assert lib.rtdbs_create(ctypes.byref(p), None, ctypes.byref(h)) == 0
-        assert lib.rtdbs_load_window(h, lib.stub_memory(8 * S, DEVICE), 1) == 0
+        assert lib.rtdbs_load_window(h, lib.stub_memory(8 * W, DEVICE), 1) == 0
         lib.stub_reset()
         assert lib.rtdbs_slide_async(h, lib.stub_memory(8 * S, DEVICE), None, None) == 0
         assert lib.stub_calls(b"launch_window_build") == 0
