@@ -89,12 +89,12 @@ typedef struct rtdbs_params {
     int32_t cell_mult;    /* K: grid cells per Eps along each axis, 1 or 2 (0 = 1); the
                              scan covers (2K+1)^dim cells of side Eps/K, so K = 2 tests
                              fewer pairs where cells are dense and costs more cells and
-                             work items where they are sparse (rtdbstream_gb300/autotune.py
+                             lookups where they are sparse (rtdbstream_gb300/autotune.py
                              picks it per stream).  The reference's grid has side Eps/sqrt(3)
                              (src/dbscan/dbscan.cpp:34-37) */
     int32_t work_grab;    /* cell runs a union warp takes from the shared queue at a time,
-                             1..64 (0 = the default), in whole blocks of sorted positions
-                             (16 or 32 of them, about 16 runs: one block up to 31): the
+                             1..64 (0 = the default), in whole blocks of 8 to 32 sorted
+                             positions, counted as 16 runs each (one block up to 31): the
                              work split between warps, picked by
                              rtdbstream_gb300/autotune.py.  No reference counterpart */
     int32_t query_lanes;  /* lanes that scan one expired or new point's neighbourhood in the
@@ -146,7 +146,7 @@ typedef struct rtdbs_phase_times {
     float sort_ms;        /* radix sort of the chunk's (cell, slot) words */
     float decrement_ms;   /* -1 on neighbours of expired points */
     float merge_ms;       /* sorted-window merge */
-    float build_ms;       /* cell table + work list */
+    float build_ms;       /* cell table */
     float increment_ms;   /* counts of new points, +1 on their neighbours */
     float union_ms;       /* union-find over core pairs */
     float flatten_ms;     /* root of every core point */

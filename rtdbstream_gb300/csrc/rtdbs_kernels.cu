@@ -322,7 +322,7 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
                                            unsigned long long key, int lane, int& rs, int& re) {
     using St = Stencil<DIM, false, K>;
     constexpr int kW = St::kW;
-    constexpr int kSlots = kW * St::kRows;           // cell slots, kept row by kept row
+    constexpr int kSlots = kW * St::kRows;           // cell slots, row by row
     constexpr int kPer = (kSlots + G - 1) / G;       // cells per lane
     static_assert(kPer <= 4 && St::kRows <= G, "stencil too large for the lane group");
     int2 rg[kPer];
@@ -345,7 +345,7 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
             e[k] = make_uint4(0, 0, 0, 0);  // no generation
             nks[k] = 0;
             const int cs = lane + k * G;
-            const int row = St::kFirst + cs / kW, d_last = cs % kW - K;
+            const int row = cs / kW, d_last = cs % kW - K;
             if (cs < kSlots) {
                 unsigned q0 = c0, q1 = c1, q2 = c2;
                 if (DIM == 1) {
@@ -378,8 +378,8 @@ __device__ __forceinline__ void row_ranges(const View& v, const ulonglong2* T, u
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
         rg[k] = make_int2(0, 0);
-        const int cs = lane + k * G;                                  // = kW * kept row + cell
-        const int row = St::kFirst + cs / kW, d_last = cs % kW - K;
+        const int cs = lane + k * G;                                  // = kW * row + cell
+        const int row = cs / kW, d_last = cs % kW - K;
         if (cs < kSlots) {
             long long q0 = c0, q1 = c1, q2 = c2;
             if (DIM == 1) {
@@ -472,7 +472,7 @@ __device__ __forceinline__ int2 row_range_lane32(const View& v, const ulonglong2
         if (q < el && !(centre && k < K)) e[k] = table_entry(T, table_home32(rowkey | (q << sl), v.pbits));
     }
     int rs = INT_MAX, re = 0;
-    if (DIM == 3 && K == 2) {
+    if constexpr (DIM == 3 && K == 2) {
         // the probes past the first slots side by side as well.  One cell's
         // after the other, in a table half full, held up the label pass and
         // the union (130k points, MinPts 40: label 286 -> 184 us with blocks of
@@ -500,18 +500,18 @@ __device__ __forceinline__ int2 row_range_lane32(const View& v, const ulonglong2
             rs = min(rs, (int)e[k].z);
             re = max(re, (int)e[k].w);
         }
-        return re > 0 ? make_int2(rs, re) : make_int2(0, 0);
-    }
+    } else {
 #pragma unroll
-    for (int k = 0; k < kW; ++k) {
-        if ((e[k].y ^ ghi) >> (kKeyBitsMax - 32)) continue;  // out of the grid, or an empty or stale slot
-        const unsigned nk = rowkey | ((ql + (unsigned)(k - K)) << sl);
-        int2 c = make_int2((int)e[k].z, (int)e[k].w);
-        if (e[k].x != nk)
-            c = table_find_from32(T, v.pmask, (table_home32(nk, v.pbits) + 1) & v.pmask, nk, ghi);
-        if (c.y > c.x) {
-            rs = min(rs, c.x);
-            re = max(re, c.y);
+        for (int k = 0; k < kW; ++k) {
+            if ((e[k].y ^ ghi) >> (kKeyBitsMax - 32)) continue;  // out of the grid, or an empty or stale slot
+            const unsigned nk = rowkey | ((ql + (unsigned)(k - K)) << sl);
+            int2 c = make_int2((int)e[k].z, (int)e[k].w);
+            if (e[k].x != nk)
+                c = table_find_from32(T, v.pmask, (table_home32(nk, v.pbits) + 1) & v.pmask, nk, ghi);
+            if (c.y > c.x) {
+                rs = min(rs, c.x);
+                re = max(re, c.y);
+            }
         }
     }
     return re > 0 ? make_int2(rs, re) : make_int2(0, 0);
@@ -556,16 +556,14 @@ __device__ __forceinline__ int2 row_range_lane(const View& v, const ulonglong2* 
     return row_range_lane64<DIM, HALF, K>(v, T, gen, key, row);
 }
 
-// The group's row ranges (group lanes 0..ROWS-1), clipped below at `lo`,
-// laid end to end: candidate idx in [0, total) lives at sorted position
-// start[r] + idx - pre[r] for the row r with pre[r] <= idx < pre[r+1].
+// The group's row ranges (group lanes 0..ROWS-1) laid end to end: candidate
+// idx in [0, total) lives at sorted position start[r] + idx - pre[r] for the row
+// r with pre[r] <= idx < pre[r+1].
 // Concatenating the rows keeps the candidate chunks full.  Called by the
 // whole warp; G-lane groups work independently.
 template <int ROWS, int G = 32>
-__device__ __forceinline__ int candidate_stream(int rs, int re, int lo, int lane, int* sstart,
-                                                int* spre) {
-    const int a = max(rs, lo);
-    const int len = lane < ROWS ? max(re - a, 0) : 0;
+__device__ __forceinline__ int candidate_stream(int rs, int re, int lane, int* sstart, int* spre) {
+    const int len = lane < ROWS ? re - rs : 0;
     int incl = len;
 #pragma unroll
     for (int o = 1; o < (ROWS > 16 ? 32 : 16); o <<= 1) {
@@ -575,7 +573,7 @@ __device__ __forceinline__ int candidate_stream(int rs, int re, int lo, int lane
     const int total = __shfl_sync(kFull, incl, ROWS - 1, G);
     __syncwarp();
     if (lane < ROWS) {
-        sstart[lane] = a;
+        sstart[lane] = rs;
         spre[lane] = incl - len;
     }
     if (lane == 0) spre[ROWS] = total;
@@ -1068,7 +1066,7 @@ __device__ __forceinline__ void decr_g(const View& v, int j, int c, int bx, Stre
     const unsigned long long key = has ? v.xkey[k] : 0ull;
     int rs, re;
     row_ranges<DIM, K, G>(v, v.table[old], gen, key, gl, rs, re);
-    int total = candidate_stream<Stencil<DIM, false, K>::kRows, G>(rs, re, 0, gl, rstart, rpre);
+    int total = candidate_stream<Stencil<DIM, false, K>::kRows, G>(rs, re, gl, rstart, rpre);
     if (!has) total = 0;
     const float4* spt = v.spt[old];
     int* scnt = v.scnt[old];
@@ -1392,10 +1390,11 @@ __global__ void __launch_bounds__(kMergeThreads) k_merge(View v, int j, int c, i
 // Cell table of the new sorted window.  A cell that starts and ends in one
 // warp's positions is entered once, by its first point; otherwise its first
 // point enters the start, its last the end.  Cells and cell runs (within 32
-// positions) are counted once per block.  Bound by the latency of the inserts
-// (a read, a CAS and a store to a random slot): 1M walkers, 275k cells, 25 us
-// (29 with a work list of cell runs for the union and the label pass, which
-// now take blocks of positions).
+// positions) are counted once per block, behind two barriers, for the statistics
+// and the choice between whole builds and chunk steps.  Bound by the latency of
+// the inserts (a read, a CAS and a store to a random slot; 25 of 36 cycles per
+// issue, the barriers 8): 1M walkers, 275k cells, 25 us (29 with a work list of
+// cell runs for the union and the label pass, which now take blocks of positions).
 struct BuildSmem {
     int cells, runs;
 };
@@ -1475,7 +1474,7 @@ __device__ __forceinline__ void incr_g(const View& v, int j, int c, int init, in
     const float4 ap = has ? v.ring[aslot] : make_float4(0.f, 0.f, 0.f, 0.f);
     int rs, re;
     row_ranges<DIM, K, G>(v, v.table[cur], gen, key, gl, rs, re);
-    int total = candidate_stream<Stencil<DIM, false, K>::kRows, G>(rs, re, 0, gl, rstart, rpre);
+    int total = candidate_stream<Stencil<DIM, false, K>::kRows, G>(rs, re, gl, rstart, rpre);
     if (!has) total = 0;
     int tmax = total;
 #pragma unroll
@@ -1843,8 +1842,9 @@ __global__ void k_fill(View v, int ob, int passes) {
 // trajectories 263 against 136).  Bound by instruction issue; against one
 // whole-stencil query per point with atomics on its neighbours, as the chunk
 // steps count, 1M walkers take 0.24 ms instead of 1.8.
-// Blocks per SM 8 / 10 / 12: 1M walkers 268 / 245 / 240 us; two cells per Eps
-// spill above 8 (48k points replaced per slide 115 / 125 / 122).
+// Blocks per SM 8 / 10 / 12: 1M walkers 268 / 245 / 240 us, though at 12 up to 16
+// bytes a thread are spilled; two cells per Eps lose more above 8 (48k points
+// replaced per slide 115 / 125 / 122).
 constexpr int kCountThreads = 128;
 
 template <int DIM, int K>
@@ -2156,10 +2156,12 @@ __device__ __forceinline__ int union_grab(const View& v) { return max(1, v.grab 
 // precision stream, 297 -> 79 us on 200k trajectories, 520 -> 62 us on 100k
 // prices, 606 -> 286 us per round of a 32-stream pool.
 // Without the root lookups before the tests: 204, 41, 129, 142, 430.
-// Row lookups in 32-bit words, and no filter flag beside the band, took its
-// register spills away (100-230 bytes a thread): walkers 168 -> 162, pool 288 ->
-// 278.  Thread blocks per SM 4 / 5 / 6: walkers 172 / 162 / 156 us, pool round
-// 298 / 278 / 287 (registers against warps in flight).
+// Row lookups in 32-bit words, and no filter flag beside the band, took most of its
+// register spills away (100-230 bytes a thread): walkers 168 -> 162, pool 288 -> 278.
+// Thread blocks per SM 4 / 5 / 6: walkers 172 / 162 / 156 us, pool round 298 / 278 /
+// 287 (registers against warps in flight).  Stores of spilled registers that are
+// left, in bytes a thread: one cell per Eps in 2-D and 3-D 48 and 52 (FP64), in
+// pools 28; two cells per Eps 88 and 96, in pools 60 and 92.
 constexpr int kUnionBlocks = 6;      // of a window slid alone
 constexpr int kPoolUnionBlocks = 5;
 
@@ -2384,7 +2386,7 @@ __device__ __forceinline__ void rebuild_list(const View& v, int at, int cur, uns
     const int a = slot_of(ap);
     int rs, re;
     row_ranges<DIM, K>(v, v.table[cur], gen, v.skey[cur][at], lane, rs, re);
-    const int total = candidate_stream<Stencil<DIM, false, K>::kRows>(rs, re, 0, lane, rstart, rpre);
+    const int total = candidate_stream<Stencil<DIM, false, K>::kRows>(rs, re, lane, rstart, rpre);
     int r = 0, nfound = 0;
     for (int base = 0; base < total; base += 32) {
         const int idx = base + lane;
@@ -3139,7 +3141,7 @@ int batch_blocks(int phase, const View& v, int c) {
         case kBatchUnion: return max(1, min(1024, (v.W + 1023) / 1024));  // persistent, queue-fed
         case kBatchLabel:
             if (v.list_cap >= 0) return max(1, min(1024, (v.W + 1023) / 1024));  // k_border
-            return max(1, min(1024, (v.W + 4095) / 4096));  // persistent, queue-fed
+            return max(1, min(1024, (v.W + 4095) / 4096));  // grid-strided
         case kBatchFlatten: return max(1, min(1024, (v.W + 1023) / 1024));  // (2,048 points a block: 74 us a round against 55)
         default: return 0;
     }
