@@ -308,8 +308,9 @@ class ClockSampler:
 
 
 def algorithmic_bytes(phase: str, W: int, S: int, dim: int, cells: int, items: int) -> float:
-    """Compulsory DRAM bytes of one launch of a phase (each live structure
-    touched once; neighbour candidates re-read from cache are not counted)."""
+    """Compulsory DRAM bytes of one launch of each of a phase's kernels (each live
+    structure touched once; neighbour candidates re-read from cache are not
+    counted)."""
     c = min(S, 16384)
     return {
         "ingest": c * (4 * dim + 16 + 8 + 16 + 8 + 8 + 8 + 8 + 16),
@@ -320,7 +321,8 @@ def algorithmic_bytes(phase: str, W: int, S: int, dim: int, cells: int, items: i
         "merge": W * (28 + 28 + 4 + 8) + c * (8 + 16),
         "build": W * 8 + cells * 32,
         "increment": c * (8 + 16) + c * 4,
-        "union": W * (16 + 4 + 4 + 4),
+        # link: hint, point, key; union: point, hint, key's cell, parent
+        "union": W * (4 + 16 + 8) + W * (16 + 4 + 4 + 4),
         # slot, root hint, parent read; root by slot and by position written
         "flatten": W * (4 + 4 + 4 + 4 + 4),
         # border pass: root by slot read; label, cid, parent, damage mark written
@@ -357,15 +359,21 @@ def measured_peak() -> tuple:
         return 6800.0, "fallback"
 
 
+# Kernels whose launches a phase's time covers, where they are not k_<phase> alone.
+PHASE_KERNELS = {"decrement": ("k_decr",), "increment": ("k_incr",), "union": ("k_link", "k_union"),
+                 "label": ("k_border",)}
+
+
 def ncu_traffic(phase: str):
-    """DRAM bytes per launch of the dominant kernel at W = 1M from the
-    committed ncu summary (profiles/ncu_traffic.json, captured at the
+    """DRAM bytes of one launch of each of the phase's kernels at W = 1M from
+    the committed ncu summary (profiles/ncu_traffic.json, captured at the
     bench's own size), or None."""
     path = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     try:
         with open(path) as f:
-            return json.load(f).get({"label": "k_border"}.get(phase, f"k_{phase}"))
-    except (OSError, ValueError):
+            per_kernel = json.load(f)
+        return sum(per_kernel[k] for k in PHASE_KERNELS.get(phase, (f"k_{phase}",)))
+    except (OSError, ValueError, KeyError):
         return None
 
 
@@ -583,7 +591,8 @@ def roofline_block(avg, st, per_slide, W, S, slide_ms, peak, peak_kind) -> dict:
     t = avg[dom] / 1000.0
     achieved = alg / t / 1e9
     slide_alg = sum(algorithmic_bytes(p, W, S, 3, st["cells"], st["work_items"]) for p in phases)
-    return {"bound": "hbm" if t_bytes >= t_flops else "fp32", "kernel": dom, "achieved": achieved, "peak": peak,
+    return {"bound": "hbm" if t_bytes >= t_flops else "fp32", "kernel": dom,
+            "kernels": list(PHASE_KERNELS.get(dom, (f"k_{dom}",))), "achieved": achieved, "peak": peak,
             "unit": "GB/s", "frac": achieved / peak, "peak_source": f"{peak_kind} hbm_gbs",
             "traffic": ncu_traffic(dom), "algorithmic_bytes_per_launch": alg,
             "fp32": {"ops_per_launch": flops, "achieved_tflops": flops / t / 1e12,
