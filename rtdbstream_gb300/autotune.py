@@ -24,9 +24,11 @@ apart: `choose` times a single engine (its first window, then a few slides),
 `choose_batched` times pool rounds over up to 16 streams of each bucket
 together.  The engine's own default is kept unless a candidate is at least 3%
 faster, so timing noise does not pick a configuration.  Candidates are
-(cell_mult, work_grab, query_lanes) triples; grabs below 32 are all one block,
-and more than one block lost wherever it was measured.  A cached choice holds
-for the kernels it was timed on (KERNELS).
+(cell_mult, work_grab, query_lanes) triples; grabs below 32 are all one block, 32
+are two.  Two blocks lose on sparse or small windows and win on large dense ones
+(a slide of 200k trajectories 159 -> 184 us, of a 500k-point 3-D mixture with 60
+neighbours 282 -> 241).  A cached choice holds for the kernels it was timed on
+(KERNELS).
 """
 from __future__ import annotations
 
@@ -42,8 +44,8 @@ from .engine import Engine, make_params
 
 # (cell_mult, work_grab, query_lanes); the first is the engine's own choice
 # (0: by launch kind and stride), one of the two after it
-CANDIDATES: Tuple[Tuple[int, int, int], ...] = ((1, 0, 0), (1, 8, 16), (1, 8, 32), (2, 8, 32))
-KERNELS = 2             # raised when kernels change what is fastest: older choices are timed again
+CANDIDATES: Tuple[Tuple[int, int, int], ...] = ((1, 0, 0), (1, 8, 16), (1, 8, 32), (1, 32, 0), (2, 8, 32), (2, 32, 32))
+KERNELS = 3             # raised when kernels change what is fastest: older choices are timed again
 MARGIN = 0.97           # a candidate replaces the default only when this much faster
 POOL_STREAMS = 16       # streams of a bucket timed together by choose_batched
 

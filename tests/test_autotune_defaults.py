@@ -29,6 +29,7 @@ def test_candidates_differ_and_start_with_the_engine_default():
     # a warp takes max(1, grab / 16) blocks of positions
     assert len({(k, max(1, grab >> 4), lanes) for k, grab, lanes in AT.CANDIDATES}) == len(AT.CANDIDATES)
     assert AT.CANDIDATES[0] == (1, 0, 0)
+    assert {(k, max(1, grab >> 4)) for k, grab, _ in AT.CANDIDATES} == {(1, 1), (1, 2), (2, 1), (2, 2)}
 
 
 def test_engine_default_is_kept_within_the_margin(tmp_path):
