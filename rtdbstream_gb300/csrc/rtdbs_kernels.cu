@@ -2626,31 +2626,35 @@ __device__ __forceinline__ void label_body(const View& v, int advance, int bx, i
     }
 }
 
-// Positions a label warp takes as one block: short
-// chains on small windows (48k points, 4 / 8 / 16 / 32: 16 / 14 / 21 / 25 us; a
-// queue of single cells took 18), and at any size for the 25 rows of two cells
-// per Eps in 3-D (8 / 16, mixture and walkers: 80k points 78 / 88, 72 / 78,
+// Positions a label warp takes as one block: short chains while the blocks are
+// few (48k points, 4 / 8 / 16 / 32: 16 / 14 / 21 / 25 us, a queue of single cells 18;
+// slides with MinPts 40 and 8 / 16 / 32: 3-D mixture with 5 neighbours 100k points
+// 91 / 93 / 103, 400k 198 / 189 / 193, 1M 503 / 472 / 462; the same with keys of 48 bits
+// 100k 179 / 196 / 233, 400k 470 / 479 / 534, queue 202 and 473; walkers 100k 105 / 104 /
+// 109, 400k 204 / 191 / 191, 1M 494 / 452 / 439).  At any size 8 for the 25 rows of two
+// cells per Eps in 3-D (8 / 16, mixture and walkers: 80k points 78 / 88, 72 / 78,
 // 130k 167 / 184, 127 / 131, 200k 180 / 186, 158 / 158; single cells 98, 94,
 // 201, 159, 227, 205; pool rounds of mixtures, MinPts 40, 32 x 2k points 709 / 829,
 // 16 x 20k 1292 / 1363, 4 x 600k 4351 / 4404, single cells 4288).
 constexpr __host__ __device__ __forceinline__ int label_block(int W, int dk, bool pooled) {
-    return dk == 7 ? 8 : (pooled || W >= 65536 ? 32 : 8);
+    if (dk == 7) return 8;
+    return pooled || W >= 524288 ? 32 : (W >= 131072 ? 16 : 8);
 }
 
-// Thread blocks of the label pass of a stream slid alone.  With two cells per Eps
-// in 3-D the warps' work is so uneven that blocks of 8 warps, 4 per SM, kept 31%
-// of an SM's warps active: 300k points (3-D mixture, MinPts 40, 25 neighbours)
-// 357 us, where single cells from a queue had taken 250.  Blocks of 2 warps, 20
-// per SM (48 registers), slide in us with 8 x 4 / 2 x 16 / 2 x 20 / 2 x 24: 12k
-// points 96 / 95 / 97 / 106, 130k 277 / 261 / 262 / 300, 300k 581 / 513 / 480 /
-// 514, 1M 2201 / 1908 / 1750 / 1827; walkers 12k 88 / 89 / 90 / 98, 300k 343 / 317 /
-// 312 / 380, 1M 1270 / 1185 / 1165 / 1389.
-constexpr __host__ __device__ int label_threads(int dk) { return dk == 7 ? 64 : kClusterThreads; }
+// Thread blocks of the label pass of a stream slid alone: two warps.  The warps'
+// work is so uneven that blocks of 8 warps, 4 per SM, kept 31% of an SM's warps
+// active (two cells per Eps in 3-D, 300k points: 357 us, where single cells from a
+// queue had taken 250).  Slide in us with blocks of 8 and 2 warps at the same
+// registers, MinPts 40: two cells per Eps, 3-D mixture with 25 neighbours, 130k
+// points 277 / 261, 300k 581 / 513, 1M 2201 / 1908; one cell, 60 neighbours, 400k 340 /
+// 315, 1M 635 / 586, walkers 1M 455 / 439.  20 blocks per SM (48 registers) instead of
+// 16 for two cells per Eps in 3-D: 300k 480, 1M 1750; 24: 514, 1827.
+constexpr int kLabelThreads = 64;
 
 template <int MODE, int DK>
-__global__ void __launch_bounds__(label_threads(DK), DK == 7 ? 20 : 4) k_label(View v, int advance) {
+__global__ void __launch_bounds__(kLabelThreads, DK == 7 ? 20 : 16) k_label(View v, int advance) {
     pdl_wait();
-    __shared__ LabelSmem<(DK & 3), (DK >> 2) + 1, label_threads(DK), label_block(INT_MAX, DK, false)> sm;
+    __shared__ LabelSmem<(DK & 3), (DK >> 2) + 1, kLabelThreads, label_block(INT_MAX, DK, false)> sm;
     label_body<MODE, DK>(v, advance, blockIdx.x, gridDim.x, sm, label_block(v.W, DK, false));
 }
 
@@ -2931,9 +2935,8 @@ cudaError_t launch_phase(int phase, const View& v, int precision, int j, int c, 
                 break;
             }
             {
-                const int threads = label_threads(dk_of(v));
-                const int per = label_block(v.W, dk_of(v), false) * (threads / 32);  // positions per thread block
-                RTDBS_DISPATCH(precision, dk_of(v), k_label, (v.W + per - 1) / per, threads, s, pdl, v, advance);
+                const int per = label_block(v.W, dk_of(v), false) * (kLabelThreads / 32);  // positions per thread block
+                RTDBS_DISPATCH(precision, dk_of(v), k_label, (v.W + per - 1) / per, kLabelThreads, s, pdl, v, advance);
             }
             break;
         case kPhaseUnion: {
